@@ -61,14 +61,20 @@ struct Work {
     int bx, by, bz;
 };
 
-struct ModelDev {
+// what the sweeps read of a model: a CTA copies it to shared memory first (load_par), where a
+// store to the wave field cannot alias it (from global memory each pointer and size was
+// loaded again after each store: 705 instructions a cell in the stress PML tiles)
+struct ModelPar {
     Grid g;
     Fields<float> f;
-    Fault<float> q;
     StepConst<float> c;
-    FvwScalars fs;
     PmlDesc D;
     PmlAux<float> X;
+};
+
+struct ModelDev : ModelPar {
+    Fault<float> q;
+    FvwScalars fs;
     HistDesc h;
     int law;
     int* it_dev;
@@ -120,6 +126,14 @@ __device__ bool grid_barrier(BatchSync* b, unsigned nblocks, int* status) {
     return ok != 0;
 }
 
+// every thread of the CTA calls it
+__device__ __forceinline__ void load_par(ModelPar& dst, const ModelPar& src) {
+    static_assert(sizeof(ModelPar) % 4 == 0, "copied by words");
+    for (int w = threadIdx.y * blockDim.x + threadIdx.x; w < (int)(sizeof(ModelPar) / 4); w += blockDim.x * blockDim.y)
+        reinterpret_cast<int*>(&dst)[w] = reinterpret_cast<const int*>(&src)[w];
+    __syncthreads();
+}
+
 struct ModelMaps {  // TMA descriptors of one model's interior sweeps (global memory, 64-byte aligned)
     VelMaps v;
     StrMaps s;
@@ -140,8 +154,10 @@ k_batch(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
     __shared__ __align__(8) uint64_t pbar;  // PML tiles staged through the ring memory
     if (threadIdx.x == 0 && threadIdx.y == 0) mbar_init(smem_addr(&pbar), 1);
     tma_ring_init(bars);
-    unsigned pc = 0;  // planes this CTA has put through its ring
+    __shared__ ModelPar P;
+    int pm = -1;      // the model that P holds
     unsigned pt = 0;  // PML tiles this CTA has staged (mbarrier phase = pt & 1)
+    unsigned pc = 0;  // planes this CTA has put through its ring
     const unsigned nb = gridDim.x;
     for (int s = 0; s < nsteps; ++s) {
         for (int ph = 0; ph < NPHASE; ++ph) {
@@ -152,37 +168,39 @@ k_batch(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
                 const int m = it.tm >> 8, type = it.tm & 255;
                 if (s >= limit[m]) continue;  // uniform over the CTA: the item belongs to one model
                 const ModelDev& M = models[m];
+                if (m != pm) load_par(P, M);  // (the last item ended with a barrier)
+                pm = m;
                 bool ok = true;
                 switch (type) {
                     case W_VEL_INT:
-                        ok = vel_interior_tma_body<float, true>(maps[m].v, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz,
+                        ok = vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz,
                                                                 ring, bars, pc, gstatus);
                         break;
                     case W_VEL_FAULT:
-                        vel_fault_body<float>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, 0);
+                        vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, 0);
                         break;
                     case W_VEL_PML:
-                        ok = vel_pml_tile<float>(M.g, M.f, M.D, M.X, M.c, it.bx, ring, smem_addr(&pbar), pt & 1u,
-                                                 gstatus);
+                        ok = vel_pml_tile<float, false, true>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(&pbar),
+                                                             pt & 1u, gstatus);
                         ++pt;
                         break;
-                    case W_VEL_FS: vel_fs_body<float>(M.g, M.f, it.bx, it.by, 0); break;
+                    case W_VEL_FS: vel_fs_body<float>(P.g, P.f, it.bx, it.by, 0); break;
                     case W_STR_INT:
-                        ok = str_interior_tma_body<float, true>(maps[m].s, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz,
+                        ok = str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz,
                                                                 ring, bars, pc, gstatus);
                         break;
-                    case W_STR_FAULT: str_fault_body<float>(M.g, M.f, M.q, M.c, it.bx, it.by, 0); break;
+                    case W_STR_FAULT: str_fault_body<float>(P.g, P.f, M.q, P.c, it.bx, it.by, 0); break;
                     case W_STR_PML:
-                        ok = str_pml_tile<float>(M.g, M.f, M.D, M.X, M.c, it.bx, ring, smem_addr(&pbar), pt & 1u,
-                                                 gstatus);
+                        ok = str_pml_tile<float, false, true>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(&pbar),
+                                                             pt & 1u, gstatus);
                         ++pt;
                         break;
-                    case W_STR_FS: str_fs_body<float>(M.g, M.f, it.bx, it.by, 0); break;
+                    case W_STR_FS: str_fs_body<float>(P.g, P.f, it.bx, it.by, 0); break;
                     case W_FBC:
-                        fault_bc_body<float>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by,
+                        fault_bc_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by,
                                              ring);
                         break;
-                    case W_NUC: nucleation_body<float>(M.g, M.q, M.c, M.fs, M.it_dev, it.bx, it.by, 0); break;
+                    case W_NUC: nucleation_body<float>(P.g, M.q, P.c, M.fs, M.it_dev, it.bx, it.by, 0); break;
                     default: break;
                 }
                 if (!ok) {  // a ring wait timed out: make every CTA leave at its next barrier
@@ -239,8 +257,9 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
     const Work it = work[b0 + blockIdx.x];
     int m;
     if (!item_live(it, limit, run_step, m)) return;
+    __shared__ ModelPar M;
+    load_par(M, models[m]);
     tma_ring_init(bars);
-    const ModelDev& M = models[m];
     unsigned pc = 0;
     if (STRESS)
         str_interior_tma_body<float, true>(maps[m].s, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc,
@@ -262,10 +281,10 @@ __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict
     const Work it = work[b0 + blockIdx.x];
     int m;
     if (!item_live(it, limit, run_step, m)) return;
-    if (threadIdx.x == 0 && threadIdx.y == 0) { mbar_init(smem_addr(&bar), 1); fence_mbar_init(); }
-    const ModelDev& M = models[m];
-    if (STRESS) str_pml_tile<float>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
-    else vel_pml_tile<float>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
+    __shared__ ModelPar M;
+    load_par(M, models[m]);
+    if (STRESS) str_pml_tile<float, false, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
+    else vel_pml_tile<float, false, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
 }
 
 // Plane items in three kernels by register need, so that light items are not held to a
@@ -985,11 +1004,11 @@ int fd3d_batch_add(fd3d_batch* b, const fd3d_params* pin, const double* lam_k, c
     M.cap = M.p.history_capacity > 0 ? M.p.history_capacity : 16;
     ModelDev& d = M.dev;
     d.g = make_grid(M.p);
-    d.c = make_const<float>(M.p);
     d.law = M.p.law;
     std::vector<Damp<float>> prof;
     make_pml<float>(M.p, d.D, prof);
-    if (!pml_modes_hold(d.D, prof)) return FD3D_ERR_ARG;
+    if (!pml_modes_hold(d.D, prof, M.p.nabc)) return FD3D_ERR_ARG;
+    d.c = make_const<float>(M.p, d.D);
     M.bytes = model_bytes(M.p, d.g, d.D, (int)prof.size(), M.nf, M.cap);
     if (!b->arena.alloc(M.bytes, &M.off)) return FD3D_ERR_NOMEM;
     Bump bp{b->arena_base + M.off};

@@ -117,57 +117,69 @@ struct FvwScalars {
 template <class T>
 struct StepConst {
     T dt, dh, dth, dth2, dht, damp_s, c1, c2;
-    T rdh;                   // RN(1/dh) for div_pre (NaN: divide directly)
+    T rdh, rdl;              // the pair of dh for div_by
+    T ds, dsi;               // the scale S of the dividends and 1/S (div_scale)
+    int pml_exact;           // 1: some divisor of the PML sweeps has no such pair, every cell uses div_exact
     double dtA, dhA, dthA;   // FP64 copies for the FP64 parts
 };
 
-// x / b rounded to nearest for a divisor b > 0 known before the launch, given
-// y = RN(1/b) formed on the host by an IEEE division.
+// x / b rounded to nearest (IEEE) for a divisor b > 0 known before the launch, in one
+// multiplication and one multiply-add: RN(x*h + RN(x*l)), with h close to 1/b and l close
+// to 1/b - h formed on the host.
 //
-// Method: Markstein's theorem (P. W. Markstein, "Computation of elementary functions
-// on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1), 1990; also in
-// J.-M. Muller et al., "Handbook of Floating-Point Arithmetic", the chapter on
-// FMA-based division): if y is within half an ulp of 1/b and q within one ulp of
-// x/b, the remainder r = x - b*q is exact and RN(q + r*y) = RN(x/b).  q0 = RN(x*y)
-// can be 1.5 ulp off, so one correction step first brings it within one ulp; the
-// second step is the theorem's.  Five FP32 operations, no reciprocal
-// approximation and no branch on the common path.
+// Method: N. Brisebarre, J.-M. Muller, S. K. Raina, "Accelerating correctly rounded
+// floating-point division when the divisor is known in advance", IEEE Trans. Computers
+// 53(8), 2004: the sum before its rounding is within a few 2^-48 of x/b (relative), so the
+// rounding can only go wrong where x/b lies that close to the midpoint of two consecutive
+// floats.  For a given b only a handful of significands of x do; div_pair (fd3d_setup.h)
+// enumerates them and takes the first pair (h, l) whose result is right, with a margin, for
+// every one.
 //
-// The theorem assumes that nothing under- or overflows.  For |x| outside
-// [2^-98, 2^98] (zero aside), NaN, infinities and a divisor outside the range checked
-// on the host (y is NaN then) the quotient is formed in FP64 and rounded to FP32: both
-// operands are exact in FP64, and rounding a quotient first to 53 bits and then to 24
-// (or fewer, for a subnormal result) gives the directly rounded quotient because
-// 53 >= 2*24 + 2 (S. A. Figueroa, "When is double rounding innocuous?", SIGNUM
-// Newsletter 30(3), 1995).  A zero dividend stays on the common path: every step then
-// yields a zero, and the sign of x put on the result makes it the signed zero x/b is
-// (for any other x in range the quotient already has the sign of x, since b > 0).  Zero
-// is the value of every cell ahead of the wavefront, so it must cost no more than a
-// normal value.  The result is therefore the IEEE FP32 quotient for every input; an
-// exhaustive GPU test over all 2^32 dividends (fd3d_check_division) holds it to that.
-// (The wave field's leading edge carries long runs of tiny values, so the fallback must
-// not be the slow path of a single-precision division.)
-__device__ __forceinline__ float div_pre(float x, float b, float y) {
-    float q = __fmul_rn(x, y);
-    float r = __fmaf_rn(-q, b, x);
-    q = __fmaf_rn(r, y, q);
-    r = __fmaf_rn(-q, b, x);
-    float q2 = copysignf(__fmaf_rn(r, y, q), x);
-    const float a = fabsf(x);
-    if (!((a >= 0x1p-98f || a == 0.0f) && a <= 0x1p98f && q2 == q2))
-        q2 = __double2float_rn(__ddiv_rn((double)x, (double)b));
-    return q2;
+// The bound on the error holds while RN(x*l) does not underflow into it, |x| >= 2^-70 for b
+// in the range that div_pair takes.  The wave field's leading edge runs through every magnitude
+// down to zero (in the first few hundred steps a third of a small model's PML cells are
+// below 2^-70, a tenth below 2^-126), so the sweeps form x scaled by a power of two S (div_scale),
+// which commutes with every rounding here, and put the factor back where the quotient is
+// used: that takes |x| down to where x/b is still a normal number, for one more
+// multiplication a cell.  A zero is exact too
+// (with l >= 0 its sign as well; with l < 0 div_by_signed puts the sign back).  Smaller
+// dividends are recorded in `key`: the least of 2*bits(x) - 1 over the quotients a thread forms,
+// which sends zero to the top of the range, so the test costs two integer operations a quotient
+// and one branch a cell.  A cell with key < DIV_KEY is done again with div_small, one with a
+// result that is not finite (x*l and x*h can cancel to NaN where x/b is infinite) with
+// div_exact.  An exhaustive GPU test over all 2^32 dividends (fd3d_check_division) holds all
+// three to the IEEE quotient.
+constexpr unsigned DIV_KEY = 2u * 0x1c800000u - 1u;  // the key of 2^-70
+__device__ __forceinline__ float div_by(float x, float h, float l, unsigned& key) {
+    key = min(key, 2u * __float_as_uint(x) - 1u);
+    return __fmaf_rn(x, h, __fmul_rn(x, l));
 }
+__device__ __forceinline__ float div_by_signed(float x, float h, float l, unsigned& key) {
+    return __uint_as_float(__float_as_uint(div_by(x, h, l, key)) | (__float_as_uint(x) & 0x80000000u));
+}
+// x / b for every finite x: scaled by 2^80 the quotient is div_by's.  Scaling it back rounds a
+// second time if the result is subnormal; where that went to the wrong side of a tie, the
+// residual x - q*b (exact here: q is a multiple of 2^-149, and less than a unit off) is more
+// than half a unit times b.
+__device__ __forceinline__ float div_small(float x, float b, float h, float l) {
+    unsigned key = 0;
+    const bool small = fabsf(x) < 0x1p-10f;
+    const float xs = x * (small ? 0x1p80f : 1.0f), qs = div_by_signed(xs, h, l, key);
+    float q = qs * (small ? 0x1p-80f : 1.0f);
+    if (small && fabsf(qs) < 0x1p-46f) {
+        const float rest = __fmaf_rn(-(q * 0x1p80f), b, xs), half = b * 0x1p-70f;
+        q += rest > half ? 0x1p-149f : rest < -half ? -0x1p-149f : 0.0f;
+        q = copysignf(q, x);  // (a negative zero plus zero is positive)
+    }
+    return q;
+}
+// The quotient formed in FP64 and rounded to FP32: both operands are exact in FP64, and
+// rounding a quotient first to 53 bits and then to 24 (or fewer, for a subnormal result)
+// gives the directly rounded one because 53 >= 2*24 + 2 (S. A. Figueroa, "When is double
+// rounding innocuous?", SIGNUM Newsletter 30(3), 1995).  Right for every x and b.
+__device__ __forceinline__ float div_exact(float x, float b) { return __double2float_rn(__ddiv_rn((double)x, (double)b)); }
 // the FP64 build divides directly (parity build, not the fast path)
-__device__ __forceinline__ double div_pre(double x, double b, double) { return x / b; }
-
-// y = RN(1/b) for div_pre, or NaN when b is outside [2^-20, 2^20] (FP64 fallback)
-template <class T>
-inline T div_pre_recip(T b) {
-    const double ab = (double)b;
-    if (!(ab >= 0x1p-20 && ab <= 0x1p20)) return (T)NAN;
-    return (T)1 / b;
-}
+__device__ __forceinline__ double div_exact(double x, double b) { return x / b; }
 
 // n / d for n < 2^24 and 1 <= d < 2^24 with rd = RN(1/d): the float product is within
 // one of the quotient, and one remainder test each way makes it exact (a few integer

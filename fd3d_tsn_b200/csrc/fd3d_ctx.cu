@@ -202,7 +202,8 @@ struct CtxBase {
     int slab_rank = -1, slab_nranks = 0;
     float last_ms = 0.f;
     bool profiling = false;
-    int pml_minb_vel = 1, pml_minb_str = 4;  // register caps of the PML sweeps (CTAs per SM; 1: none), measured fastest
+    // register caps of the PML sweeps (CTAs per SM; 1: none), set in alloc
+    int pml_minb_vel = 0, pml_minb_str = 0;
     std::vector<cudaEvent_t> kev;   // 2 per kernel id
     float ktimes[FD3D_NKERNELS] = {0};
     int klaunch[FD3D_NKERNELS] = {0};
@@ -240,6 +241,7 @@ struct Ctx : CtxBase {
     StepConst<T> c{};
     PmlDesc D{};
     PmlAux<T> X{};
+    std::vector<Damp<T>> prof;  // damping profiles (X.prof on the device)
     VelMaps vmaps{};        // TMA descriptors of the interior sweeps
     StrMaps smaps{};
     bool tma_ok = false;
@@ -303,12 +305,11 @@ struct Ctx : CtxBase {
         for (auto& e : kev) CK(cudaEventCreate(&e));
         g = slab ? make_slab_grid(p, slab_lo, slab_hi) : make_grid(p);
         if (slab) { split_bc = true; overlap = 0; }
-        c = make_const<T>(p);
         law = p.law;
         nf = (law == FD3D_LAW_FVW) ? 5 : 4;
-        std::vector<Damp<T>> prof;
         make_pml<T>(p, D, prof);
-        if (!pml_modes_hold(D, prof)) return FD3D_ERR_ARG;
+        if (!pml_modes_hold(D, prof, p.nabc)) return FD3D_ERR_ARG;
+        c = make_const<T>(p, D);
         D.klo = g.klo;
         D.khi = g.khi;
         const int stride = std::max(1, p.history_stride);
@@ -367,6 +368,10 @@ struct Ctx : CtxBase {
         X.prof = dprof;
         tma_ok = make_interior_maps<T>(g, f, vmaps, smaps) && prepare_tma_kernels<T>();
         if (slab && !tma_ok) return FD3D_ERR_CUDA;
+        // measured fastest (0.214 G cells, us): velocity 293 at 4 (330 at 3, 72 registers), stress 389
+        // at 4 (424 at 3; 5 spills, 399); FP64 (0.6 M cells) 20 at 3, 30 at 2 (no spills)
+        if (!pml_minb_vel) pml_minb_vel = sizeof(T) == 8 ? 3 : 4;
+        if (!pml_minb_str) pml_minb_str = sizeof(T) == 8 ? 2 : 4;
         if (!tma_ok && icfg.variant == IV_TMA) {
             std::fprintf(stderr, "fd3d: tensor maps of the interior sweeps could not be encoded for this grid; "
                                  "the interior sweeps fall back to plain loads (fd3d_ctx_info reports it)\n");
@@ -613,6 +618,8 @@ struct Ctx : CtxBase {
             if (std::fread(buf.data(), 1, n, fp) != n) return FD3D_ERR_IO;
             CK(cudaMemcpy(block + off, buf.data(), n, cudaMemcpyHostToDevice));
         }
+        // the profiles follow from the parameters; a file may hold them in an older layout
+        CK(cudaMemcpy((void*)X.prof, prof.data(), prof.size() * sizeof(Damp<T>), cudaMemcpyHostToDevice));
         steps_done = h.steps_done; rec_written = h.rec_written;
         medium_ok = h.medium_ok != 0; fault_ok = h.fault_ok != 0;
         f.lay = h.layered ? dlay : nullptr;
@@ -951,8 +958,8 @@ static int create_ctx(const fd3d_params* p, int slab_lo, int slab_hi, fd3d_ctx**
     if (const char* e = std::getenv("FD3D_PML_MINB")) {
         int v = 1, s = 0;
         const int n = std::sscanf(e, "%d,%d", &v, &s);
-        c->pml_minb_vel = std::min(4, std::max(1, v));
-        c->pml_minb_str = n == 2 ? std::min(4, std::max(1, s)) : c->pml_minb_vel;
+        c->pml_minb_vel = std::min(6, std::max(1, v));
+        c->pml_minb_str = n == 2 ? std::min(6, std::max(1, s)) : c->pml_minb_vel;
     }
     if (slab && c->icfg.variant != IV_TMA) { delete c; return FD3D_ERR_ARG; }  // z-slabs: the TMA sweeps only
     rc = c->alloc();

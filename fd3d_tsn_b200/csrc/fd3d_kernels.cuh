@@ -163,6 +163,9 @@ struct PmlDesc {
     long long cnt[PML_MAXS];      // cells of each strip's u/w loop range (0 for an absent strip)
     int ns;                       // strips present: 4, or 5 under FSPACE
     int klo, khi;                 // planes updated (Grid::klo, khi)
+    int tile0[PML_MAXS + 1];      // cum in tiles
+    int exact;                    // a divisor 1 + omega has no pair for div_by (StepConst::pml_exact)
+    double bmax;                  // the largest of them
 };
 
 // PML auxiliary components (the 24 split fields that init_pml allocates per strip,
@@ -180,11 +183,11 @@ inline long long pml_aux_cells(const PmlDesc& D) { return (D.cum[PML_MAXS] + PML
 inline size_t pml_aux_elems(const PmlDesc& D) { return (size_t)pml_aux_cells(D) * (AUX_NV + AUX_NS); }
 
 // One entry of a damping profile (init_pml's omega at one index): the factors
-// 1 - omega and 1 + omega of the split-field update and y = RN(1/(1 + omega)) for
-// div_pre, formed on the host with the same IEEE operations the reference performs.
+// 1 - omega and 1 + omega of the split-field update, formed on the host with the same IEEE
+// operations the reference performs, and the pair of 1 + omega for div_by_signed.
 template <class T>
 struct alignas(4 * sizeof(T)) Damp {
-    T m, p, r, o;  // 1 - omega, 1 + omega, RN(1/(1 + omega)), omega
+    T m, p, h, l;  // 1 - omega, 1 + omega, pair
 };
 
 // Damping of one split direction over a strip, from where init_pml leaves the profiles
@@ -192,10 +195,10 @@ struct alignas(4 * sizeof(T)) Damp {
 // and, in its corners, in x; the z strips in z and, in their corners and edges, in x and
 // y.  SPLIT_NEVER: omega = 0 over the whole strip, the update is p + inc.  SPLIT_ALWAYS:
 // the general form (p*(1-omega) + inc)/(1+omega), which is also exact where omega = 0
-// (a*1 = a, x/1 = x).  SPLIT_MAYBE: the general form where any lane of the warp is
-// damped, p + inc where none is (a warp-uniform branch, so no lane forms a quotient it
-// discards).  The host checks the SPLIT_NEVER directions against the profiles
-// (pml_modes_hold).
+// (a*1 = a, x/1 = x).  SPLIT_MAYBE: the general form where any lane of the warp lies in the
+// direction's nabc-1 outer cells, p + inc where none does (a warp-uniform branch, so no lane
+// loads a profile entry or forms a quotient it discards).  The host checks the undamped
+// ranges against the profiles (pml_modes_hold).
 enum { SPLIT_NEVER = 0, SPLIT_MAYBE = 1, SPLIT_ALWAYS = 2 };
 // strip class: 0 the x strips (1, 2), 1 the y strip (3), 2 the z strips (4, and 5 under FSPACE)
 __host__ __device__ constexpr int pml_class(int s) { return s <= 1 ? 0 : (s == 2 ? 1 : 2); }
@@ -204,11 +207,43 @@ __host__ __device__ constexpr int split_mode(int C, int DIR) {
     return DIR == C ? SPLIT_ALWAYS : (DIR < C ? SPLIT_MAYBE : SPLIT_NEVER);
 }
 
-template <class T, int MODE>
-__device__ __forceinline__ T pml_split(T p, T inc, const Damp<T>& o, bool warp_damped) {
-    if (MODE == SPLIT_NEVER || (MODE == SPLIT_MAYBE && !warp_damped)) return p + inc;
-    return div_pre(p * o.m + inc, o.p, o.r);
-}
+// The two divisions of a split-field update, by dh and by 1 + omega.
+//   DIV_FAST: the quotients of div_by on dividends scaled by c.ds; `key` tells whether
+//             all of them are right.  The quotient by dh stays scaled: its only use is an
+//             addition, where a multiply-add takes the factor out without a rounding.
+//   DIV_TINY: right for finite operands of any size, DIV_FULL: for all
+enum { DIV_FAST = 0, DIV_TINY = 1, DIV_FULL = 2 };
+template <class T, int HOW>
+struct PmlDiv {
+    const StepConst<T>& c;
+    unsigned key = 0xffffffffu;
+    __device__ __forceinline__ T scaled(T r) const {
+        if constexpr (HOW == DIV_FAST) return r * c.ds;
+        else return r;
+    }
+    // x / dh (of a scaled x: scaled)
+    __device__ __forceinline__ T by_dh(T x) {
+        if constexpr (HOW == DIV_FAST) return div_by(x, c.rdh, c.rdl, key);
+        else if constexpr (HOW == DIV_TINY) return div_small(x, c.dh, c.rdh, c.rdl);
+        else return div_exact(x, c.dh);
+    }
+    __device__ __forceinline__ T plus(T a, T q) const {  // a + x / dh
+        if constexpr (HOW == DIV_FAST) return __fmaf_rn(q, c.dsi, a);
+        else return a + q;
+    }
+    // the new split component: p old, q = by_dh(...) of its increment
+    template <int MODE>
+    __device__ __forceinline__ T split(T p, T q, const Damp<T>& o, bool warp_damped) {
+        if (MODE == SPLIT_NEVER || (MODE == SPLIT_MAYBE && !warp_damped)) return plus(p, q);
+        const T x = plus(p * o.m, q);
+        if constexpr (HOW == DIV_FAST) return div_by_signed(x * c.ds, o.h, o.l, key) * c.dsi;
+        else if constexpr (HOW == DIV_TINY) return div_small(x, o.p, o.h, o.l);
+        else return div_exact(x, o.p);
+    }
+};
+// false for a sum of magnitudes with one that is not finite (a sum that overflows only sends
+// the cell to the exact form)
+__device__ __forceinline__ bool pml_finite(float s) { return fabsf(s) <= 3.402823466e38f; }
 
 template <class T>
 struct PmlAux {
@@ -224,12 +259,14 @@ inline void pml_aux_bind(PmlAux<T>& X, T* pool, const PmlDesc& D) {
     X.str = pool + pml_aux_cells(D) * AUX_NV;
 }
 
-// shared-memory slot of component c of the cell that thread l of a tile owns
-__device__ __forceinline__ int aux_sm(int l, int ncomp, int c) { return (l >> 5) * 32 * ncomp + 32 * c + (l & 31); }
+// first component of the cell with compact index t in a group of ncomp components; the others
+// follow at steps of 32 elements
+__device__ __forceinline__ long long aux_at(long long t, int ncomp) { return (t >> 5) * (32 * ncomp) + (t & 31); }
 
 // strip of the tile that starts at compact index t0
 __device__ __forceinline__ int pml_tile_strip(const PmlDesc& D, long long t0) {
-    return (t0 >= D.cum[1]) + (t0 >= D.cum[2]) + (t0 >= D.cum[3]) + (t0 >= D.cum[4]);
+    const int tile = (int)(t0 / PML_TILE);
+    return (tile >= D.tile0[1]) + (tile >= D.tile0[2]) + (tile >= D.tile0[3]) + (tile >= D.tile0[4]);
 }
 
 // (i,j,k) of compact cell index t of strip s; false past the strip's last cell and, for
@@ -254,23 +291,35 @@ __device__ __forceinline__ bool pml_cell(const PmlDesc& D, int s, long long t, i
     return !SLAB || (k >= D.klo && k <= D.khi);
 }
 
-// Start of a tile: every thread orders its earlier generic accesses of the staging
-// buffer before the async copy, then one thread issues the bulk load of the tile's
-// range of the group (ncomp components).
-template <class T>
-__device__ __forceinline__ void pml_tile_begin(T* sm, const T* src, int ncomp, uint32_t bar) {
-    fence_proxy_async_smem();
-    __syncthreads();
+// The PML sweeps.  A tile's split components come by one bulk copy into shared memory while each
+// thread loads its cell's neighbours, profile entries and medium (all before the wait); the new
+// components go straight back from registers, one full line per warp and component (a bulk
+// copy back had to drain before the CTA could leave: 25% slower at 0.5 M cells, 3% at 12 M).
+// Bound by memory latency and instruction issue together at 4 CTAs per SM (64 registers).
+// Measured, velocity / stress, in us, against five-operation quotients with a branch each and
+// partly written sectors in the x strips (pml_sector_rest): 11.9 M PML cells 279 / 381 (340 /
+// 543), 13 M cells of 64 models 375 / 526 (446 / 638), 0.5 M cells 14.3 / 18.9 (15.5 / 22.7).
+// Left out, measured: the components by plain loads (the registers hold a third of the inputs
+// at a time); all inputs through shared memory by bulk copies of row pieces (a copy is issued
+// by one lane, 30 a tile); u, v, w and the normal and shear stresses in CTAs of their own.
+//
+// Starts the copy of a tile's range of a group (bytes); every thread calls it.  REUSED: sm and
+// bar served an earlier tile of this CTA.
+template <bool REUSED>
+__device__ __forceinline__ void pml_tile_begin(uint32_t sm, const void* src, uint32_t bytes, uint32_t bar) {
+    if (REUSED) {
+        fence_proxy_async_smem();
+        __syncthreads();
+    }
     if (threadIdx.x == 0 && threadIdx.y == 0) {
+        if (!REUSED) { mbar_init(bar, 1); fence_mbar_init(); }
         fence_proxy_async_global();
-        const uint32_t bytes = PML_TILE * ncomp * (uint32_t)sizeof(T);
         mbar_expect_tx(bar, bytes);
-        bulk_load(smem_addr(sm), src, bytes, bar);
+        bulk_load(sm, src, bytes, bar);
     }
 }
-// Wait (bounded) for the tile's load; false on every thread if any thread gave up
-// (ST_TIMEOUT recorded after one more bounded wait for the copy in flight).  Every
-// thread of the CTA leaves it converged.
+// Waits (bounded) for the tile's load; false on every thread if any thread gave up
+// (ST_TIMEOUT recorded after one more bounded wait for the copy in flight).
 __device__ __forceinline__ bool pml_tile_wait(uint32_t bar, uint32_t parity, int* status) {
     const bool ok = mbar_wait(bar, parity);
     if (__syncthreads_or(!ok)) {
@@ -280,85 +329,165 @@ __device__ __forceinline__ bool pml_tile_wait(uint32_t bar, uint32_t parity, int
     }
     return true;
 }
+// whether any of a warp's cells lies in the damped ends of the strip in x / y (SPLIT_MAYBE);
+// every lane of the warp calls it
+template <int C>
+__device__ __forceinline__ void pml_damped(const Grid& g, const Strip& S, bool act, int i, int j, bool& wx, bool& wy) {
+    const int i2 = i - S.nxb, n = g.nabc - 1;
+    wx = wy = true;
+    if (split_mode(C, 0) == SPLIT_MAYBE) wx = __any_sync(0xffffffffu, act && (i2 < n || i2 >= S.ni - n));
+    if (split_mode(C, 1) == SPLIT_MAYBE) wy = __any_sync(0xffffffffu, act && j - S.nyb < n);
+}
 
-// pml_uvw in one tile of strip class C (fd3d_deriv.f90:1927-2293): one cell per thread.
-template <class T, int C, bool SLAB>
-__device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D,
-                                               const PmlAux<T>& X, const StepConst<T>& c, int s, long long t0, T* sm,
-                                               uint32_t bar, uint32_t parity, int* status) {
-    constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
-    const int l = threadIdx.y * blockDim.x + threadIdx.x;
-    T* gaux = X.vel + t0 * AUX_NV;
-    pml_tile_begin(sm, gaux, AUX_NV, bar);
-    int i = 0, j = 0, k = 0;
-    const bool act = pml_cell<SLAB>(D, s, t0 + l, i, j, k);
-    T d = 1, rl = 0, xx0 = 0, xx1 = 0, xy0 = 0, xy1 = 0, xz0 = 0, xz1 = 0, xz2 = 0, yz0 = 0, yz1 = 0, zz0 = 0, zz1 = 0;
-    T xy2 = 0, yy0 = 0, yy1 = 0, yz2 = 0, vold = 0;
-    Damp<T> ox{}, oxS{}, oy{}, oz{};
-    long long p = 0;
-    bool dov = false;
-    const long long sy = g.px, sz = g.plane;
-    if (act) {  // field loads overlap the staging copy
-        const Strip& S = D.s[s];
-        if (MX != SPLIT_NEVER) { ox = X.prof[S.ox_off + i - S.nxb]; oxS = X.prof[S.oxS_off + i - S.nxb]; }
-        if (MY != SPLIT_NEVER) oy = X.prof[S.oy_off + j - S.nyb];
-        if (MZ != SPLIT_NEVER) oz = X.prof[S.oz_off + k - S.nzb];
-        p = g.at(i, j, k);
-        dov = (j <= S.nye);
-        if (f.lay) rl = f.lay[4 * g.nzt + k - 1];  // dt/d of the plane (1-D medium)
-        else d = f.d[p];
+// The x strips' rows are nabc-1 cells, one of them (the outermost) alone in its 32-byte sector:
+// a store of 4 bytes that the L2 has to merge with the rest of the sector from memory, a third of
+// the stress sweep's time at 18 M cells.  The rest of that sector is the boundary cell (i = 1 or
+// nxt, which nothing updates) and the row's padding, both 0: the strip's other lanes store
+// the zeros, so the sector is written whole.  o: the field; returns the element of this lane
+// (i2 cells into the strip), or -1.
+template <class T>
+__device__ __forceinline__ int pml_sector_rest(const Grid& g, const Strip& S, int i2) {
+    constexpr int N = 32 / (int)sizeof(T);
+    if (S.nxb == 2) {
+        const int e = g.off + 1, q = (e & ~(N - 1)) + i2;
+        return q < e ? q : -1;
+    }
+    const int e = g.off + S.nxe - 1, q = e + 1 + i2;
+    return q <= (e | (N - 1)) ? q : -1;
+}
+
+// inputs of a velocity cell, loaded while its split components fly
+template <class T, int C>
+struct VelPmlIn {
+    T xx0, xx1, xy0, xy1, xy2, xz0, xz1, xz2, yz0, yz1, yz2, yy0, yy1, zz0, zz1, r;  // r = dt / d
+    Damp<T> ox, oxS, oy, oz;
+    __device__ __forceinline__ void load(const Grid& g, const Fields<T>& f, const PmlAux<T>& X, const StepConst<T>& c,
+                                         const Strip& S, int i, int j, int k, bool wx, bool wy) {
+        const long long p = g.at(i, j, k), sy = g.px, sz = g.plane;
+        const int i2 = i - S.nxb, j2 = j - S.nyb, k2 = k - S.nzb;
+        if (f.lay) r = f.lay[4 * g.nzt + k - 1];  // dt/d of the plane (1-D medium)
+        else r = f.d[p];
         xx0 = f.xx[p]; xx1 = f.xx[p - 1]; xy0 = f.xy[p]; xy1 = f.xy[p - sy]; xz0 = f.xz[p]; xz1 = f.xz[p - sz];
         xz2 = f.xz[p + 1]; yz0 = f.yz[p]; yz1 = f.yz[p - sy]; zz0 = f.zz[p]; zz1 = f.zz[p + sz];
-        if (dov) {
-            xy2 = f.xy[p + 1]; yy0 = f.yy[p + sy]; yy1 = f.yy[p]; yz2 = f.yz[p - sz];
-            if (j == g.nyt - 1) vold = f.v[p];
+        xy2 = yy0 = yy1 = yz2 = 0;
+        if (j <= S.nye) { xy2 = f.xy[p + 1]; yy0 = f.yy[p + sy]; yy1 = f.yy[p]; yz2 = f.yz[p - sz]; }
+        constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
+        ox = oxS = oy = oz = Damp<T>{1, 1, 1, 0};
+        if (MX == SPLIT_ALWAYS || (MX == SPLIT_MAYBE && wx)) { ox = X.prof[S.ox_off + i2]; oxS = X.prof[S.oxS_off + i2]; }
+        if (MY == SPLIT_ALWAYS || (MY == SPLIT_MAYBE && wy)) oy = X.prof[S.oy_off + j2];
+        if (MZ == SPLIT_ALWAYS) oz = X.prof[S.oz_off + k2];
+        if (!f.lay) r = c.dt / r;
+    }
+};
+
+// pml_uvw at one cell of strip S (fd3d_deriv.f90:1927-2293); a: its first split component in
+// shared memory.  Returns HOW, or the form that the cell needs, with nothing stored.
+template <class T, int C, int HOW>
+__device__ __forceinline__ int vel_pml_cell(const Grid& g, const Fields<T>& f, const StepConst<T>& c, const Strip& S,
+                                            const VelPmlIn<T, C>& q, const T* a, T* ga, int i, int j,
+                                            int k, bool wx, bool wy) {
+    constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
+    const bool dov = j <= S.nye;
+    // p = (p*(1 - omega) + (dt/d)*diff/dh) / (1 + omega), every division rounded as IEEE
+    PmlDiv<T, HOW> dv{c};
+    const T r = dv.scaled(q.r);
+    auto inc = [&](T diff) { return dv.by_dh(r * diff); };
+    auto at = [&](int n) { return a[32 * n]; };
+    auto put = [&](int n) -> T& { return ga[32 * n]; };
+    const T u0 = dv.template split<MX>(at(AX_U0), inc(q.xx0 - q.xx1), q.ox, wx);
+    const T u1 = dv.template split<MY>(at(AX_U1), inc(q.xy0 - q.xy1), q.oy, wy);
+    const T u2 = dv.template split<MZ>(at(AX_U2), inc(q.xz0 - q.xz1), q.oz, true);
+    const T w0 = dv.template split<MX>(at(AX_W0), inc(q.xz2 - q.xz0), q.oxS, wx);
+    const T w1 = dv.template split<MY>(at(AX_W1), inc(q.yz0 - q.yz1), q.oy, wy);
+    const T w2 = dv.template split<MZ>(at(AX_W2), inc(q.zz1 - q.zz0), q.oz, true);
+    // (on the fault row, which has no v: the components are 0 and stay so)
+    const T v0 = dv.template split<MX>(at(AX_V0), inc(q.xy2 - (dov ? q.xy0 : (T)0)), q.oxS, wx);
+    const T v1 = dv.template split<MY>(at(AX_V1), inc(q.yy0 - q.yy1), q.oy, wy);
+    const T v2 = dv.template split<MZ>(at(AX_V2), inc((dov ? q.yz0 : (T)0) - q.yz2), q.oz, true);
+    const T u = u0 + u1 + u2, w = w0 + w1 + w2, v = v0 + v1 + v2;
+    if constexpr (HOW == DIV_FAST) {
+        if (c.pml_exact || !pml_finite(fabsf(u) + fabsf(v) + fabsf(w))) return DIV_FULL;
+        if (dv.key < DIV_KEY) return DIV_TINY;
+    }
+    put(AX_U0) = u0; put(AX_U1) = u1; put(AX_U2) = u2; put(AX_W0) = w0; put(AX_W1) = w1; put(AX_W2) = w2;
+    const long long p = g.at(i, j, k), sy = g.px;
+    f.u[p] = u;
+    f.w[p] = w;
+    if (dov) {
+        put(AX_V0) = v0; put(AX_V1) = v1; put(AX_V2) = v2;
+        if (j == g.nyt - 1) f.v[p + sy] = f.v[p];  // bnd2d mirror of the value before this update
+        f.v[p] = v;
+    }
+    if (C == 0) {
+        const int e = pml_sector_rest<T>(g, S, i - S.nxb);
+        if (e >= 0) {
+            const long long z = p - (g.off + i - 1) + e;
+            f.u[z] = (T)0;
+            f.w[z] = (T)0;
+            if (dov) f.v[z] = (T)0;
         }
     }
+    return HOW;
+}
+
+// The cells that need the full form, out of line.
+template <class T, int C>
+__device__ __noinline__ void vel_pml_redo(const Grid* g, const Fields<T>* f, const PmlAux<T>* X, const StepConst<T>* c,
+                                          const Strip* S, const T* a, T* ga, int i, int j, int k, bool wx, bool wy) {
+    VelPmlIn<T, C> q;
+    q.load(*g, *f, *X, *c, *S, i, j, k, wx, wy);
+    vel_pml_cell<T, C, DIV_FULL>(*g, *f, *c, *S, q, a, ga, i, j, k, wx, wy);
+}
+
+// pml_uvw in one tile of strip class C, one cell per thread.  false if the copy timed out.
+template <class T, int C, bool SLAB, bool REUSED>
+__device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
+                                               const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar,
+                                               uint32_t parity, int* status) {
+    constexpr uint32_t BYTES = PML_TILE * AUX_NV * sizeof(T);
+    pml_tile_begin<REUSED>(smem_addr(sm), X.vel + t0 * AUX_NV, BYTES, bar);
+    const Strip& S = D.s[s];
+    const int l = threadIdx.y * blockDim.x + threadIdx.x;
+    int i = 0, j = 0, k = 0;
+    bool wx, wy;
+    const bool act = pml_cell<SLAB>(D, s, t0 + l, i, j, k);
+    pml_damped<C>(g, S, act, i, j, wx, wy);
+    VelPmlIn<T, C> q;
+    // (the persistent kernel has no registers to hold the inputs across the wait)
+    if (!REUSED && act) q.load(g, f, X, c, S, i, j, k, wx, wy);
+    if (!REUSED) __syncthreads();  // the barrier is initialised
     if (!pml_tile_wait(bar, parity, status)) return false;
-    // warp-uniform: does any cell of this warp lie where the direction is damped?
-    const bool wx = MX == SPLIT_MAYBE && __any_sync(0xffffffffu, ox.o != (T)0 || oxS.o != (T)0);
-    const bool wy = MY == SPLIT_MAYBE && __any_sync(0xffffffffu, oy.o != (T)0);
+    if (REUSED && act) q.load(g, f, X, c, S, i, j, k, wx, wy);
     if (act) {
-        const T dt = c.dt, dh = c.dh, rdh = c.rdh;
-        const T r = f.lay ? rl : dt / d;
-        // p = (p*(1 - omega) + (dt/d)*diff/dh) / (1 + omega), every division rounded as IEEE.
-        // The result goes straight back to the component's global slot (one coalesced
-        // 128-byte row per warp and component), so no bulk store has to drain.
-        auto inc = [&](T diff) { return div_pre(r * diff, dh, rdh); };
-        auto put = [&](int comp, T a) { gaux[aux_sm(l, AUX_NV, comp)] = a; return a; };
-        auto aux = [&](int comp) { return sm[aux_sm(l, AUX_NV, comp)]; };
-        const T u0 = put(AX_U0, pml_split<T, MX>(aux(AX_U0), inc(xx0 - xx1), ox, wx));
-        const T u1 = put(AX_U1, pml_split<T, MY>(aux(AX_U1), inc(xy0 - xy1), oy, wy));
-        const T u2 = put(AX_U2, pml_split<T, MZ>(aux(AX_U2), inc(xz0 - xz1), oz, false));
-        const T w0 = put(AX_W0, pml_split<T, MX>(aux(AX_W0), inc(xz2 - xz0), oxS, wx));
-        const T w1 = put(AX_W1, pml_split<T, MY>(aux(AX_W1), inc(yz0 - yz1), oy, wy));
-        const T w2 = put(AX_W2, pml_split<T, MZ>(aux(AX_W2), inc(zz1 - zz0), oz, false));
-        f.u[p] = u0 + u1 + u2;
-        f.w[p] = w0 + w1 + w2;
-        if (dov) {
-            const T v0 = put(AX_V0, pml_split<T, MX>(aux(AX_V0), inc(xy2 - xy0), oxS, wx));
-            const T v1 = put(AX_V1, pml_split<T, MY>(aux(AX_V1), inc(yy0 - yy1), oy, wy));
-            const T v2 = put(AX_V2, pml_split<T, MZ>(aux(AX_V2), inc(yz0 - yz2), oz, false));
-            if (j == g.nyt - 1) f.v[p + sy] = vold;  // bnd2d mirror of the value before this update
-            f.v[p] = v0 + v1 + v2;
+        const T* a = sm + aux_at(l, AUX_NV);
+        T* ga = X.vel + aux_at(t0 + l, AUX_NV);
+        constexpr int HOW = sizeof(T) == 8 ? DIV_FULL : DIV_FAST;
+        const int how = vel_pml_cell<T, C, HOW>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+        if constexpr (HOW == DIV_FAST) {
+            if (how == DIV_TINY) {  // the same again: nothing is stored yet
+                asm volatile("" ::: "memory");  // (the inputs are loaded anew, not kept in registers)
+                q.load(g, f, X, c, S, i, j, k, wx, wy);
+                vel_pml_cell<T, C, DIV_TINY>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+            } else if (how == DIV_FULL) {
+                vel_pml_redo<T, C>(&g, &f, &X, &c, &S, a, ga, i, j, k, wx, wy);
+            }
         }
     }
     return true;
 }
 
-// pml_uvw: split-field PML velocity in the strips (fd3d_deriv.f90:1927-2293), one
-// tile of PML_TILE consecutive cells per CTA of PML_TILE threads.  Returns false if the
-// staging copy timed out.
-template <class T, bool SLAB = false>
+// pml_uvw: split-field PML velocity in the strips (fd3d_deriv.f90:1927-2293), one tile of
+// PML_TILE consecutive cells per CTA (a tile lies in one strip).
+template <class T, bool SLAB, bool REUSED>
 __device__ __forceinline__ bool vel_pml_tile(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
                                              const StepConst<T>& c, int tile, T* sm, uint32_t bar, uint32_t parity,
                                              int* status) {
     const long long t0 = (long long)tile * PML_TILE;
     const int s = pml_tile_strip(D, t0);
     switch (pml_class(s)) {
-        case 0: return vel_pml_tile_c<T, 0, SLAB>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        case 1: return vel_pml_tile_c<T, 1, SLAB>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        default: return vel_pml_tile_c<T, 2, SLAB>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        case 0: return vel_pml_tile_c<T, 0, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        case 1: return vel_pml_tile_c<T, 1, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        default: return vel_pml_tile_c<T, 2, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
     }
 }
 
@@ -485,110 +614,175 @@ __device__ __forceinline__ void str_fault_body(Grid g, Fields<T> f, Fault<T> q, 
     }
 }
 
-// pml_xyz in one tile of strip class C (fd3d_deriv.f90:2304-3143), as vel_pml_tile_c
-template <class T, int C, bool SLAB>
-__device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D,
-                                               const PmlAux<T>& X, const StepConst<T>& c, int s, long long t0, T* sm,
-                                               uint32_t bar, uint32_t parity, int* status) {
-    constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
-    const int l = threadIdx.y * blockDim.x + threadIdx.x;
-    T* gaux = X.str + t0 * AUX_NS;
-    pml_tile_begin(sm, gaux, AUX_NS, bar);
-    int i = 0, j = 0, k = 0;
-    const bool act = pml_cell<SLAB>(D, s, t0 + l, i, j, k);
-    long long p = 0;
-    bool dxy = false, top = false;
-    const long long sy = g.px, sz = g.plane;
-    T xl = 0, xm = 0, mz = 0, up = 0, ux = 0, uz = 0, vp = 0, vy = 0, wp = 0, wz = 0, wx = 0;
-    T my = 0, md = 0, uy = 0, vx = 0, vz = 0, wy = 0, xyo = 0, yzo = 0;
-    // xy and yz take omegayS in strips 3-5 and xz, yz omegazS in strips 4-5; in the other
-    // strips those directions are undamped (SPLIT_NEVER), so oyS / ozS serve every class
-    Damp<T> ox{}, oxS{}, oy{}, oyS{}, oz{}, ozS{};
-    if (act) {  // field loads overlap the staging copy
-        const Strip& S = D.s[s];
+// inputs of a stress cell
+template <class T, int C>
+struct StrPmlIn {
+    T up, ux, uy, uz, vp, vx, vy, vz, wp, wx, wy, wz, xl, xm, my, mz, md;
+    Damp<T> ox, oxS, oy, oyS, oz, ozS;
+    __device__ __forceinline__ void load(const Grid& g, const Fields<T>& f, const PmlAux<T>& X, const Strip& S, int i,
+                                         int j, int k, bool damped_x, bool damped_y) {
+        const long long p = g.at(i, j, k), sy = g.px, sz = g.plane;
         const int i2 = i - S.nxb, j2 = j - S.nyb, k2 = k - S.nzb;
-        if (MX != SPLIT_NEVER) { ox = X.prof[S.ox_off + i2]; oxS = X.prof[S.oxS_off + i2]; }
-        if (MY != SPLIT_NEVER) { oy = X.prof[S.oy_off + j2]; oyS = X.prof[S.oyS_off + j2]; }
-        if (MZ != SPLIT_NEVER) { oz = X.prof[S.oz_off + k2]; ozS = X.prof[S.ozS_off + k2]; }
-        p = g.at(i, j, k);
-        dxy = (j <= S.nye);
-        top = !g.fspace && (C <= 1) && (k == S.nze);  // xz/yz aux zeroed at the top row, strips 1-3 (not FSPACE)
+        const bool dxy = j <= S.nye;
+        my = md = uy = vx = vz = wy = 0;
         if (f.lay) {  // 1-D medium: mu(i,j+1,k) = mu(i,j,k), mu(i+1,j+1,k+1) = mu(i,j,k+1)
             xl = f.lay[k - 1]; xm = f.lay[g.nzt + k - 1]; mz = f.lay[g.nzt + k];
+            my = xm; md = mz;
         } else {
             xl = f.lam[p]; xm = f.mu[p]; mz = f.mu[p + sz];
+            if (dxy) { my = f.mu[p + sy]; md = f.mu[p + 1 + sy + sz]; }
         }
-        up = f.u[p]; ux = f.u[p + 1]; uz = f.u[p + sz];
-        vp = f.v[p]; vy = f.v[p - sy];
+        up = f.u[p]; ux = f.u[p + 1]; uz = f.u[p + sz]; vp = f.v[p]; vy = f.v[p - sy];
         wp = f.w[p]; wz = f.w[p - sz]; wx = f.w[p - 1];
-        if (dxy) {
-            if (f.lay) { my = xm; md = mz; }
-            else { my = f.mu[p + sy]; md = f.mu[p + 1 + sy + sz]; }
-            uy = f.u[p + sy]; vx = f.v[p - 1]; vz = f.v[p + sz]; wy = f.w[p + sy];
+        if (dxy) { uy = f.u[p + sy]; vx = f.v[p - 1]; vz = f.v[p + sz]; wy = f.w[p + sy]; }
+        // xy and yz take omegayS in strips 3-5 and xz, yz omegazS in strips 4-5; in the other
+        // strips those directions are undamped (SPLIT_NEVER), so oyS / ozS serve every class
+        constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
+        ox = oxS = oy = oyS = oz = ozS = Damp<T>{1, 1, 1, 0};
+        if (MX == SPLIT_ALWAYS || (MX == SPLIT_MAYBE && damped_x)) { ox = X.prof[S.ox_off + i2]; oxS = X.prof[S.oxS_off + i2]; }
+        if (MY == SPLIT_ALWAYS || (MY == SPLIT_MAYBE && damped_y)) { oy = X.prof[S.oy_off + j2]; oyS = X.prof[S.oyS_off + j2]; }
+        if (MZ == SPLIT_ALWAYS) { oz = X.prof[S.oz_off + k2]; ozS = X.prof[S.ozS_off + k2]; }
+    }
+};
+
+// pml_xyz at one cell of a strip (fd3d_deriv.f90:2304-3143), as vel_pml_cell; free_top: the
+// strip's xz and yz components are zeroed at its top row (strips 1-3, not FSPACE)
+template <class T, int C, int HOW>
+__device__ __forceinline__ int str_pml_cell(const Grid& g, const Fields<T>& f, const StepConst<T>& c, const Strip& S,
+                                            bool free_top, const StrPmlIn<T, C>& q, const T* a, T* ga, int i, int j,
+                                            int k, bool wx, bool wy) {
+    constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
+    const bool dxy = j <= S.nye;
+    // p = (p*(1 - omega) + dt*modulus*diff/dh) / (1 + omega), every division rounded as IEEE
+    PmlDiv<T, HOW> dv{c};
+    auto at = [&](int comp) { return a[32 * (comp - AUX_NV)]; };
+    auto put = [&](int comp) -> T& { return ga[32 * (comp - AUX_NV)]; };
+    const T dt = c.dt;
+    const T ma = dv.scaled(dt * (q.xl + (T)2 * q.xm)), mb = dv.scaled(dt * q.xl);
+    // the six products of the normal stresses
+    const T diff1 = q.ux - q.up, diff2 = q.vp - q.vy, diff3 = q.wp - q.wz;
+    const T qa1 = dv.by_dh(ma * diff1), qb1 = dv.by_dh(mb * diff1);
+    const T x0 = dv.template split<MX>(at(AX_XX0), qa1, q.oxS, wx);
+    const T y0 = dv.template split<MX>(at(AX_YY0), qb1, q.oxS, wx);
+    const T z0 = dv.template split<MX>(at(AX_ZZ0), qb1, q.oxS, wx);
+    const T qa2 = dv.by_dh(ma * diff2), qb2 = dv.by_dh(mb * diff2);
+    const T x1 = dv.template split<MY>(at(AX_XX1), qb2, q.oy, wy);
+    const T y1 = dv.template split<MY>(at(AX_YY1), qa2, q.oy, wy);
+    const T z1 = dv.template split<MY>(at(AX_ZZ1), qb2, q.oy, wy);
+    const T qa3 = dv.by_dh(ma * diff3), qb3 = dv.by_dh(mb * diff3);
+    const T x2 = dv.template split<MZ>(at(AX_XX2), qb3, q.oz, true);
+    const T y2 = dv.template split<MZ>(at(AX_YY2), qb3, q.oz, true);
+    const T z2 = dv.template split<MZ>(at(AX_ZZ2), qa3, q.oz, true);
+    const T xx = x0 + x1 + x2, yy = y0 + y1 + y2, zz = z0 + z1 + z2;
+    const T mxz = dv.scaled(dt * ((q.xm + q.mz) / (T)2));
+    T q0 = dv.template split<MZ>(at(AX_XZ0), dv.by_dh(mxz * (q.uz - q.up)), q.ozS, true);
+    T q1 = dv.template split<MX>(at(AX_XZ1), dv.by_dh(mxz * (q.wp - q.wx)), q.ox, wx);
+    const T xz = q0 + q1;
+    T e0 = 0, e1 = 0, h0 = 0, h1 = 0;
+    if (dxy) {
+        const T mxy = dv.scaled(dt * ((q.xm + q.my) / (T)2)), myz = dv.scaled(dt * ((q.xm + q.md) / (T)2));
+        e0 = dv.template split<MY>(at(AX_XY0), dv.by_dh(mxy * (q.uy - q.up)), q.oyS, wy);
+        e1 = dv.template split<MX>(at(AX_XY1), dv.by_dh(mxy * (q.vp - q.vx)), q.ox, wx);
+        h0 = dv.template split<MZ>(at(AX_YZ0), dv.by_dh(myz * (q.vz - q.vp)), q.ozS, true);
+        h1 = dv.template split<MY>(at(AX_YZ1), dv.by_dh(myz * (q.wy - q.wp)), q.oyS, wy);
+    }
+    const T xy = e0 + e1, yz = h0 + h1;
+    if constexpr (HOW == DIV_FAST) {
+        if (c.pml_exact || !pml_finite(fabsf(xx) + fabsf(yy) + fabsf(zz) + fabsf(xy) + fabsf(xz) + fabsf(yz)))
+            return DIV_FULL;
+        if (dv.key < DIV_KEY) return DIV_TINY;
+    }
+    if (free_top && k == S.nze) q0 = q1 = h0 = h1 = (T)0;
+    put(AX_XX0) = x0; put(AX_XX1) = x1; put(AX_XX2) = x2; put(AX_YY0) = y0; put(AX_YY1) = y1; put(AX_YY2) = y2;
+    put(AX_ZZ0) = z0; put(AX_ZZ1) = z1; put(AX_ZZ2) = z2; put(AX_XZ0) = q0; put(AX_XZ1) = q1;
+    const long long p = g.at(i, j, k), sy = g.px;
+    f.xx[p] = xx;
+    f.yy[p] = yy;
+    f.zz[p] = zz;
+    f.xz[p] = xz;
+    if (dxy) {
+        put(AX_XY0) = e0; put(AX_XY1) = e1; put(AX_YZ0) = h0; put(AX_YZ1) = h1;
+        if (j == g.nyt - 1) {  // strbnd mirror of the values before this update
+            f.xy[p + sy] = f.xy[p];
+            f.yz[p + sy] = f.yz[p];
+        }
+        f.xy[p] = xy;
+        f.yz[p] = yz;
+    }
+    if (C == 0) {
+        const int e = pml_sector_rest<T>(g, S, i - S.nxb);
+        if (e >= 0) {
+            const long long z = p - (g.off + i - 1) + e;
+            f.xx[z] = (T)0;
+            f.yy[z] = (T)0;
+            f.zz[z] = (T)0;
+            f.xz[z] = (T)0;
+            if (dxy) {
+                f.xy[z] = (T)0;
+                f.yz[z] = (T)0;
+            }
         }
     }
+    return HOW;
+}
+
+template <class T, int C>
+__device__ __noinline__ void str_pml_redo(const Grid* g, const Fields<T>* f, const PmlAux<T>* X, const StepConst<T>* c,
+                                          const Strip* S, bool free_top, const T* a, T* ga, int i, int j, int k,
+                                          bool wx, bool wy) {
+    StrPmlIn<T, C> q;
+    q.load(*g, *f, *X, *S, i, j, k, wx, wy);
+    str_pml_cell<T, C, DIV_FULL>(*g, *f, *c, *S, free_top, q, a, ga, i, j, k, wx, wy);
+}
+
+template <class T, int C, bool SLAB, bool REUSED>
+__device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
+                                               const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar,
+                                               uint32_t parity, int* status) {
+    constexpr uint32_t BYTES = PML_TILE * AUX_NS * sizeof(T);
+    pml_tile_begin<REUSED>(smem_addr(sm), X.str + t0 * AUX_NS, BYTES, bar);
+    const Strip& S = D.s[s];
+    const bool free_top = C <= 1 && !g.fspace;
+    const int l = threadIdx.y * blockDim.x + threadIdx.x;
+    int i = 0, j = 0, k = 0;
+    bool wx, wy;
+    const bool act = pml_cell<SLAB>(D, s, t0 + l, i, j, k);
+    pml_damped<C>(g, S, act, i, j, wx, wy);
+    StrPmlIn<T, C> q;
+    // (the persistent kernel has no registers to hold the inputs across the wait)
+    if (!REUSED && act) q.load(g, f, X, S, i, j, k, wx, wy);
+    if (!REUSED) __syncthreads();  // the barrier is initialised
     if (!pml_tile_wait(bar, parity, status)) return false;
-    const bool dx = MX == SPLIT_MAYBE && __any_sync(0xffffffffu, ox.o != (T)0 || oxS.o != (T)0);
-    const bool dy = MY == SPLIT_MAYBE && __any_sync(0xffffffffu, oy.o != (T)0 || oyS.o != (T)0);
+    if (REUSED && act) q.load(g, f, X, S, i, j, k, wx, wy);
     if (act) {
-        const T dt = c.dt, dh = c.dh, rdh = c.rdh;
-        const T a = xl + (T)2 * xm, b = xl;
-        const T diff1 = ux - up, diff2 = vp - vy, diff3 = wp - wz;
-        // p = (p*(1 - omega) + dt*modulus*diff/dh) / (1 + omega), every division rounded as IEEE
-        auto inc = [&](T mod, T diff) { return div_pre(dt * mod * diff, dh, rdh); };
-        auto aux = [&](int comp) { return sm[aux_sm(l, AUX_NS, comp - AUX_NV)]; };
-        auto put = [&](int comp, T v) { gaux[aux_sm(l, AUX_NS, comp - AUX_NV)] = v; return v; };
-        const T x0 = put(AX_XX0, pml_split<T, MX>(aux(AX_XX0), inc(a, diff1), oxS, dx));
-        const T x1 = put(AX_XX1, pml_split<T, MY>(aux(AX_XX1), inc(b, diff2), oy, dy));
-        const T x2 = put(AX_XX2, pml_split<T, MZ>(aux(AX_XX2), inc(b, diff3), oz, false));
-        f.xx[p] = x0 + x1 + x2;
-        const T y0 = put(AX_YY0, pml_split<T, MX>(aux(AX_YY0), inc(b, diff1), oxS, dx));
-        const T y1 = put(AX_YY1, pml_split<T, MY>(aux(AX_YY1), inc(a, diff2), oy, dy));
-        const T y2 = put(AX_YY2, pml_split<T, MZ>(aux(AX_YY2), inc(b, diff3), oz, false));
-        f.yy[p] = y0 + y1 + y2;
-        const T z0 = put(AX_ZZ0, pml_split<T, MX>(aux(AX_ZZ0), inc(b, diff1), oxS, dx));
-        const T z1 = put(AX_ZZ1, pml_split<T, MY>(aux(AX_ZZ1), inc(b, diff2), oy, dy));
-        const T z2 = put(AX_ZZ2, pml_split<T, MZ>(aux(AX_ZZ2), inc(a, diff3), oz, false));
-        f.zz[p] = z0 + z1 + z2;
-        {   // xz (j up to jend_uw)
-            const T xmu = (xm + mz) / (T)2;
-            const T q0 = put(AX_XZ0, pml_split<T, MZ>(aux(AX_XZ0), inc(xmu, uz - up), ozS, false));
-            const T q1 = put(AX_XZ1, pml_split<T, MX>(aux(AX_XZ1), inc(xmu, wp - wx), ox, dx));
-            f.xz[p] = q0 + q1;
-            if (top) { put(AX_XZ0, (T)0); put(AX_XZ1, (T)0); }
-        }
-        if (dxy) {
-            T xmu = (xm + my) / (T)2;
-            const T e0 = put(AX_XY0, pml_split<T, MY>(aux(AX_XY0), inc(xmu, uy - up), oyS, dy));
-            const T e1 = put(AX_XY1, pml_split<T, MX>(aux(AX_XY1), inc(xmu, vp - vx), ox, dx));
-            xmu = (xm + md) / (T)2;
-            const T h0 = put(AX_YZ0, pml_split<T, MZ>(aux(AX_YZ0), inc(xmu, vz - vp), ozS, false));
-            const T h1 = put(AX_YZ1, pml_split<T, MY>(aux(AX_YZ1), inc(xmu, wy - wp), oyS, dy));
-            if (j == g.nyt - 1) {  // strbnd mirror of the values before this update (read here, not
-                xyo = f.xy[p];     // held across the staging wait: four fewer live registers)
-                yzo = f.yz[p];
-                f.xy[p + sy] = xyo;
-                f.yz[p + sy] = yzo;
+        const T* a = sm + aux_at(l, AUX_NS);
+        T* ga = X.str + aux_at(t0 + l, AUX_NS);
+        constexpr int HOW = sizeof(T) == 8 ? DIV_FULL : DIV_FAST;
+        const int how = str_pml_cell<T, C, HOW>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+        if constexpr (HOW == DIV_FAST) {
+            if (how == DIV_TINY) {  // the same again: nothing is stored yet
+                asm volatile("" ::: "memory");  // (the inputs are loaded anew, not kept in registers)
+                q.load(g, f, X, S, i, j, k, wx, wy);
+                str_pml_cell<T, C, DIV_TINY>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+            } else if (how == DIV_FULL) {
+                str_pml_redo<T, C>(&g, &f, &X, &c, &S, free_top, a, ga, i, j, k, wx, wy);
             }
-            f.xy[p] = e0 + e1;
-            f.yz[p] = h0 + h1;
-            if (top) { put(AX_YZ0, (T)0); put(AX_YZ1, (T)0); }
         }
     }
     return true;
 }
 
 // pml_xyz in the strips (fd3d_deriv.f90:2304-3143), one tile per CTA as vel_pml_tile
-template <class T, bool SLAB = false>
+template <class T, bool SLAB, bool REUSED>
 __device__ __forceinline__ bool str_pml_tile(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
                                              const StepConst<T>& c, int tile, T* sm, uint32_t bar, uint32_t parity,
                                              int* status) {
     const long long t0 = (long long)tile * PML_TILE;
     const int s = pml_tile_strip(D, t0);
     switch (pml_class(s)) {
-        case 0: return str_pml_tile_c<T, 0, SLAB>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        case 1: return str_pml_tile_c<T, 1, SLAB>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        default: return str_pml_tile_c<T, 2, SLAB>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        case 0: return str_pml_tile_c<T, 0, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        case 1: return str_pml_tile_c<T, 1, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        default: return str_pml_tile_c<T, 2, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
     }
 }
 
@@ -1160,13 +1354,12 @@ __global__ void k_vel_fault(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c, int
 // One PML tile per CTA of PML_TILE threads.  MINB: CTAs that must fit one SM
 // (register cap); 1 leaves it free.
 template <class T, int MINB = 1, bool SLAB = false>
-__global__ void __launch_bounds__(PML_TILE, MINB) k_vel_pml(Grid g, Fields<T> f, const __grid_constant__ PmlDesc D,
-                                                             const __grid_constant__ PmlAux<T> X, StepConst<T> c,
-                                                             int* status, long long tile0) {
+__global__ void __launch_bounds__(PML_TILE, MINB)
+k_vel_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ PmlDesc D,
+          const __grid_constant__ PmlAux<T> X, const __grid_constant__ StepConst<T> c, int* status, long long tile0) {
     __shared__ __align__(128) T sm[PML_TILE * AUX_NV];
     __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); fence_mbar_init(); }
-    vel_pml_tile<T, SLAB>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), 0u, status);
+    vel_pml_tile<T, SLAB, false>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), 0u, status);
 }
 
 template <class T>
@@ -1180,13 +1373,12 @@ __global__ void k_str_fault(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c) {
 }
 
 template <class T, int MINB = 1, bool SLAB = false>
-__global__ void __launch_bounds__(PML_TILE, MINB) k_str_pml(Grid g, Fields<T> f, const __grid_constant__ PmlDesc D,
-                                                             const __grid_constant__ PmlAux<T> X, StepConst<T> c,
-                                                             int* status, long long tile0) {
+__global__ void __launch_bounds__(PML_TILE, MINB)
+k_str_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ PmlDesc D,
+          const __grid_constant__ PmlAux<T> X, const __grid_constant__ StepConst<T> c, int* status, long long tile0) {
     __shared__ __align__(128) T sm[PML_TILE * AUX_NS];
     __shared__ __align__(8) uint64_t bar;
-    if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); fence_mbar_init(); }
-    str_pml_tile<T, SLAB>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), 0u, status);
+    str_pml_tile<T, SLAB, false>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), 0u, status);
 }
 
 // The tiles of strip s that hold cells of planes klo..khi: [t0, t1) (k is the slowest
@@ -1227,6 +1419,7 @@ inline void launch_pml(bool stress, int minb, cudaStream_t st, const Grid& g, co
         FD3D_PML_CASE(2)
         FD3D_PML_CASE(3)
         FD3D_PML_CASE(4)
+        FD3D_PML_CASE(5)
         default:
             if (stress) k_str_pml<T, 1><<<nblk, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);
             else k_vel_pml<T, 1><<<nblk, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);

@@ -1,29 +1,42 @@
-// fd3d_selftest.cu -- exhaustive device check of div_pre against the IEEE division.
+// fd3d_selftest.cu -- exhaustive device check of the PML quotients against the IEEE division.
 //
-// The PML updates divide by dh and by 1 + omega, divisors known before the launch;
-// div_pre (fd3d_common.cuh) forms those quotients from a host-computed reciprocal.
-// fd3d_check_division runs div_pre and __fdiv_rn on every one of the 2^32 float bit
-// patterns for each divisor given and counts the dividends whose results differ in
-// any bit (two NaNs count as equal).
+// The PML updates divide by dh and by 1 + omega, divisors known before the launch; div_by and
+// div_by_signed (fd3d_common.cuh) form those quotients from a pair made on the host, and
+// div_small and div_exact those they do not cover.  fd3d_check_division runs them, chosen as the
+// sweeps choose them, and __fdiv_rn on every one of the 2^32 float bit patterns for each divisor
+// given and counts the dividends whose results differ in any bit (two NaNs count as equal).
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "../../include/fd3d_gpu.h"
 #include "fd3d_common.cuh"
+#include "fd3d_setup.h"
 
 using namespace fd3d;
 
 namespace {
 
-__global__ void k_check_division(float b, float y, unsigned long long* bad, unsigned* first) {
+struct Pair { float h, l, s; int ok; };
+
+// the sweeps' quotient: div_by on the scaled dividend, or what its key or result asks for
+__device__ float quotient(float x, float b, const Pair& y, bool sign) {
+    unsigned key = 0xffffffffu;
+    const float xs = x * y.s, q = (sign ? div_by_signed(xs, y.h, y.l, key) : div_by(xs, y.h, y.l, key)) * (1.0f / y.s);
+    if (!y.ok || !pml_finite(q)) return div_exact(x, b);
+    return key < DIV_KEY ? div_small(x, b, y.h, y.l) : q;
+}
+
+// y: the pair with l >= 0 (the divisor dh), ys: the pair of any sign (1 + omega)
+__global__ void k_check_division(float b, Pair y, Pair ys, unsigned long long* bad, unsigned* first) {
     const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
     unsigned long long local = 0;
     unsigned ex = 0;
     for (uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; n < (1ull << 32); n += nthreads) {
         const unsigned bits = (unsigned)n;
         const float x = __uint_as_float(bits);
-        const float q = div_pre(x, b, y);
         const float r = __fdiv_rn(x, b);
-        const bool same = (__float_as_uint(q) == __float_as_uint(r)) || (q != q && r != r);
+        auto is = [&](float q) { return (__float_as_uint(q) == __float_as_uint(r)) || (q != q && r != r); };
+        bool same = is(quotient(x, b, y, false)) && is(quotient(x, b, ys, true)) && is(div_exact(x, b));
+        if (ys.ok && pml_finite(x)) same = same && is(div_small(x, b, ys.h, ys.l));
         if (!same) {
             if (local == 0) ex = bits;
             ++local;
@@ -52,14 +65,17 @@ extern "C" int fd3d_check_division(const float* divisors, int n, unsigned long l
     int rc = FD3D_OK;
     for (int i = 0; i < n && rc == FD3D_OK; ++i) {
         const float b = divisors[i];
-        const float y = div_pre_recip(b);
+        Pair y, ys;
+        y.s = ys.s = b > 0 ? (float)div_scale(b) : 1.0f;
+        y.ok = div_pair(b, true, y.h, y.l);
+        ys.ok = div_pair(b, false, ys.h, ys.l);
         const unsigned none = 0xffffffffu;
         if (cudaMemset(dbad, 0, sizeof(unsigned long long)) != cudaSuccess ||
             cudaMemcpy(dfirst, &none, sizeof(unsigned), cudaMemcpyHostToDevice) != cudaSuccess) {
             rc = FD3D_ERR_CUDA;
             break;
         }
-        k_check_division<<<nsm * 8, 256>>>(b, y, dbad, dfirst);
+        k_check_division<<<nsm * 8, 256>>>(b, y, ys, dbad, dfirst);
         unsigned long long hb = 0;
         unsigned hf = none;
         if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||

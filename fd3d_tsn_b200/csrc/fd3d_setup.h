@@ -3,6 +3,8 @@
 // per-step scalars in the field type.
 #pragma once
 #include <algorithm>
+#include <cmath>
+#include <cstdint>
 #include <vector>
 #include "../../include/fd3d_gpu.h"
 #include "fd3d_common.cuh"
@@ -67,6 +69,76 @@ inline bool slab_range_ok(const fd3d_params& p, int klo, int khi) {
     if (khi < p.nzt && khi >= ks - 2) return false;  // the slab above would not own ks-2 .. nzt
     return true;
 }
+
+// The pair (h, l) of div_by for the divisor b: see there for the method.  With b's significand
+// Y and x's significand X as integers in [2^23, 2^24), x/b sits at a midpoint up to
+// R / (Y (2Q+1)) relative, where 2^s X = Y (2Q+1) + R (s = 24 if X >= Y, else 25).  The error
+// of the sum is at most 6*2^-48 (h nearest to 1/b, l within two units of 1/b - h), |R| <= 12, or
+// 36*2^-48 (h up to three units below 1/b), |R| <= 72; RM is a little above that.  For each R
+// the X that satisfy the congruence are a residue class mod Y, a few values at most.
+inline bool div_pair_holds(float b, float h, float l, int64_t RM) {
+    int e;
+    const uint64_t Y = (uint64_t)std::ldexp((double)std::frexp(b, &e), 24);
+    int t = 0;
+    while (!((Y >> t) & 1)) ++t;
+    const int64_t Yo = (int64_t)(Y >> t);
+    if (Yo == 1) return l == 0x1p-149f;  // a power of two: x*h is exact, l only keeps x*l finite
+    for (int s = 24; s <= 25; ++s) {
+        int64_t p2 = 1;  // 2^(s-t) mod Yo and its inverse
+        for (int k = 0; k < s - t; ++k) p2 = p2 * 2 % Yo;
+        int64_t t0 = 0, t1 = 1, r0 = Yo, r1 = p2;
+        while (r1) {
+            const int64_t q = r0 / r1;
+            int64_t x = t0 - q * t1; t0 = t1; t1 = x;
+            x = r0 - q * r1; r0 = r1; r1 = x;
+        }
+        const int64_t inv = (t0 % Yo + Yo) % Yo;
+        for (int64_t R = -RM; R <= RM; ++R) {
+            if (R == 0 || R % ((int64_t)1 << t) != 0) continue;
+            const int64_t Rm = ((R >> t) % Yo + Yo) % Yo;
+            const int64_t lo = (int64_t)1 << 23;
+            int64_t X = inv * Rm % Yo;  // both below 2^24
+            if (X < lo) X += (lo - X + Yo - 1) / Yo * Yo;
+            for (; X < 2 * lo; X += Yo) {
+                if ((s == 24) != (X >= (int64_t)Y)) continue;
+                const float x = (float)X, xl = x * l;
+                if (std::fmaf(x, h, xl) != x / b) return false;
+                // the sum's distance from the midpoint next to it must be more than what an
+                // underflow of x*l could add for |x| >= 2^-70 (2^-66 relative)
+                const double q = (double)x / (double)b;
+                int qe;
+                std::frexp(q, &qe);
+                const double unit = std::ldexp(1.0, qe - 25);  // half a unit in the last place
+                const double mid = (2.0 * std::floor(q / unit / 2.0) + 1.0) * unit;
+                const double d = ((double)x * (double)h - mid) + (double)xl;
+                if (std::fabs(d) < std::ldexp(q, -57)) return false;
+            }
+        }
+    }
+    return true;
+}
+// nonneg: only pairs with l >= 0 (the sign of a zero dividend is kept without more work).
+// false: no pair found (or b out of range); the sweeps use div_exact then.
+inline bool div_pair(float b, bool nonneg, float& h, float& l) {
+    h = l = 0.f;
+    if (!(b >= 0x1p-20f && b <= 0x1p20f)) return false;
+    const double z = 1.0 / (double)b;
+    h = (float)z;
+    if (nonneg && (double)h > z) h = std::nextafterf(h, 0.f);
+    for (int k = 0; k < (nonneg ? 3 : 1); ++k, h = std::nextafterf(h, 0.f)) {
+        const float l0 = (float)(std::fma(-(double)b, (double)h, 1.0) / (double)b);
+        for (int o = 0; o < 5; ++o) {  // the nearest l, then up to two units either way
+            l = l0 == 0.f ? 0x1p-149f : l0;
+            for (int u = 0; u < (o + 1) / 2; ++u) l = std::nextafterf(l, (o & 1) ? INFINITY : -INFINITY);
+            if (div_pair_holds(b, h, l, nonneg ? 80 : 16)) return true;
+        }
+    }
+    return false;
+}
+inline bool div_pair(double, bool, double& h, double& l) { h = l = 0; return true; }  // divides directly
+// The scale of div_by's dividends for divisors up to b: a scaled dividend of 2^-70 or more has a
+// quotient by b that is a normal number when it is scaled back, 2^-70 / S / b >= 2^-126.
+inline double div_scale(double b) { return std::ldexp(1.0, std::min(56, 56 - (int)std::ceil(std::log2(b)))); }
 
 // init_pml (fd3d_deriv.f90:1319-1493): strip boxes and damping profiles, in T.
 template <class T>
@@ -136,16 +208,29 @@ void make_pml(const fd3d_params& p, PmlDesc& D, std::vector<Damp<T>>& prof) {
             oyS[4][i - 1] = omRM[i - 1];
         }
     }
+    for (int s = 0; s <= PML_MAXS; ++s) D.tile0[s] = (int)(D.cum[s] / PML_TILE);
+    std::vector<Damp<T>> pairs;  // the strips share their divisors: one search for each
+    D.exact = 0;
+    D.bmax = 1.0;
     for (int s = 0; s < D.ns; ++s) {
         Strip& S = D.s[s];
         auto put = [&](const std::vector<T>& v) {
             const int o = (int)prof.size();
+            int last = -1;
             for (T om : v) {
                 Damp<T> e;
-                e.o = om;
                 e.m = (T)1 - om;
                 e.p = (T)1 + om;
-                e.r = div_pre_recip(e.p);
+                D.bmax = std::max(D.bmax, (double)e.p);
+                if (last < 0 || pairs[last].p != e.p) {
+                    for (last = 0; last < (int)pairs.size() && pairs[last].p != e.p;) ++last;
+                    if (last == (int)pairs.size()) {
+                        if (!div_pair(e.p, false, e.h, e.l)) D.exact = 1;
+                        pairs.push_back(e);
+                    }
+                }
+                e.h = pairs[last].h;
+                e.l = pairs[last].l;
                 prof.push_back(e);
             }
             return o;
@@ -157,27 +242,34 @@ void make_pml(const fd3d_params& p, PmlDesc& D, std::vector<Damp<T>>& prof) {
 }
 
 // The PML sweeps update a split direction as p + inc where its strip class says the
-// direction is never damped (split_mode, fd3d_kernels.cuh); that is exact only if every
-// omega of that direction's profiles is zero over the strip.  Checked once per set-up.
+// direction is never damped (split_mode, fd3d_kernels.cuh), and where a warp's cells lie
+// outside the damped ends of a SPLIT_MAYBE direction; that is exact only if every omega there
+// is zero.  Checked once per set-up.
 template <class T>
-bool pml_modes_hold(const PmlDesc& D, const std::vector<Damp<T>>& prof) {
+bool pml_modes_hold(const PmlDesc& D, const std::vector<Damp<T>>& prof, int nabc) {
+    const int n = nabc - 1;
     for (int s = 0; s < D.ns; ++s) {
         const Strip& S = D.s[s];
         const int C = pml_class(s);
         const int offs[3][2] = {{S.ox_off, S.oxS_off}, {S.oy_off, S.oyS_off}, {S.oz_off, S.ozS_off}};
         const int len[3] = {S.ni, S.nj1, S.nk};
         for (int dir = 0; dir < 3; ++dir) {
-            if (split_mode(C, dir) != SPLIT_NEVER) continue;
+            const int mode = split_mode(C, dir);
+            if (mode == SPLIT_ALWAYS) continue;
+            const int q0 = mode == SPLIT_NEVER ? 0 : n;
+            const int q1 = mode == SPLIT_MAYBE && dir == 0 ? len[dir] - n : len[dir];
             for (int v = 0; v < 2; ++v)
-                for (int q = 0; q < len[dir]; ++q)
-                    if (prof[(size_t)offs[dir][v] + q].o != (T)0) return false;
+                for (int q = q0; q < q1; ++q) {
+                    const Damp<T>& e = prof[(size_t)offs[dir][v] + q];
+                    if (e.m != (T)1 || e.p != (T)1) return false;
+                }
         }
     }
     return true;
 }
 
 template <class T>
-StepConst<T> make_const(const fd3d_params& p) {
+StepConst<T> make_const(const fd3d_params& p, const PmlDesc& D) {
     StepConst<T> c;
     c.dt = (T)p.dt; c.dh = (T)p.dh;
     c.dth = c.dt / c.dh;
@@ -186,7 +278,10 @@ StepConst<T> make_const(const fd3d_params& p) {
     c.damp_s = (T)p.damp_s;
     c.c1 = (T)9 / (T)8;
     c.c2 = (T)-1 / (T)24;
-    c.rdh = div_pre_recip(c.dh);
+    const double scale = div_scale(std::max(D.bmax, (double)c.dh));
+    c.ds = (T)scale;
+    c.dsi = (T)(1.0 / scale);
+    c.pml_exact = !div_pair(c.dh, true, c.rdh, c.rdl) || D.exact;
     c.dtA = p.dt;
     c.dhA = (double)c.dh;
     c.dthA = c.dtA / c.dhA;
