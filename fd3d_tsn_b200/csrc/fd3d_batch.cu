@@ -177,7 +177,7 @@ k_batch(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
                                                                 ring, bars, pc, gstatus);
                         break;
                     case W_VEL_FAULT:
-                        vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, 0);
+                        vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
                         break;
                     case W_VEL_PML:
                         ok = vel_pml_tile<float, false, true>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(&pbar),
@@ -189,16 +189,16 @@ k_batch(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
                         ok = str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz,
                                                                 ring, bars, pc, gstatus);
                         break;
-                    case W_STR_FAULT: str_fault_body<float>(P.g, P.f, M.q, P.c, it.bx, it.by, 0); break;
+                    case W_STR_FAULT: str_fault_body<float>(P.g, P.f, M.q, P.c, it.bx, it.by, it.bz); break;
                     case W_STR_PML:
                         ok = str_pml_tile<float, false, true>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(&pbar),
                                                              pt & 1u, gstatus);
                         ++pt;
                         break;
-                    case W_STR_FS: str_fs_body<float>(P.g, P.f, it.bx, it.by, 0); break;
+                    case W_STR_FS: str_fs_body<float>(P.g, P.f, 1 + it.bx * 32 + threadIdx.x, 1 + it.by * 8 + threadIdx.y); break;
                     case W_FBC:
-                        fault_bc_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by,
-                                             ring);
+                        fault_bc_body<float, 256>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by,
+                                                  ring, threadIdx.y * 32 + threadIdx.x);
                         break;
                     case W_NUC: nucleation_body<float>(P.g, M.q, P.c, M.fs, M.it_dev, it.bx, it.by, 0); break;
                     default: break;
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict
 // with them, 78 registers), KIND 2 the fault-band velocity (its rate-and-state Newton path
 // takes 114), KIND 0 the rest (free surface, stress fault band, nucleation ramp).
 template <int KIND>
-__global__ void __launch_bounds__(256) k_bplane(const ModelDev* __restrict__ models, const Work* __restrict__ work,
+__global__ void __launch_bounds__(256, KIND == 1 ? 3 : 1) k_bplane(const ModelDev* __restrict__ models, const Work* __restrict__ work,
                                                 int b0, const int* __restrict__ limit, const int* run_step) {
     __shared__ float sm[KIND == 1 ? FBC_SMEM : 1];
     pdl_wait();
@@ -303,20 +303,21 @@ __global__ void __launch_bounds__(256) k_bplane(const ModelDev* __restrict__ mod
     const ModelDev& M = models[m];
     if (KIND == 2) {
         if ((it.tm & 255) == W_VEL_FAULT)
-            vel_fault_body<float>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, 0);
+            vel_fault_body<float>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
         return;
     }
     if (KIND == 1) {
         if ((it.tm & 255) == W_FBC)
-            fault_bc_body<float>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by, sm);
+            fault_bc_body<float, 256>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by, sm,
+                                      threadIdx.y * 32 + threadIdx.x);
         else if ((it.tm & 255) == W_STR_FS)
-            str_fs_body<float>(M.g, M.f, it.bx, it.by, 0);
+            str_fs_body<float>(M.g, M.f, 1 + it.bx * 32 + threadIdx.x, 1 + it.by * 8 + threadIdx.y);
         return;
     }
     switch (it.tm & 255) {
         case W_VEL_FS: vel_fs_body<float>(M.g, M.f, it.bx, it.by, 0); break;
-        case W_STR_FAULT: str_fault_body<float>(M.g, M.f, M.q, M.c, it.bx, it.by, 0); break;
-        case W_STR_FS: str_fs_body<float>(M.g, M.f, it.bx, it.by, 0); break;
+        case W_STR_FAULT: str_fault_body<float>(M.g, M.f, M.q, M.c, it.bx, it.by, it.bz); break;
+        case W_STR_FS: str_fs_body<float>(M.g, M.f, 1 + it.bx * 32 + threadIdx.x, 1 + it.by * 8 + threadIdx.y); break;
         case W_NUC: nucleation_body<float>(M.g, M.q, M.c, M.fs, M.it_dev, it.bx, it.by, 0); break;
         default: break;
     }
@@ -552,7 +553,8 @@ void build_model_items(Model& M, int m, int kch) {
             }
     const int fx = (std::max(nxT, p.nxt) + 31) / 32, fz = (nzT + 7) / 8;
     for (int y = 0; y < fz; ++y)
-        for (int x = 0; x < fx; ++x) per[0].push_back(Work{tm | W_VEL_FAULT, x, y, 0});
+        for (int x = 0; x < fx; ++x)
+            for (int z = 0; z < VEL_FAULT_PARTS; ++z) per[0].push_back(Work{tm | W_VEL_FAULT, x, y, z});
     const int npml = (int)((M.dev.D.cum[PML_MAXS] + PML_TILE - 1) / PML_TILE);
     for (int x = 0; x < npml; ++x) {
         per[0].push_back(Work{tm | W_VEL_PML, x, 0, 0});
@@ -566,10 +568,11 @@ void build_model_items(Model& M, int m, int kch) {
         }
     const int px = (nxT + 31) / 32;
     for (int y = 0; y < fz; ++y)
-        for (int x = 0; x < px; ++x) per[2].push_back(Work{tm | W_STR_FAULT, x, y, 0});
+        for (int x = 0; x < px; ++x)
+            for (int z = 0; z < STR_FAULT_PARTS; ++z) per[2].push_back(Work{tm | W_STR_FAULT, x, y, z});
     {   // fused fault BC tiles (fault_bc_body)
         int nfres, tx, nt;
-        fault_bc_grid(g, nfres, tx, nt);
+        fault_bc_grid(g, 8, nfres, tx, nt);
         for (int t = 0; t < nt; ++t) per[3].push_back(Work{tm | W_FBC, t % tx, t / tx, 0});
     }
     if (M.p.law == FD3D_LAW_FVW && M.dev.fs.nucleation) {

@@ -716,7 +716,7 @@ struct Ctx : CtxBase {
             else launch_vel_interior<T>(icfg, g, f, c, st);
             kend(0);
             kbeg(1);
-            k_vel_fault<T><<<dim3((std::max(nxT, p.nxt) + 31) / 32, (nzT + 7) / 8), b2, 0, sp>>>(g, f, q, c, law, fs, it_dev, status);
+            k_vel_fault<T><<<dim3((std::max(nxT, p.nxt) + 31) / 32, (nzT + 7) / 8, VEL_FAULT_PARTS), b2, 0, sp>>>(g, f, q, c, law, fs, it_dev, status);
             kend(1);
             kbeg(2);
             launch_pml<T>(false, pml_minb_vel, sp, g, f, D, X, c, status);
@@ -733,7 +733,7 @@ struct Ctx : CtxBase {
             else launch_str_interior<T>(icfg, g, f, c, st);
             kend(4);
             kbeg(5);
-            k_str_fault<T><<<dim3((nxT + 31) / 32, (nzT + 7) / 8), b2, 0, sp>>>(g, f, q, c);
+            k_str_fault<T><<<dim3((nxT + 31) / 32, (nzT + 7) / 8, STR_FAULT_PARTS), b2, 0, sp>>>(g, f, q, c);
             kend(5);
             kbeg(6);
             launch_pml<T>(true, pml_minb_str, sp, g, f, D, X, c, status);
@@ -743,9 +743,7 @@ struct Ctx : CtxBase {
         case 2:  // fault boundary condition
             kbeg(7);
             if (!split_bc) {   // fres and the fused trial traction, friction and output tiles in one launch
-                int nfres, tiles_x, tiles;
-                fault_bc_grid(g, nfres, tiles_x, tiles);
-                k_fault_bc<T><<<nfres + tiles, b2, 0, st>>>(g, f, q, c, law, fs, it_dev, h, status, nfres, tiles_x);
+                launch_fault_bc<T>(law, icfg.nsm, st, g, f, q, c, fs, it_dev, h, status);
             } else {           // the same as separate launches, trial tractions in q.txt / q.tzt
                 if (!p.fspace && top) k_str_fs<T><<<dim3((p.nxt + 31) / 32, (p.nyt + 7) / 8), b2, 0, st>>>(g, f);  // fres
                 k_traction<T><<<dim3((nxT + 31) / 32, (nzT + 7) / 8), b2, 0, st>>>(g, f, q, c, it_dev);

@@ -75,53 +75,69 @@ __device__ __forceinline__ double fvw_newton(double vtilde, double cdelta, doubl
     return uw;
 }
 
-// Band j=nyt-1 (2nd order + damping, v mirror) and split-node fault velocity at j=nyt.
+// Band j=nyt-1 (2nd order + damping, v mirror) and split-node fault velocity at j=nyt.  The
+// parts are independent and go to CTAs of their own (bz_): 0 the band (and the step counter), 1
+// u and 2 w on the fault.  Bound by latency on a few hundred CTAs or less, so every part loads
+// all it needs before it stores (a store to one field holds back a load from the next).
+// One launch, us (before: one thread for all parts, each field loaded after the store to the one
+// before): rate-and-state 11 K fault nodes 8.4 (13.8), slip weakening 19 K nodes 4.7 (7.1);
+// the stress band of 11 K nodes 4.1 (8.8).
+constexpr int VEL_FAULT_PARTS = 3;
 template <class T>
-__device__ __forceinline__ void vel_fault_body(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c, int law, FvwScalars s,
-                            int* it_dev, int* status, int bx_, int by_, int bz_) {
+__device__ __forceinline__ void vel_fault_body(const Grid& g, const Fields<T>& f, const Fault<T>& q,
+                                               const StepConst<T>& c, int law, const FvwScalars& s, int* it_dev,
+                                               int* status, int bx_, int by_, int bz_) {
     const int ii = bx_ * blockDim.x + threadIdx.x;
     const int kk = by_ * blockDim.y + threadIdx.y;
-    if (ii == 0 && kk == 0) atomicAdd(it_dev, 1);  // step counter read by the fault BC launches
     const int ks = g.ks();
     const long long sy = g.px, sz = g.plane;
-    // ghost row k=ks+1: v(:,nyt,ks+1) = v(:,nyt-1,ks+1)  (bnd2d mirror, fd3d_deriv.f90:225-232);
-    // under FSPACE that row belongs to the top PML strip, whose tiles mirror it
-    if (!g.fspace && kk == 0 && ii < g.nxt && g.owns(ks + 1)) {
-        const long long p = g.at(ii + 1, g.nyt - 1, ks + 1);
-        f.v[p + sy] = f.v[p];
-    }
     const int i = g.nabc + 1 + ii, k = g.kin_lo() + kk;
-    if (i > g.nxt - g.nabc || k > g.kin_hi()) return;
+    const bool in = i <= g.nxt - g.nabc && k <= g.kin_hi();
     const int n2 = g.at2(i, k);
-    {   // uxx0a / vyy0a / wzz0a  (fd3d_deriv.f90:284-508)
+    if (bz_ == 0) {
+        if (ii == 0 && kk == 0) atomicAdd(it_dev, 1);  // step counter read by the fault BC launches
+        // ghost row k=ks+1: v(:,nyt,ks+1) = v(:,nyt-1,ks+1)  (bnd2d mirror, fd3d_deriv.f90:225-232);
+        // under FSPACE that row belongs to the top PML strip, whose tiles mirror it
+        if (!g.fspace && kk == 0 && ii < g.nxt && g.owns(ks + 1)) {
+            const long long p = g.at(ii + 1, g.nyt - 1, ks + 1);
+            f.v[p + sy] = f.v[p];
+        }
+        if (!in) return;
+        // uxx0a / vyy0a / wzz0a  (fd3d_deriv.f90:284-508)
         const long long p = g.at(i, g.nyt - 1, k);
-        const T r = c.dth / f.d[p];
+        const T d = f.d[p], u = f.u[p], v = f.v[p], w = f.w[p], au1 = q.au1[n2], av1 = q.av1[n2], aw1 = q.aw1[n2];
         const T pdx = (f.xx[p] - f.xx[p - 1]) + (f.xy[p] - f.xy[p - sy]) + (f.xz[p] - f.xz[p - sz]);
-        const T au = pdx - q.au1[n2];
-        f.u[p] = f.u[p] + r * (pdx + c.damp_s * au);
-        q.au1[n2] = pdx;
         const T pdy = (f.xy[p + 1] - f.xy[p]) + (f.yy[p + sy] - f.yy[p]) + (f.yz[p] - f.yz[p - sz]);
-        const T av = pdy - q.av1[n2];
-        const T vn = f.v[p] + r * (pdy + c.damp_s * av);
+        const T pdz = (f.xz[p + 1] - f.xz[p]) + (f.yz[p] - f.yz[p - sy]) + (f.zz[p + sz] - f.zz[p]);
+        const T r = c.dth / d;
+        const T au = pdx - au1, av = pdy - av1, aw = pdz - aw1;
+        const T vn = v + r * (pdy + c.damp_s * av);
+        f.u[p] = u + r * (pdx + c.damp_s * au);
         f.v[p] = vn;
         f.v[p + sy] = vn;  // mirror into the fault plane
+        f.w[p] = w + r * (pdz + c.damp_s * aw);
+        q.au1[n2] = pdx;
         q.av1[n2] = pdy;
-        const T pdz = (f.xz[p + 1] - f.xz[p]) + (f.yz[p] - f.yz[p - sy]) + (f.zz[p + sz] - f.zz[p]);
-        const T aw = pdz - q.aw1[n2];
-        f.w[p] = f.w[p] + r * (pdz + c.damp_s * aw);
         q.aw1[n2] = pdz;
+        return;
     }
+    if (!in) return;
     const long long pf = g.at(i, g.nyt, k);
     if (law == 0) {  // tasu1/tasw1 slip weakening
-        const T r = c.dth / f.d[pf];
-        f.u[pf] = f.u[pf] + r * (T)2 * (q.tx[n2] + q.RFx[n2]);
-        f.w[pf] = f.w[pf] + r * ((T)2 * (q.tz[n2] + q.RFz[n2]));
+        const T d = f.d[pf];
+        if (bz_ == 1) {
+            const T u = f.u[pf], t = q.tx[n2], rf = q.RFx[n2], r = c.dth / d;
+            f.u[pf] = u + r * (T)2 * (t + rf);
+        } else {
+            const T w = f.w[pf], t = q.tz[n2], rf = q.RFz[n2], r = c.dth / d;
+            f.w[pf] = w + r * ((T)2 * (t + rf));
+        }
         return;
     }
     // FVW (fd3d_deriv.f90:1141-1162, 1204-1226), FP64
     const double d = (double)f.d[pf];
     const double rr = c.dthA / d;
-    {
+    if (bz_ == 1) {
         const double u = (double)f.u[pf];
         const double a = (double)q.aX[n2];
         const double s1 = 2.0 * (fabs((double)q.wX[n2]) + fabs(s.wini)), s2 = 2.0 * (fabs(u) + fabs(s.uini));
@@ -136,8 +152,7 @@ __device__ __forceinline__ void vel_fault_body(Grid g, Fields<T> f, Fault<T> q, 
         uw = fvw_newton(vt, cdelta, uw, q.psiX[n2], a, s.v0, status);
         f.u[pf] = (T)(((double)q.tx[n2] + (double)q.T0X[n2]) * (-sinh(uw)) * s.v0 * exp(-q.psiX[n2] / a) /
                       (double)q.tabsX[n2] + s.uini);
-    }
-    {
+    } else {
         const double w = (double)f.w[pf];
         const double a = (double)q.aZ[n2];
         const double s1 = 2.0 * (w - s.wini), s2 = 2.0 * ((double)q.uZ[n2] - s.uini);
@@ -568,49 +583,54 @@ __global__ void __launch_bounds__(256) k_str_interior(Grid g, Fields<T> f, StepC
     }
 }
 
-// Band j=nyt-1 stresses (2nd order) + xy/yz mirror; sxz1 and tasii at j=nyt.
+// Band j=nyt-1 stresses (2nd order) + xy/yz mirror (bz_ = 0); sxz1 and tasii at j=nyt (bz_ = 1):
+// CTAs of their own, loads before stores, as vel_fault_body.
+constexpr int STR_FAULT_PARTS = 2;
 template <class T>
-__device__ __forceinline__ void str_fault_body(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c, int bx_, int by_, int bz_) {
+__device__ __forceinline__ void str_fault_body(const Grid& g, const Fields<T>& f, const Fault<T>& q,
+                                               const StepConst<T>& c, int bx_, int by_, int bz_) {
     const int i = g.nabc + 1 + bx_ * blockDim.x + threadIdx.x;
     const int k = g.kin_lo() + by_ * blockDim.y + threadIdx.y;
     if (i > g.nxt - g.nabc || k > g.kin_hi()) return;
     const long long sy = g.px, sz = g.plane;
     const T dth = c.dth, dth2 = c.dth2, c1 = c.c1, c2 = c.c2;
-    {   // sxx, sxy0, sxz0, syz0 at j=nyt-1 (fd3d_deriv.f90:818-1012)
+    if (bz_ == 0) {   // sxx, sxy0, sxz0, syz0 at j=nyt-1 (fd3d_deriv.f90:818-1012)
         const long long p = g.at(i, g.nyt - 1, k);
-        const T xl = f.lam[p], xm = f.mu[p];
-        const T a = xl + (T)2 * xm, b = xl;
+        const T xl = f.lam[p], xm = f.mu[p], my = f.mu[p + sy], mz = f.mu[p + sz], md = f.mu[p + 1 + sy + sz];
         const T up = f.u[p], vp = f.v[p], wp = f.w[p];
         const T ux = f.u[p + 1], vy = f.v[p - sy], wz = f.w[p - sz];
-        f.xx[p] = f.xx[p] + dth * a * (ux - up) + dth * b * (vp - vy + wp - wz);
-        f.yy[p] = f.yy[p] + dth * a * (vp - vy) + dth * b * (ux - up + wp - wz);
-        f.zz[p] = f.zz[p] + dth * a * (wp - wz) + dth * b * (ux - up + vp - vy);
-        T xmu = xm + f.mu[p + sy];
-        const T xyn = f.xy[p] + dth2 * xmu * (f.u[p + sy] - up + vp - f.v[p - 1]);
+        const T uy = f.u[p + sy], vx = f.v[p - 1], uz = f.u[p + sz], wx = f.w[p - 1], vz = f.v[p + sz], wy = f.w[p + sy];
+        const T xx = f.xx[p], yy = f.yy[p], zz = f.zz[p], xy = f.xy[p], xz = f.xz[p], yz = f.yz[p];
+        const T a = xl + (T)2 * xm, b = xl;
+        f.xx[p] = xx + dth * a * (ux - up) + dth * b * (vp - vy + wp - wz);
+        f.yy[p] = yy + dth * a * (vp - vy) + dth * b * (ux - up + wp - wz);
+        f.zz[p] = zz + dth * a * (wp - wz) + dth * b * (ux - up + vp - vy);
+        T xmu = xm + my;
+        const T xyn = xy + dth2 * xmu * (uy - up + vp - vx);
         f.xy[p] = xyn; f.xy[p + sy] = xyn;
-        xmu = xm + f.mu[p + sz];
-        f.xz[p] = f.xz[p] + dth2 * xmu * (f.u[p + sz] - up + wp - f.w[p - 1]);
-        xmu = xm + f.mu[p + 1 + sy + sz];
-        const T yzn = f.yz[p] + dth2 * xmu * (f.v[p + sz] - vp + f.w[p + sy] - wp);
+        xmu = xm + mz;
+        f.xz[p] = xz + dth2 * xmu * (uz - up + wp - wx);
+        xmu = xm + md;
+        const T yzn = yz + dth2 * xmu * (vz - vp + wy - wp);
         f.yz[p] = yzn; f.yz[p + sy] = yzn;
-    }
-    {   // sxz1 (tasxz) and tasii at j=nyt (fd3d_deriv.f90:677-722, 1263-1314)
+    } else {   // sxz1 (tasxz) and tasii at j=nyt (fd3d_deriv.f90:677-722, 1263-1314)
         const long long p = g.at(i, g.nyt, k);
         const T* u = f.u; const T* w = f.w;
-        T xmu = f.mu[p] + f.mu[p + sz];
-        f.xz[p] = f.xz[p] + dth2 * xmu * (c1 * (u[p + sz] - u[p]) + c2 * (u[p + 2 * sz] - u[p - sz]) +
-                                          c1 * (w[p] - w[p - 1]) + c2 * (w[p + 1] - w[p - 2]));
-        const T xl = f.lam[p], xm = f.mu[p];
-        const T a = xl + (T)2 * xm, b = xl;
+        const T xl = f.lam[p], xm = f.mu[p], mz = f.mu[p + sz];
+        const T xx = f.xx[p], yy = f.yy[p], zz = f.zz[p], xz = f.xz[p], vb = f.v[p - sy];
+        const T duz = c1 * (u[p + sz] - u[p]) + c2 * (u[p + 2 * sz] - u[p - sz]);
         const T diff1 = c1 * (u[p + 1] - u[p]) + c2 * (u[p + 2] - u[p - 1]);
         const T diff3 = c1 * (w[p] - w[p - sz]) + c2 * (w[p + sz] - w[p - 2 * sz]);
-        const T vb = f.v[p - sy];
+        const T dwx1 = c1 * (w[p] - w[p - 1]), dwx2 = c2 * (w[p + 1] - w[p - 2]);
+        const T xmu = xm + mz;
+        f.xz[p] = xz + dth2 * xmu * (duz + dwx1 + dwx2);
+        const T a = xl + (T)2 * xm, b = xl;
         const T v1t = vb - b * (diff1 + diff3) / ((T)2 * a);
         q.v1t[g.at2(i, k)] = v1t;
         const T dv = v1t - vb;
-        f.xx[p] = f.xx[p] + dth * a * (diff1) + dth * b * ((T)2 * dv + diff3);
-        f.yy[p] = f.yy[p] + dth * a * (T)2 * dv + dth * b * (diff1 + diff3);
-        f.zz[p] = f.zz[p] + dth * a * (diff3) + dth * b * (diff1 + (T)2 * dv);
+        f.xx[p] = xx + dth * a * (diff1) + dth * b * ((T)2 * dv + diff3);
+        f.yy[p] = yy + dth * a * (T)2 * dv + dth * b * (diff1 + diff3);
+        f.zz[p] = zz + dth * a * (diff3) + dth * b * (diff1 + (T)2 * dv);
     }
 }
 
@@ -786,19 +806,18 @@ __device__ __forceinline__ bool str_pml_tile(const Grid& g, const Fields<T>& f, 
     }
 }
 
-// fres (fd3d_deriv.f90:1067-1104)
+// fres (fd3d_deriv.f90:1067-1104), all loads before the stores
 template <class T>
-__device__ __forceinline__ void str_fs_body(Grid g, Fields<T> f, int bx_, int by_, int bz_) {
-    const int i = 1 + bx_ * blockDim.x + threadIdx.x;
-    const int j = 1 + by_ * blockDim.y + threadIdx.y;
+__device__ __forceinline__ void str_fs_body(const Grid& g, const Fields<T>& f, int i, int j) {
     if (i > g.nxt || j > g.nyt) return;
     const long long p = g.at(i, j, g.ks()), sz = g.plane;
-    f.zz[p + sz] = -f.zz[p];
-    f.zz[p + 2 * sz] = -f.zz[p - sz];
-    f.xz[p + sz] = -f.xz[p - sz];
-    f.xz[p + 2 * sz] = -f.xz[p - 2 * sz];
-    f.yz[p + sz] = -f.yz[p - sz];
-    f.yz[p + 2 * sz] = -f.yz[p - 2 * sz];
+    const T z0 = f.zz[p], z1 = f.zz[p - sz], x1 = f.xz[p - sz], x2 = f.xz[p - 2 * sz], y1 = f.yz[p - sz], y2 = f.yz[p - 2 * sz];
+    f.zz[p + sz] = -z0;
+    f.zz[p + 2 * sz] = -z1;
+    f.xz[p + sz] = -x1;
+    f.xz[p + 2 * sz] = -x2;
+    f.yz[p + sz] = -y1;
+    f.yz[p + 2 * sz] = -y2;
     f.xz[p] = (T)0;
     f.yz[p] = (T)0;
 }
@@ -1082,117 +1101,160 @@ __device__ __forceinline__ TrialTraction<T> trial_traction(const Grid& g, const 
     return t;
 }
 
-// Friction at the X node (i,k) (fd3d_theo.f90:375-410) from trial tractions in shared
-// memory: returns the traction after friction; OWN: also the node's state (tabsX, wX,
-// slip path, psi, strength).
-template <class T, bool OWN>
-__device__ __forceinline__ T friction_x(const Grid& g, const Fields<T>& f, const Fault<T>& q, const StepConst<T>& c,
-                                        int law, const FvwScalars& s, const double* distX_rd, double* distX_wr,
-                                        T txt0, T tint, int i, int k) {
+// What the friction law reads at a node beside the trial tractions, loaded before them where the
+// CTA has a thread for every node (fault_bc_body).  p0..p3: the law's parameters, slip weakening
+// peak, dynamic, Dc (DcX) and cohesion; rate-and-state a, b, vw and fw.
+template <class T>
+struct FricZ {  // Z node
+    T t0z, t0x, t0x1, t0x2, t0x3, U, U1, U2, U3, W, p0, p1, p2, p3, Dc;
+    double dist, slipZ, slipX, rt, st, psi;
+    __device__ __forceinline__ void load(const Grid& g, const Fields<T>& f, const Fault<T>& q, int law, int i, int k) {
+        const int n2 = g.at2(i, k), e1 = g.at2(i + 1, k), e2 = g.at2(i, k + 1), e3 = g.at2(i + 1, k + 1);
+        const long long p = g.at(i, g.nyt, k), sz = g.plane;
+        t0z = q.T0Z[n2]; t0x = q.T0X[n2]; t0x1 = q.T0X[e1]; t0x2 = q.T0X[e2]; t0x3 = q.T0X[e3];
+        U = f.u[p]; U1 = f.u[p + 1]; U2 = f.u[p + sz]; U3 = f.u[p + 1 + sz]; W = f.w[p];
+        if (law == 1) { p0 = q.aZ[n2]; p1 = q.bZ[n2]; p2 = q.vwZ[n2]; p3 = q.fwZ[n2]; psi = q.psiZ[n2]; }
+        else { p0 = q.peakZ[n2]; p1 = q.dynZ[n2]; p2 = q.DcZ[n2]; p3 = q.coh[n2]; }
+        Dc = q.Dc[n2];
+        dist = q.distZ[n2]; slipZ = q.slipZ[n2]; slipX = q.slipX[n2]; rt = q.ruptime[n2]; st = q.sliptime[n2];
+    }
+};
+template <class T>
+struct FricX {  // X node
+    T t0x, t0z, t0z1, t0z2, t0z3, U, W, W1, W2, W3, p0, p1, p2, p3, Dc;
+    double dist, psi;
+    __device__ __forceinline__ void load(const Grid& g, const Fields<T>& f, const Fault<T>& q, int law,
+                                         const double* distX_rd, int i, int k) {
+        const int n2 = g.at2(i, k), w1 = g.at2(i - 1, k), w2 = g.at2(i, k - 1), w3 = g.at2(i - 1, k - 1);
+        const long long p = g.at(i, g.nyt, k), sz = g.plane;
+        t0x = q.T0X[n2]; t0z = q.T0Z[n2]; t0z1 = q.T0Z[w1]; t0z2 = q.T0Z[w2]; t0z3 = q.T0Z[w3];
+        U = f.u[p]; W = f.w[p]; W1 = f.w[p - 1]; W2 = f.w[p - sz]; W3 = f.w[p - 1 - sz];
+        if (law == 1) { p0 = q.aX[n2]; p1 = q.bX[n2]; p2 = q.vwX[n2]; p3 = q.fwX[n2]; psi = q.psiX[n2]; }
+        else { p0 = q.peakX[n2]; p1 = q.dynX[n2]; p2 = q.DcX[n2]; p3 = q.coh[n2]; }
+        Dc = q.Dc[n2];
+        dist = distX_rd[n2];
+    }
+};
+
+// strength and new state variable of the rate-and-state law (fd3d_theo.f90:333-350): v1, v2 the
+// two velocity components at the node
+__device__ __forceinline__ double fvw_strength(const FvwScalars& s, double v1, double v2, double a, double b, double vw,
+                                               double fw, double Dc, double dtA, double psi0, double& psi) {
+    const double s1 = 2.0 * (fabs(v1) + fabs(s.wini)), s2 = 2.0 * (fabs(v2) + fabs(s.uini));
+    const double sr = sqrt(s1 * s1 + s2 * s2);
+    const double flv = s.f0 - (b - a) * log(sr / s.v0);
+    const double fss = fw + (flv - fw) / pow(1.0 + pow(sr / vw, 8.0), 1.0 / 8.0);
+    const double psiss = a * (log(sinh(fss / a)) + log(2.0 * s.v0 / sr));
+    psi = (psi0 - psiss) * exp(-sr * dtA / Dc) + psiss;
+    return s.Sn * a * asinh(sr * exp(psi / a) / (2.0 * s.v0));
+}
+
+// Friction at the X node (i,k) (fd3d_theo.f90:375-410): returns the traction after friction;
+// own: also the node's state (tabsX, wX, slip path, psi, strength).
+template <class T>
+__device__ __forceinline__ T friction_x(const Grid& g, const Fault<T>& q, const StepConst<T>& c, int law,
+                                        const FvwScalars& s, const FricX<T>& x, double* distX_wr, T txt0, T tint, bool own,
+                                        int i, int k) {
     const int n2 = g.at2(i, k);
     const double dtA = c.dtA;
-    const long long sz = g.plane;
-    const T sxv = txt0 + q.T0X[n2];
+    const T sxv = txt0 + x.t0x;
     const T tabsX = sqrt(sxv * sxv + tint * tint);
-    const long long p = g.at(i, g.nyt, k);
-    const T U = f.u[p], W = f.w[p];
-    const T wX = (W + f.w[p - 1] + f.w[p - sz] + f.w[p - 1 - sz]) / (T)4;
-    const T u1out = -sqrt(wX * wX + U * U);
+    const T wX = (x.W + x.W1 + x.W2 + x.W3) / (T)4;
+    const T u1out = -sqrt(wX * wX + x.U * x.U);
     T txn = txt0;
-    if (OWN) { q.tabsX[n2] = tabsX; q.wX[n2] = wX; }
+    if (own) { q.tabsX[n2] = tabsX; q.wX[n2] = wX; }
     if (law == 1) {
-        if (OWN) {
-            const double a = (double)q.aX[n2];
-            const double s1 = 2.0 * (fabs((double)wX) + fabs(s.wini)), s2 = 2.0 * (fabs((double)U) + fabs(s.uini));
-            const double sr = sqrt(s1 * s1 + s2 * s2);
-            const double flv = s.f0 - ((double)q.bX[n2] - a) * log(sr / s.v0);
-            const double fw = (double)q.fwX[n2];
-            const double fss = fw + (flv - fw) / pow(1.0 + pow(sr / (double)q.vwX[n2], 8.0), 1.0 / 8.0);
-            const double psiss = a * (log(sinh(fss / a)) + log(2.0 * s.v0 / sr));
-            const double psi = (q.psiX[n2] - psiss) * exp(-sr * dtA / (double)q.Dc[n2]) + psiss;
+        if (own) {
+            double psi;
+            const double fric = fvw_strength(s, (double)wX, (double)x.U, (double)x.p0, (double)x.p1, (double)x.p2,
+                                             (double)x.p3, (double)x.Dc, dtA, x.psi, psi);
             q.psiX[n2] = psi;
-            const double fric = s.Sn * a * asinh(sr * exp(psi / a) / (2.0 * s.v0));
-            distX_wr[n2] = distX_rd[n2] - 2.0 * (double)u1out * dtA;
+            distX_wr[n2] = x.dist - 2.0 * (double)u1out * dtA;
             q.schangeX[n2] = (T)fric;
         }
     } else {
-        const double dx = distX_rd[n2], dcx = (double)q.DcX[n2];
+        const double dx = x.dist, dcx = (double)x.p2;
         double fric;
-        if (dx <= (double)q.Dc[n2]) fric = (double)q.peakX[n2] * (1.0 - dx / dcx) + (double)q.dynX[n2] * dx / dcx + (double)q.coh[n2];
-        else                        fric = (double)q.dynX[n2] + (double)q.coh[n2];
+        if (dx <= (double)x.Dc) fric = (double)x.p0 * (1.0 - dx / dcx) + (double)x.p1 * dx / dcx + (double)x.p3;
+        else                    fric = (double)x.p1 + (double)x.p3;
         double dnew = dx;
         if ((double)tabsX >= fric) {
             dnew = dx - 2.0 * (double)u1out * dtA;
-            txn = (T)(((double)txn + (double)q.T0X[n2]) * fric / (double)tabsX - (double)q.T0X[n2]);
+            txn = (T)(((double)txn + (double)x.t0x) * fric / (double)tabsX - (double)x.t0x);
         }
-        if (OWN) distX_wr[n2] = dnew;
+        if (own) distX_wr[n2] = dnew;
     }
-    if (OWN) q.tx[n2] = txn;
+    if (own) q.tx[n2] = txn;
     return txn;
 }
 
-// Friction at the Z node (i,k) (fd3d_theo.f90:326-373): state, slip, rupture time; returns tz.
+// Friction at the Z node (i,k) (fd3d_theo.f90:326-373): state, slip, rupture time; returns tz and,
+// rate-and-state, the strength.
 template <class T>
-__device__ __forceinline__ T friction_z(const Grid& g, const Fields<T>& f, const Fault<T>& q, const StepConst<T>& c,
-                                        int law, const FvwScalars& s, double time, T tzt0, T tint, int i, int k) {
+__device__ __forceinline__ T friction_z(const Grid& g, const Fault<T>& q, const StepConst<T>& c, int law,
+                                        const FvwScalars& s, const FricZ<T>& z, double time, T tzt0, T tint, int i, int k,
+                                        T& strength, T& psi_out) {
     const int n2 = g.at2(i, k);
     const double dtA = c.dtA, rup = 1.e-3;
-    const long long sz = g.plane;
-    const T* T0Z = q.T0Z;
-    const T szv = tzt0 + T0Z[n2];
+    const T szv = tzt0 + z.t0z;
     const T tabsZ = sqrt(tint * tint + szv * szv);
     q.tabsZ[n2] = tabsZ;
-    const long long p = g.at(i, g.nyt, k);
-    const T U = f.u[p], W = f.w[p];
-    const T uZ = (U + f.u[p + 1] + f.u[p + sz] + f.u[p + 1 + sz]) / (T)4;
+    const T uZ = (z.U + z.U1 + z.U2 + z.U3) / (T)4;
     q.uZ[n2] = uZ;
-    const T u1out = -sqrt(W * W + uZ * uZ);
+    const T u1out = -sqrt(z.W * z.W + uZ * uZ);
     T tzn = tzt0;
+    double dist = z.dist;
+    bool moving;
     if (law == 1) {
-        const double a = (double)q.aZ[n2];
-        const double s1 = 2.0 * (fabs((double)W) + fabs(s.wini)), s2 = 2.0 * (fabs((double)uZ) + fabs(s.uini));
-        const double sr = sqrt(s1 * s1 + s2 * s2);
-        const double flv = s.f0 - ((double)q.bZ[n2] - a) * log(sr / s.v0);
-        const double fw = (double)q.fwZ[n2];
-        const double fss = fw + (flv - fw) / pow(1.0 + pow(sr / (double)q.vwZ[n2], 8.0), 1.0 / 8.0);
-        const double psiss = a * (log(sinh(fss / a)) + log(2.0 * s.v0 / sr));
-        const double psi = (q.psiZ[n2] - psiss) * exp(-sr * dtA / (double)q.Dc[n2]) + psiss;
+        double psi;
+        const double fric = fvw_strength(s, (double)z.W, (double)uZ, (double)z.p0, (double)z.p1, (double)z.p2,
+                                         (double)z.p3, (double)z.Dc, dtA, z.psi, psi);
         q.psiZ[n2] = psi;
-        const double fric = s.Sn * a * asinh(sr * exp(psi / a) / (2.0 * s.v0));
-        q.distZ[n2] = q.distZ[n2] - 2.0 * (double)u1out * dtA;
-        q.schangeZ[n2] = (T)fric;
-        if (fabs(2.0 * (double)u1out) > rup) {
-            if (q.ruptime[n2] != 1.e4) q.rise[n2] = time;
-            if (q.ruptime[n2] == 1.e4) q.ruptime[n2] = time;
-        }
+        dist = z.dist - 2.0 * (double)u1out * dtA;
+        strength = (T)fric;
+        psi_out = (T)psi;
+        q.schangeZ[n2] = strength;
+        moving = fabs(2.0 * (double)u1out) > rup;
     } else {
-        const double dz = q.distZ[n2], dcz = (double)q.DcZ[n2];
+        const double dz = z.dist, dcz = (double)z.p2;
         double fric;
-        if (dz <= dcz) fric = (double)q.peakZ[n2] * (1.0 - dz / dcz) + (double)q.dynZ[n2] * dz / dcz + (double)q.coh[n2];
-        else           fric = (double)q.dynZ[n2] + (double)q.coh[n2];
-        if ((double)tabsZ >= fric) {
-            q.distZ[n2] = dz - 2.0 * (double)u1out * dtA;
-            tzn = (T)(((double)tzn + (double)T0Z[n2]) * fric / (double)tabsZ - (double)T0Z[n2]);
-            if (-2.0 * (double)u1out > rup) {
-                if (q.ruptime[n2] != 1.e4) q.rise[n2] = time;
-                if (q.ruptime[n2] == 1.e4) q.ruptime[n2] = time;
-            }
+        if (dz <= dcz) fric = (double)z.p0 * (1.0 - dz / dcz) + (double)z.p1 * dz / dcz + (double)z.p3;
+        else           fric = (double)z.p1 + (double)z.p3;
+        const bool slips = (double)tabsZ >= fric;
+        if (slips) {
+            dist = dz - 2.0 * (double)u1out * dtA;
+            tzn = (T)(((double)tzn + (double)z.t0z) * fric / (double)tabsZ - (double)z.t0z);
         }
+        moving = slips && -2.0 * (double)u1out > rup;
+    }
+    q.distZ[n2] = dist;
+    if (moving) {
+        if (z.rt != 1.e4) q.rise[n2] = time;
+        else q.ruptime[n2] = time;
     }
     q.tz[n2] = tzn;
-    q.slipZ[n2] = q.slipZ[n2] - 2.0 * (double)W * dtA;
-    q.slipX[n2] = q.slipX[n2] - 2.0 * (double)uZ * dtA;
-    if (q.sliptime[n2] == 1.e4 && q.distZ[n2] > (double)q.Dc[n2]) q.sliptime[n2] = time;
+    q.slipZ[n2] = z.slipZ - 2.0 * (double)z.W * dtA;
+    q.slipX[n2] = z.slipX - 2.0 * (double)uZ * dtA;
+    if (z.st == 1.e4 && dist > (double)z.Dc) q.sliptime[n2] = time;
     return tzn;
 }
 
-// One tile of the fused fault boundary condition (without fres).  A CTA of 32 x 8 threads;
-// sm holds FBC_SMEM elements.
-template <class T>
+// One tile of the fused fault boundary condition (without fres) on a CTA of NT threads (thread
+// tid); sm holds FBC_SMEM elements.
+//
+// Bound by latency: a small grid has one tile per SM or less.  With FBC_THREADS each trial
+// traction of the tile and its ring, each Z node and each X node has a thread of its own, and what
+// the friction law reads is loaded before the trial tractions, so a tile is two rounds of memory
+// latency and one friction law long.  With 256 threads the same parts run one after the other.
+// One launch, us (before: 256 threads, loads in the law): slip weakening, 50 tiles 11.3 (17.1), 1250
+// tiles 69 (72).
+constexpr int FBC_THREADS = 576;  // >= 256 Z nodes + 297 X nodes, and the 340 trial tractions
+template <class T, int NT>
 __device__ __forceinline__ void fault_bc_body(const Grid& g, const Fields<T>& f, const Fault<T>& q,
                                               const StepConst<T>& c, int law, const FvwScalars& s, const int* it_dev,
-                                              const HistDesc& h, int* status, int bx_, int by_, T* sm) {
-    const int tid = threadIdx.y * 32 + threadIdx.x;
+                                              const HistDesc& h, int* status, int bx_, int by_, T* sm, int tid) {
+    constexpr int NZ = FBC_TX * FBC_TZ, NXH = FBC_PX * FBC_PZ - NZ;  // own nodes; X nodes of the column and row beyond
+    constexpr bool ALL = NT >= NZ + NZ + NXH;
     const int i0 = g.nabc + 1 + bx_ * FBC_TX, k0 = g.nabc + 1 + by_ * FBC_TZ;
     const int ie = g.nxt - g.nabc, ks = g.ks();
     const int it = *it_dev;
@@ -1202,71 +1264,92 @@ __device__ __forceinline__ void fault_bc_body(const Grid& g, const Fields<T>& f,
     T* s_txt = sm;                        // [FBC_HZ][FBC_HX], node (i,k) at (i-i0+1) + (k-k0+1)*FBC_HX
     T* s_tzt = sm + FBC_HX * FBC_HZ;
     T* s_tx = sm + 2 * FBC_HX * FBC_HZ;   // [FBC_PZ][FBC_PX], node (i,k) at (i-i0) + (k-k0)*FBC_PX
+
+    // the Z node of a thread below NZ, and the n-th X node: the tile's, then the column
+    // i0+FBC_TX (k0..k0+FBC_TZ), then the row k0+FBC_TZ (i0..i0+FBC_TX-1)
+    const int i = i0 + tid % FBC_TX, k = k0 + tid / FBC_TX;
+    const bool own = tid < NZ && i <= ie && k <= ks;
+    auto x_node = [&](int n, int& xi, int& xk) {
+        if (n < NZ) { xi = i0 + n % FBC_TX; xk = k0 + n / FBC_TX; }
+        else if (n < NZ + FBC_PZ) { xi = i0 + FBC_TX; xk = k0 + n - NZ; }
+        else { xi = i0 + n - NZ - FBC_PZ; xk = k0 + FBC_TZ; }
+        return n < NZ + NXH && xi <= ie && xk <= ks;
+    };
+    FricZ<T> z;
+    FricX<T> x;
+    int xi = 0, xk = 0;
+    bool has_x = false;
+    if (ALL) {
+        if (own) z.load(g, f, q, law, i, k);
+        has_x = tid >= NZ && x_node(tid - NZ, xi, xk);
+        if (has_x) x.load(g, f, q, law, distX_rd, xi, xk);
+    }
     __syncthreads();                      // the shared memory may hold the previous item's values
 
     // 1. trial tractions of the tile and its ring; the owner stores a node's state
-    for (int n = tid; n < FBC_HX * FBC_HZ; n += 256) {
+    for (int n = tid; n < FBC_HX * FBC_HZ; n += NT) {
         const int ri = n % FBC_HX, rk = n / FBC_HX;
-        const int i = i0 - 1 + ri, k = k0 - 1 + rk;
+        const int ti = i0 - 1 + ri, tk = k0 - 1 + rk;
         T tx_ = 0, tz_ = 0;   // outside the traction loops the reference's tx, tz stay 0
-        if (i >= g.nabc + 1 && i <= ie) {
-            if (k >= g.nabc + 1 && k <= ks) {
-                const TrialTraction<T> t = trial_traction<T, true>(g, f, c, avdz_rd, avdx_rd, i, k);
+        if (ti >= g.nabc + 1 && ti <= ie) {
+            if (tk >= g.nabc + 1 && tk <= ks) {
+                const TrialTraction<T> t = trial_traction<T, true>(g, f, c, avdz_rd, avdx_rd, ti, tk);
                 tx_ = t.txv;
                 tz_ = t.tzv;
                 if (ri >= 1 && ri <= FBC_TX && rk >= 1 && rk <= FBC_TZ) {
-                    const int n2 = g.at2(i, k);
+                    const int n2 = g.at2(ti, tk);
                     q.RFz[n2] = t.rfz;
                     q.RFx[n2] = t.rfx;
                     avdz_wr[n2] = t.pdz;
                     avdx_wr[n2] = t.pdx;
                 }
-            } else if (!g.fspace && k == ks + 1) {  // ghost row: tx(nzt-1) = tx(nzt-2), tz(nzt-1) = -tz(nzt-3)
-                tx_ = +trial_traction<T, true>(g, f, c, avdz_rd, avdx_rd, i, ks).txv;
-                tz_ = -trial_traction<T, true>(g, f, c, avdz_rd, avdx_rd, i, ks - 1).tzv;
+            } else if (!g.fspace && tk == ks + 1) {  // ghost row: tx(nzt-1) = tx(nzt-2), tz(nzt-1) = -tz(nzt-3)
+                tx_ = +trial_traction<T, true>(g, f, c, avdz_rd, avdx_rd, ti, ks).txv;
+                tz_ = -trial_traction<T, true>(g, f, c, avdz_rd, avdx_rd, ti, ks - 1).tzv;
             }
         }
         s_txt[n] = tx_;
         s_tzt[n] = tz_;
     }
     __syncthreads();
-    auto TXT = [&](int i, int k) { return s_txt[(i - i0 + 1) + (k - k0 + 1) * FBC_HX]; };
-    auto TZT = [&](int i, int k) { return s_tzt[(i - i0 + 1) + (k - k0 + 1) * FBC_HX]; };
-    auto TINT_X = [&](int i, int k) {  // 4-point average of tz + T0Z around X node (i,k)
-        const int n2 = g.at2(i, k), w1 = g.at2(i - 1, k), w2 = g.at2(i, k - 1), w3 = g.at2(i - 1, k - 1);
-        return (TZT(i, k) + q.T0Z[n2] + TZT(i - 1, k) + q.T0Z[w1] + TZT(i, k - 1) + q.T0Z[w2] + TZT(i - 1, k - 1) +
-                q.T0Z[w3]) / (T)4;
-    };
+    auto TXT = [&](int ii, int kk) { return s_txt[(ii - i0 + 1) + (kk - k0 + 1) * FBC_HX]; };
+    auto TZT = [&](int ii, int kk) { return s_tzt[(ii - i0 + 1) + (kk - k0 + 1) * FBC_HX]; };
 
-    // 2. friction: the Z and X nodes of the tile (thread = node), then the X nodes of the
-    //    column and row beyond it (their tractions after friction, for the output)
-    const int ti = threadIdx.x, tk = threadIdx.y;
-    const int i = i0 + ti, k = k0 + tk;
-    const bool own = i <= ie && k <= ks;
-    T tzn = 0, txo = 0;   // beyond the interior plane the reference's tx stays 0
+    // 2. friction at the Z nodes of the tile and at its X nodes with those of the column and row
+    //    beyond it (their tractions after friction, for the output)
+    T tzn = 0, strength = 0, psi = 0;
     if (own) {
-        const double time = (double)it * c.dtA;
-        const int n2 = g.at2(i, k), e1 = g.at2(i + 1, k), e2 = g.at2(i, k + 1), e3 = g.at2(i + 1, k + 1);
-        const T tintz = (TXT(i, k) + q.T0X[n2] + TXT(i + 1, k) + q.T0X[e1] + TXT(i, k + 1) + q.T0X[e2] +
-                         TXT(i + 1, k + 1) + q.T0X[e3]) / (T)4;
-        tzn = friction_z<T>(g, f, q, c, law, s, time, TZT(i, k), tintz, i, k);
-        txo = friction_x<T, true>(g, f, q, c, law, s, distX_rd, distX_wr, TXT(i, k), TINT_X(i, k), i, k);
+        if (!ALL) z.load(g, f, q, law, i, k);
+        const T tint = (TXT(i, k) + z.t0x + TXT(i + 1, k) + z.t0x1 + TXT(i, k + 1) + z.t0x2 + TXT(i + 1, k + 1) +
+                        z.t0x3) / (T)4;
+        tzn = friction_z<T>(g, q, c, law, s, z, (double)it * c.dtA, TZT(i, k), tint, i, k, strength, psi);
         if (k == ks) {  // the reference's tx/tz arrays also carry the ghost row nzt-1
             const int gh = g.at2(i, k + 1);
             q.tx[gh] = TXT(i, k + 1);
             q.tz[gh] = TZT(i, k + 1);
         }
     }
-    s_tx[ti + tk * FBC_PX] = txo;
-    if (tid < FBC_PX + FBC_TZ) {  // column i0+FBC_TX (k0..k0+FBC_TZ), then row k0+FBC_TZ (i0..i0+FBC_TX-1)
-        const int hi = tid < FBC_PZ ? i0 + FBC_TX : i0 + (tid - FBC_PZ);
-        const int hk = tid < FBC_PZ ? k0 + tid : k0 + FBC_TZ;
-        T txh = 0;
-        if (hi <= ie && hk <= ks && law == 0)
-            txh = friction_x<T, false>(g, f, q, c, law, s, distX_rd, distX_wr, TXT(hi, hk), TINT_X(hi, hk), hi, hk);
-        else if (hi <= ie && hk <= ks)
-            txh = TXT(hi, hk);
-        s_tx[(hi - i0) + (hk - k0) * FBC_PX] = txh;
+    auto do_x = [&](int n) {
+        T t = 0;   // beyond the interior plane the reference's tx stays 0
+        if (has_x) {
+            if (law == 1 && n >= NZ) {
+                t = TXT(xi, xk);
+            } else {
+                const T tint = (TZT(xi, xk) + x.t0z + TZT(xi - 1, xk) + x.t0z1 + TZT(xi, xk - 1) + x.t0z2 +
+                                TZT(xi - 1, xk - 1) + x.t0z3) / (T)4;
+                t = friction_x<T>(g, q, c, law, s, x, distX_wr, TXT(xi, xk), tint, n < NZ, xi, xk);
+            }
+        }
+        s_tx[(xi - i0) + (xk - k0) * FBC_PX] = t;
+    };
+    if (ALL) {
+        if (tid >= NZ && tid < NZ + NZ + NXH) do_x(tid - NZ);
+    } else {
+        for (int n = tid; n < NZ + NXH; n += NT) {
+            has_x = x_node(n, xi, xk);
+            if (has_x) x.load(g, f, q, law, distX_rd, xi, xk);
+            do_x(n);
+        }
     }
     __syncthreads();
 
@@ -1280,29 +1363,25 @@ __device__ __forceinline__ void fault_bc_body(const Grid& g, const Fields<T>& f,
     if (!own) return;
     auto TX = [&](int ii, int kk) { return s_tx[(ii - i0) + (kk - k0) * FBC_PX]; };
     const bool top = (k == ks);
-    const long long p = g.at(i, g.nyt, k), sz = g.plane;
-    const int n2 = g.at2(i, k), e1 = g.at2(i + 1, k), e2 = g.at2(i, k + 1), e3 = g.at2(i + 1, k + 1);
-    const T U = f.u[p], U2 = f.u[p + 1], W = f.w[p];
+    const int n2 = g.at2(i, k);
     T srx, srz, scx, scz;
-    srz = (T)-2 * W;
+    srz = (T)-2 * z.W;
     if (!top) {
-        const T U3 = f.u[p + sz], U4 = f.u[p + 1 + sz];
-        srx = ((T)-2 * U - (T)2 * U2 - (T)2 * U3 - (T)2 * U4) / (T)4;
+        srx = ((T)-2 * z.U - (T)2 * z.U1 - (T)2 * z.U2 - (T)2 * z.U3) / (T)4;
         if (law == 0) {
-            scz = tzn + q.T0Z[n2];
-            scx = (TX(i, k) + q.T0X[n2] + TX(i + 1, k) + q.T0X[e1] + TX(i, k + 1) + q.T0X[e2] + TX(i + 1, k + 1) +
-                   q.T0X[e3]) / (T)4;
+            scz = tzn + z.t0z;
+            scx = (TX(i, k) + z.t0x + TX(i + 1, k) + z.t0x1 + TX(i, k + 1) + z.t0x2 + TX(i + 1, k + 1) + z.t0x3) / (T)4;
         }
     } else {
         if (law == 1) {
-            srx = ((T)-2 * U - (T)2 * U2) / (T)4;
+            srx = ((T)-2 * z.U - (T)2 * z.U1) / (T)4;
         } else {
-            scz = tzn + q.T0Z[n2];
-            scx = (TX(i, k) + q.T0X[n2] + TX(i + 1, k) + q.T0X[e1]) / (T)2;
-            srx = ((T)-2 * U - (T)2 * U2) / (T)2;
+            scz = tzn + z.t0z;
+            scx = (TX(i, k) + z.t0x + TX(i + 1, k) + z.t0x1) / (T)2;
+            srx = ((T)-2 * z.U - (T)2 * z.U1) / (T)2;
         }
     }
-    if (law == 1) { scx = q.schangeX[n2]; scz = q.schangeZ[n2]; }
+    if (law == 1) { scx = q.schangeX[n2]; scz = strength; }  // (schangeX: this CTA's X node, before the barrier)
     else { q.schangeX[n2] = scx; q.schangeZ[n2] = scz; }
     if (!(isfinite((double)srx) && isfinite((double)srz) && isfinite((double)scx) && isfinite((double)scz)))
         atomicOr(status, ST_NONFINITE);
@@ -1315,13 +1394,13 @@ __device__ __forceinline__ void fault_bc_body(const Grid& g, const Fields<T>& f,
         r[plane] = srz;
         r[2 * plane] = scx;
         r[3 * plane] = scz;
-        if (h.nf > 4) r[4 * plane] = (T)q.psiZ[n2];
+        if (h.nf > 4) r[4 * plane] = psi;
     }
 }
 
-// grid of the fused fault BC: fres CTAs (32 x 8 (i,j) each), then the fault tiles
-inline void fault_bc_grid(const Grid& g, int& nfres, int& tiles_x, int& tiles) {
-    nfres = g.fspace ? 0 : ((g.nxt + 31) / 32) * ((g.nyt + 7) / 8);
+// grid of the fused fault BC: fres CTAs (32 x rows (i,j) each), then the fault tiles
+inline void fault_bc_grid(const Grid& g, int rows, int& nfres, int& tiles_x, int& tiles) {
+    nfres = g.fspace ? 0 : ((g.nxt + 31) / 32) * ((g.nyt + rows - 1) / rows);
     const int nxT = g.nxt - 2 * g.nabc, nzT = g.ks() - g.nabc;
     tiles_x = (nxT + FBC_TX - 1) / FBC_TX;
     tiles = tiles_x * ((nzT + FBC_TZ - 1) / FBC_TZ);
@@ -1346,8 +1425,9 @@ __device__ __forceinline__ void nucleation_body(Grid g, Fault<T> q, StepConst<T>
 
 // ---------------------------------------------------------------- launch wrappers
 template <class T>
-__global__ void k_vel_fault(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c, int law, FvwScalars s,
-                            int* it_dev, int* status) {
+__global__ void __launch_bounds__(256)
+k_vel_fault(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ Fault<T> q,
+            const __grid_constant__ StepConst<T> c, int law, const __grid_constant__ FvwScalars s, int* it_dev, int* status) {
     vel_fault_body<T>(g, f, q, c, law, s, it_dev, status, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -1368,7 +1448,9 @@ __global__ void k_vel_fs(Grid g, Fields<T> f) {
 }
 
 template <class T>
-__global__ void k_str_fault(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c) {
+__global__ void __launch_bounds__(256)
+k_str_fault(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ Fault<T> q,
+            const __grid_constant__ StepConst<T> c) {
     str_fault_body<T>(g, f, q, c, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -1429,7 +1511,7 @@ inline void launch_pml(bool stress, int minb, cudaStream_t st, const Grid& g, co
 
 template <class T>
 __global__ void k_str_fs(Grid g, Fields<T> f) {
-    str_fs_body<T>(g, f, blockIdx.x, blockIdx.y, blockIdx.z);
+    str_fs_body<T>(g, f, 1 + blockIdx.x * blockDim.x + threadIdx.x, 1 + blockIdx.y * blockDim.y + threadIdx.y);
 }
 
 template <class T>
@@ -1450,20 +1532,47 @@ __global__ void k_output(Grid g, Fields<T> f, Fault<T> q, int law, const int* it
 }
 
 // The fused fault boundary condition of one step: nfres CTAs of fres, then the fault tiles
-// (tiles_x per row of tiles); CTA of 32 x 8 threads.
-template <class T>
-__global__ void __launch_bounds__(256) k_fault_bc(Grid g, Fields<T> f, Fault<T> q, StepConst<T> c, int law,
-                                                  FvwScalars s, const int* it_dev, const __grid_constant__ HistDesc h,
-                                                  int* status, int nfres, int tiles_x) {
+// (tiles_x per row of tiles); CTA of NT threads.  LAW is a template argument for its registers:
+// slip weakening in FP32 fits two CTAs of FBC_THREADS per SM, the others one.
+template <class T, int LAW, int NT>
+__global__ void __launch_bounds__(NT, NT == 256 ? (sizeof(T) == 4 ? 3 : 2) : LAW == 0 && sizeof(T) == 4 ? 2 : 1)
+k_fault_bc(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ Fault<T> q,
+           const __grid_constant__ StepConst<T> c, const __grid_constant__ FvwScalars s, const int* it_dev,
+           const __grid_constant__ HistDesc h, int* status, int nfres, int tiles_x) {
     __shared__ T sm[FBC_SMEM];
     const int b = blockIdx.x;
     if (b < nfres) {
         const int sx = (g.nxt + 31) / 32;
-        str_fs_body<T>(g, f, b % sx, b / sx, 0);
+        str_fs_body<T>(g, f, 1 + b % sx * 32 + threadIdx.x % 32, 1 + b / sx * (NT / 32) + threadIdx.x / 32);
         return;
     }
     const int t = b - nfres;
-    fault_bc_body<T>(g, f, q, c, law, s, it_dev, h, status, t % tiles_x, t / tiles_x, sm);
+    fault_bc_body<T, NT>(g, f, q, c, LAW, s, it_dev, h, status, t % tiles_x, t / tiles_x, sm, threadIdx.x);
+}
+
+template <class T, int LAW, int NT>
+inline void launch_fault_bc_n(cudaStream_t st, const Grid& g, const Fields<T>& f, const Fault<T>& q, const StepConst<T>& c,
+                              const FvwScalars& s, const int* it_dev, const HistDesc& h, int* status) {
+    int nfres, tiles_x, tiles;
+    fault_bc_grid(g, NT / 32, nfres, tiles_x, tiles);
+    k_fault_bc<T, LAW, NT><<<nfres + tiles, NT, 0, st>>>(g, f, q, c, s, it_dev, h, status, nfres, tiles_x);
+}
+// FBC_THREADS threads a tile where two tiles fit an SM (slip weakening, FP32), and elsewhere where
+// there are no more tiles than SMs; 256 threads beyond that, since the kernel is then bound by
+// the warps it has in flight (rate-and-state, us: 50 tiles 13.9 against 20.5, 950 tiles 78
+// against 48.6).
+template <class T>
+inline void launch_fault_bc(int law, int nsm, cudaStream_t st, const Grid& g, const Fields<T>& f, const Fault<T>& q,
+                            const StepConst<T>& c, const FvwScalars& s, const int* it_dev, const HistDesc& h, int* status) {
+    int nfres, tiles_x, tiles;
+    fault_bc_grid(g, 8, nfres, tiles_x, tiles);
+    if (law == 0) {
+        if (sizeof(T) == 4 || tiles <= nsm) launch_fault_bc_n<T, 0, FBC_THREADS>(st, g, f, q, c, s, it_dev, h, status);
+        else launch_fault_bc_n<T, 0, 256>(st, g, f, q, c, s, it_dev, h, status);
+    } else {
+        if (tiles <= nsm) launch_fault_bc_n<T, 1, FBC_THREADS>(st, g, f, q, c, s, it_dev, h, status);
+        else launch_fault_bc_n<T, 1, 256>(st, g, f, q, c, s, it_dev, h, status);
+    }
 }
 
 template <class T>
