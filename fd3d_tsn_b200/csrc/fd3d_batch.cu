@@ -329,25 +329,6 @@ __global__ void k_step_end(int* run_step) {
     *run_step += 1;
 }
 
-// A launch of the graph schedule, with programmatic stream serialization when pdl is set:
-// the kernel's CTAs may be scheduled while the kernel before it drains, and wait in
-// pdl_wait (every kernel of the schedule starts with it) for its completion.
-template <class... K, class... A>
-static cudaError_t launch_g(bool pdl, void (*kern)(K...), unsigned grid, dim3 blk, size_t smem, cudaStream_t s,
-                            A... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = blk;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, args...);
-}
-
 // OR of the live models' device status words into out (one read-back per sync)
 __global__ void k_or_status(int* const* __restrict__ st, int n, int* out) {
     int v = 0;
@@ -689,9 +670,9 @@ int enqueue_graph_step(fd3d_batch* b) {
         const int* rs = b->d_run_step;
         const ModelDev* md = b->d_models;
         const Work* wt = b->d_work_t;
-        if (t0 <= W_FBC && W_FBC < t1) chk(launch_g(pdl, k_bplane<1>, n, blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
-        else if (t0 == W_VEL_FAULT) chk(launch_g(pdl, k_bplane<2>, n, blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
-        else chk(launch_g(pdl, k_bplane<0>, n, blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
+        if (t0 <= W_FBC && W_FBC < t1) chk(launch_kernel(pdl, k_bplane<1>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
+        else if (t0 == W_VEL_FAULT) chk(launch_kernel(pdl, k_bplane<2>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
+        else chk(launch_kernel(pdl, k_bplane<0>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
     };
     // the fault-band and PML sweeps on side streams beside the interior sweep, or (branches
     // off) all on the main stream one after another
@@ -711,13 +692,13 @@ int enqueue_graph_step(fd3d_batch* b) {
         const int* rs = b->d_run_step;
         if (n_of(ti) > 0) {
             const size_t sm = tma_ring_bytes<float>();
-            if (half) chk(launch_g(pdl, k_bint<true>, n_of(ti), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, kc, b->d_status));
-            else chk(launch_g(pdl, k_bint<false>, n_of(ti), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, kc, b->d_status));
+            if (half) chk(launch_kernel(pdl, k_bint<true>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, kc, b->d_status));
+            else chk(launch_kernel(pdl, k_bint<false>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, kc, b->d_status));
         }
         plane(s0, tf, tf + 1);
         if (n_of(tp) > 0) {
-            if (half) chk(launch_g(pdl, k_bpml<true>, n_of(tp), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, b->d_status));
-            else chk(launch_g(pdl, k_bpml<false>, n_of(tp), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, b->d_status));
+            if (half) chk(launch_kernel(pdl, k_bpml<true>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, b->d_status));
+            else chk(launch_kernel(pdl, k_bpml<false>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, b->d_status));
         }
         if (b->branches) {
             BCK(cudaEventRecord(b->evf[1], b->side[0]));
@@ -728,7 +709,7 @@ int enqueue_graph_step(fd3d_batch* b) {
         plane(b->st, tfs, half ? W_FBC + 1 : tfs + 1);  // after the stresses: fres and the fault BC tiles
     }
     plane(b->st, W_NUC, W_NUC + 1);
-    chk(launch_g(pdl, k_step_end, 1, dim3(1), 0, b->st, b->d_run_step));
+    chk(launch_kernel(pdl, k_step_end, dim3(1), dim3(1), 0, b->st, b->d_run_step));
     BCK(err);
     BCK(cudaGetLastError());
     return FD3D_OK;

@@ -189,6 +189,8 @@ struct CtxBase {
         return best < 0 ? cudaStreamSynchronize(st) : cudaEventSynchronize(mark_ev[best]);
     }
     int overlap = 1;
+    // the step's half-steps as one launch each (small_step)
+    bool small_grid = false;
     // the fault boundary condition as separate launches (fres, traction, friction, output)
     // with the trial tractions in q.txt / q.tzt instead of the fused kernel
     bool split_bc = false;
@@ -372,6 +374,7 @@ struct Ctx : CtxBase {
         // at 4 (424 at 3; 5 spills, 399); FP64 (0.6 M cells) 20 at 3, 30 at 2 (no spills)
         if (!pml_minb_vel) pml_minb_vel = sizeof(T) == 8 ? 3 : 4;
         if (!pml_minb_str) pml_minb_str = sizeof(T) == 8 ? 2 : 4;
+        small_grid = small_step(icfg, g, D);
         if (!tma_ok && icfg.variant == IV_TMA) {
             std::fprintf(stderr, "fd3d: tensor maps of the interior sweeps could not be encoded for this grid; "
                                  "the interior sweeps fall back to plain loads (fd3d_ctx_info reports it)\n");
@@ -698,6 +701,7 @@ struct Ctx : CtxBase {
         const int nzT = std::max(1, g.kin_hi() - g.kin_lo() + 1);  // fault rows updated (a launch has one at least)
         const dim3 b2(32, 8);
         const bool ov = overlap > 0 && !profiling;
+        const bool small = small_grid && ov && !split_bc && icfg.variant == IV_TMA;
         const bool top = g.owns(g.ks());  // the free-surface rows are this context's
         cudaStream_t sp = ov ? st2 : st;  // fault band and PML
         auto fork = [&](int e) { cudaEventRecord(evf[e], st); cudaStreamWaitEvent(st2, evf[e], 0); };
@@ -710,6 +714,11 @@ struct Ctx : CtxBase {
         }
         switch (ph) {
         case 0:  // velocity half-step
+            if (small) {
+                launch_half_small<T>(false, vmaps, smaps, icfg, g, f, q, D, X, c, law, fs, it_dev, status, st);
+                if (!p.fspace) launch_kernel(true, k_vel_fs<T>, dim3((p.nxt + 31) / 32, (p.nyt + 7) / 8), b2, 0, st, g, f);
+                break;
+            }
             if (ov) fork(0);
             kbeg(0);
             if (icfg.variant == IV_TMA) launch_vel_interior_tma<T>(vmaps, icfg, g, f, c, status, st);
@@ -727,6 +736,10 @@ struct Ctx : CtxBase {
             kend(3);
             break;
         case 1:  // stress sweeps
+            if (small) {
+                launch_half_small<T>(true, vmaps, smaps, icfg, g, f, q, D, X, c, law, fs, it_dev, status, st);
+                break;
+            }
             if (ov) fork(2);
             kbeg(4);
             if (icfg.variant == IV_TMA) launch_str_interior_tma<T>(smaps, icfg, g, f, c, status, st);
@@ -743,7 +756,7 @@ struct Ctx : CtxBase {
         case 2:  // fault boundary condition
             kbeg(7);
             if (!split_bc) {   // fres and the fused trial traction, friction and output tiles in one launch
-                launch_fault_bc<T>(law, icfg.nsm, st, g, f, q, c, fs, it_dev, h, status);
+                launch_fault_bc<T>(small, law, icfg.nsm, st, g, f, q, c, fs, it_dev, h, status);
             } else {           // the same as separate launches, trial tractions in q.txt / q.tzt
                 if (!p.fspace && top) k_str_fs<T><<<dim3((p.nxt + 31) / 32, (p.nyt + 7) / 8), b2, 0, st>>>(g, f);  // fres
                 k_traction<T><<<dim3((nxT + 31) / 32, (nzT + 7) / 8), b2, 0, st>>>(g, f, q, c, it_dev);
@@ -756,7 +769,7 @@ struct Ctx : CtxBase {
             if (split_bc) k_output<T><<<dim3((nxT + 31) / 32, (nzT + 7) / 8), b2, 0, st>>>(g, f, q, law, it_dev, h, status);
             if (law == FD3D_LAW_FVW && fs.nucleation) {  // every node of the plane (a z-slab too: no halo needed)
                 const int ni = (p.nxt - p.nabc) - (p.nabc - 1) + 1, nk = g.ks() - (p.nabc - 1) + 1;
-                k_nucleation<T><<<dim3((ni + 31) / 32, (nk + 7) / 8), b2, 0, st>>>(g, q, c, fs, it_dev);
+                launch_kernel(small, k_nucleation<T>, dim3((ni + 31) / 32, (nk + 7) / 8), b2, 0, st, g, q, c, fs, it_dev);
             }
             kend(7);
             break;

@@ -1424,6 +1424,24 @@ __device__ __forceinline__ void nucleation_body(Grid g, Fault<T> q, StepConst<T>
 }
 
 // ---------------------------------------------------------------- launch wrappers
+// A launch, with programmatic stream serialization when pdl is set: the kernel's CTAs may be
+// scheduled while the kernel before it drains, and wait in pdl_wait (which such a kernel starts
+// with) for its completion.
+template <class... K, class... A>
+inline cudaError_t launch_kernel(bool pdl, void (*kern)(K...), dim3 grid, dim3 blk, size_t smem, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = blk;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = pdl ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 template <class T>
 __global__ void __launch_bounds__(256)
 k_vel_fault(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ Fault<T> q,
@@ -1444,6 +1462,8 @@ k_vel_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, c
 
 template <class T>
 __global__ void k_vel_fs(Grid g, Fields<T> f) {
+    pdl_wait();
+    pdl_launch_dependents();
     vel_fs_body<T>(g, f, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -1541,6 +1561,8 @@ k_fault_bc(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, 
            const __grid_constant__ HistDesc h, int* status, int nfres, int tiles_x) {
     __shared__ T sm[FBC_SMEM];
     const int b = blockIdx.x;
+    pdl_wait();
+    pdl_launch_dependents();
     if (b < nfres) {
         const int sx = (g.nxt + 31) / 32;
         str_fs_body<T>(g, f, 1 + b % sx * 32 + threadIdx.x % 32, 1 + b / sx * (NT / 32) + threadIdx.x / 32);
@@ -1551,32 +1573,34 @@ k_fault_bc(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, 
 }
 
 template <class T, int LAW, int NT>
-inline void launch_fault_bc_n(cudaStream_t st, const Grid& g, const Fields<T>& f, const Fault<T>& q, const StepConst<T>& c,
+inline void launch_fault_bc_n(bool pdl, cudaStream_t st, const Grid& g, const Fields<T>& f, const Fault<T>& q, const StepConst<T>& c,
                               const FvwScalars& s, const int* it_dev, const HistDesc& h, int* status) {
     int nfres, tiles_x, tiles;
     fault_bc_grid(g, NT / 32, nfres, tiles_x, tiles);
-    k_fault_bc<T, LAW, NT><<<nfres + tiles, NT, 0, st>>>(g, f, q, c, s, it_dev, h, status, nfres, tiles_x);
+    launch_kernel(pdl, k_fault_bc<T, LAW, NT>, dim3(nfres + tiles), dim3(NT), 0, st, g, f, q, c, s, it_dev, h, status, nfres, tiles_x);
 }
 // FBC_THREADS threads a tile where two tiles fit an SM (slip weakening, FP32), and elsewhere where
 // there are no more tiles than SMs; 256 threads beyond that, since the kernel is then bound by
 // the warps it has in flight (rate-and-state, us: 50 tiles 13.9 against 20.5, 950 tiles 78
 // against 48.6).
 template <class T>
-inline void launch_fault_bc(int law, int nsm, cudaStream_t st, const Grid& g, const Fields<T>& f, const Fault<T>& q,
+inline void launch_fault_bc(bool pdl, int law, int nsm, cudaStream_t st, const Grid& g, const Fields<T>& f, const Fault<T>& q,
                             const StepConst<T>& c, const FvwScalars& s, const int* it_dev, const HistDesc& h, int* status) {
     int nfres, tiles_x, tiles;
     fault_bc_grid(g, 8, nfres, tiles_x, tiles);
     if (law == 0) {
-        if (sizeof(T) == 4 || tiles <= nsm) launch_fault_bc_n<T, 0, FBC_THREADS>(st, g, f, q, c, s, it_dev, h, status);
-        else launch_fault_bc_n<T, 0, 256>(st, g, f, q, c, s, it_dev, h, status);
+        if (sizeof(T) == 4 || tiles <= nsm) launch_fault_bc_n<T, 0, FBC_THREADS>(pdl, st, g, f, q, c, s, it_dev, h, status);
+        else launch_fault_bc_n<T, 0, 256>(pdl, st, g, f, q, c, s, it_dev, h, status);
     } else {
-        if (tiles <= nsm) launch_fault_bc_n<T, 1, FBC_THREADS>(st, g, f, q, c, s, it_dev, h, status);
-        else launch_fault_bc_n<T, 1, 256>(st, g, f, q, c, s, it_dev, h, status);
+        if (tiles <= nsm) launch_fault_bc_n<T, 1, FBC_THREADS>(pdl, st, g, f, q, c, s, it_dev, h, status);
+        else launch_fault_bc_n<T, 1, 256>(pdl, st, g, f, q, c, s, it_dev, h, status);
     }
 }
 
 template <class T>
 __global__ void k_nucleation(Grid g, Fault<T> q, StepConst<T> c, FvwScalars s, const int* it_dev) {
+    pdl_wait();
+    pdl_launch_dependents();
     nucleation_body<T>(g, q, c, s, it_dev, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 

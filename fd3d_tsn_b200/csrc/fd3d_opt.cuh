@@ -439,6 +439,58 @@ bool make_interior_maps(const Grid& g, const Fields<T>& f, VelMaps& V, StrMaps& 
     return ok;
 }
 
+// A half-step of a small grid in one launch: the interior tiles, the fault band and fault-plane
+// parts and the PML tiles in one grid (the three read only the other half-step's fields and write
+// disjoint cells), in that order, the longest-running CTAs first.  A step is then four launches
+// one after the other, each started while the one before drains, instead of eight over two
+// streams with two forks and joins: see small_step for where that is faster.
+template <class T, bool LAYERED>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
+k_vel_small(const __grid_constant__ VelMaps M, const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f,
+            const __grid_constant__ Fault<T> q, const __grid_constant__ PmlDesc D, const __grid_constant__ PmlAux<T> X,
+            const __grid_constant__ StepConst<T> c, int law, const __grid_constant__ FvwScalars s, int* it_dev, int* status,
+            int kchunk, dim3 ni, dim3 nf) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T* ring = reinterpret_cast<T*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
+    __shared__ __align__(8) uint64_t bars[TMA_NS];
+    pdl_wait();
+    pdl_launch_dependents();
+    int b = blockIdx.x;
+    const int n_int = (int)(ni.x * ni.y * ni.z), n_fault = (int)(nf.x * nf.y * nf.z);
+    if (b < n_int) {
+        tma_ring_init(bars);
+        unsigned pc = 0;
+        vel_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, b % ni.x, b / ni.x % ni.y, b / (ni.x * ni.y), ring, bars, pc, status);
+    } else if ((b -= n_int) < n_fault) {
+        vel_fault_body<T>(g, f, q, c, law, s, it_dev, status, b % nf.x, b / nf.x % nf.y, b / (nf.x * nf.y));
+    } else {
+        vel_pml_tile<T, false, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), 0u, status);
+    }
+}
+
+template <class T, bool LAYERED>
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
+k_str_small(const __grid_constant__ StrMaps M, const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f,
+            const __grid_constant__ Fault<T> q, const __grid_constant__ PmlDesc D, const __grid_constant__ PmlAux<T> X,
+            const __grid_constant__ StepConst<T> c, int* status, int kchunk, dim3 ni, dim3 nf) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    T* ring = reinterpret_cast<T*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
+    __shared__ __align__(8) uint64_t bars[TMA_NS];
+    pdl_wait();
+    pdl_launch_dependents();
+    int b = blockIdx.x;
+    const int n_int = (int)(ni.x * ni.y * ni.z), n_fault = (int)(nf.x * nf.y * nf.z);
+    if (b < n_int) {
+        tma_ring_init(bars);
+        unsigned pc = 0;
+        str_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, b % ni.x, b / ni.x % ni.y, b / (ni.x * ni.y), ring, bars, pc, status);
+    } else if ((b -= n_int) < n_fault) {
+        str_fault_body<T>(g, f, q, c, b % nf.x, b / nf.x % nf.y, b / (nf.x * nf.y));
+    } else {
+        str_pml_tile<T, false, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), 0u, status);
+    }
+}
+
 template <class T>
 bool prepare_tma_kernels() {
     const int vs = TMA_NS * VelSlot::ELEMS * (int)sizeof(T) + TMA_SMEM_PAD, ss = str_ring_bytes<T, false>(),
@@ -447,8 +499,51 @@ bool prepare_tma_kernels() {
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_vel_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssl) == cudaSuccess;
+    ok &= cudaFuncSetAttribute(k_vel_small<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
+    ok &= cudaFuncSetAttribute(k_vel_small<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
+    ok &= cudaFuncSetAttribute(k_str_small<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) == cudaSuccess;
+    ok &= cudaFuncSetAttribute(k_str_small<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssl) == cudaSuccess;
     if (!ok) cudaGetLastError();
     return ok;
+}
+
+// CTAs of one of those launches, and its grids of interior tiles (ni) and fault parts (nf)
+inline unsigned half_small_grid(bool stress, const InteriorCfg& cfg, const Grid& g, const PmlDesc& D, int& kch, dim3& ni, dim3& nf) {
+    const int nxT = g.nxt - 2 * g.nabc, nyI = g.nyt - 2 - g.nabc, nzT = interior_nz(g);
+    const unsigned cx = (nxT + 31) / 32, cy = (nyI + 7) / 8;
+    kch = interior_kchunk(cfg, stress ? cfg.kchunk_str : cfg.kchunk, (long long)cx * cy, nzT);
+    ni = dim3(cx, cy, (nzT + kch - 1) / kch);
+    nf = dim3(stress ? (nxT + 31) / 32 : (g.nxt + 31) / 32, (nzT + 7) / 8, stress ? STR_FAULT_PARTS : VEL_FAULT_PARTS);
+    return ni.x * ni.y * ni.z + nf.x * nf.y * nf.z + (unsigned)(D.cum[PML_MAXS] / PML_TILE);
+}
+// Whether a model takes one launch per half-step: up to twelve CTAs per SM, three waves at the
+// four that fit (FP32).  Beyond that the interior CTAs miss the fifth and sixth place per SM that
+// they have in a launch of their own.  A solve, one launch / separate launches: 0.2 K CTAs 1.76 /
+// 1.95 ms, 1.4 K 36.7 / 38.7, 1.5 K 13.4 / 15.1 (rate-and-state), FP64 1.4 K 13.9 / 14.1; 2.7 K 88.4 /
+// 87.7 and 18.7 / 17.7, 9 K 22.3 / 21.7.
+inline bool small_step(const InteriorCfg& cfg, const Grid& g, const PmlDesc& D) {
+    int kch;
+    dim3 ni, nf;
+    return half_small_grid(false, cfg, g, D, kch, ni, nf) <= 12u * (unsigned)cfg.nsm;
+}
+
+// the two half-steps of a small grid (k_vel_small, k_str_small)
+template <class T>
+void launch_half_small(bool stress, const VelMaps& V, const StrMaps& S, const InteriorCfg& cfg, const Grid& g,
+                       const Fields<T>& f, const Fault<T>& q, const PmlDesc& D, const PmlAux<T>& X, const StepConst<T>& c,
+                       int law, const FvwScalars& s, int* it_dev, int* status, cudaStream_t st) {
+    int kch;
+    dim3 ni, nf;
+    const dim3 grid(half_small_grid(stress, cfg, g, D, kch, ni, nf)), blk(32, 8);
+    if (!stress) {
+        const size_t sm = TMA_NS * VelSlot::ELEMS * sizeof(T) + TMA_SMEM_PAD;
+        if (f.lay) launch_kernel(true, k_vel_small<T, true>, grid, blk, sm, st, V, g, f, q, D, X, c, law, s, it_dev, status, kch, ni, nf);
+        else launch_kernel(true, k_vel_small<T, false>, grid, blk, sm, st, V, g, f, q, D, X, c, law, s, it_dev, status, kch, ni, nf);
+    } else if (f.lay) {
+        launch_kernel(true, k_str_small<T, true>, grid, blk, str_ring_bytes<T, true>(), st, S, g, f, q, D, X, c, status, kch, ni, nf);
+    } else {
+        launch_kernel(true, k_str_small<T, false>, grid, blk, str_ring_bytes<T, false>(), st, S, g, f, q, D, X, c, status, kch, ni, nf);
+    }
 }
 
 template <class T>
