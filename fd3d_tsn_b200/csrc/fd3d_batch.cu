@@ -163,8 +163,10 @@ k_batch(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
         for (int ph = 0; ph < NPHASE; ++ph) {
             const int b0 = pbeg[ph], b1 = pbeg[ph + 1];
             if (b0 == b1) continue;  // an empty phase needs no barrier (uniform over the grid)
+            Work next = work[min(b0 + (int)blockIdx.x, b1 - 1)];
             for (int w = b0 + blockIdx.x; w < b1; w += nb) {
-                const Work it = work[w];
+                const Work it = next;
+                next = work[min(w + (int)nb, b1 - 1)];  // (in flight during this item)
                 const int m = it.tm >> 8, type = it.tm & 255;
                 if (s >= limit[m]) continue;  // uniform over the CTA: the item belongs to one model
                 const ModelDev& M = models[m];
@@ -340,22 +342,6 @@ __global__ void k_or_status(int* const* __restrict__ st, int n, int* out) {
     if ((threadIdx.x & 31) == 0) atomicOr(&acc, v);
     __syncthreads();
     if (threadIdx.x == 0) *out = acc;
-}
-
-// 1-D layered medium -> padded 3-D arrays of one model
-__global__ void k_fill_layers(Grid g, float* lam, float* mu, float* d, const float* lk, const float* mk,
-                              const float* dk) {
-    const long long n = g.plane * g.nzt;
-    for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < n; q += (long long)gridDim.x * blockDim.x) {
-        const int k = (int)(q / g.plane);
-        const long long r = q - (long long)k * g.plane;
-        const int x = (int)(r % g.px), j = (int)(r / g.px);
-        (void)j;
-        const bool in = (x >= g.off) && (x < g.off + g.nxt);
-        lam[q] = in ? lk[k] : 0.f;
-        mu[q] = in ? mk[k] : 0.f;
-        d[q] = in ? dk[k] : 0.f;
-    }
 }
 
 // initial fault state (fd3d_theo.f90:59-88) on top of zeroed arrays
@@ -1048,7 +1034,7 @@ int fd3d_batch_add(fd3d_batch* b, const fd3d_params* pin, const double* lam_k, c
         lay[4 * p.nzt + k] = d.c.dt / lay[2 * p.nzt + k];
     }
     BCK(cudaMemcpyAsync(layers, lay.data(), lay.size() * sizeof(float), cudaMemcpyHostToDevice, b->sst));
-    k_fill_layers<<<1024, 256, 0, b->sst>>>(d.g, lam, mu, dd, layers, layers + p.nzt, layers + 2 * p.nzt);
+    k_fill_layers<float><<<1184, 256, 0, b->sst>>>(d.g, lam, mu, dd, layers);
     BCK(cudaGetLastError());
     std::vector<std::vector<float>> F;
     std::vector<double> pz, px;

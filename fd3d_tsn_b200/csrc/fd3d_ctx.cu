@@ -470,19 +470,14 @@ struct Ctx : CtxBase {
 
     int upload_medium_layers(const double* l, const double* m, const double* d) override {
         if (!l || !m || !d) return FD3D_ERR_ARG;
-        std::vector<T> slab_((size_t)g.plane);
-        T* dst[3] = {(T*)f.lam, (T*)f.mu, (T*)f.d};
+        std::vector<T> lay(3 * (size_t)p.nzt);
         const double* src[3] = {l, m, d};
         for (int a = 0; a < 3; ++a)
-            for (int k = g.kofs; k < g.kofs + g.nzl; ++k) {
-                std::fill(slab_.begin(), slab_.end(), (T)0);
-                const T v = (T)src[a][k];
-                for (int j = 0; j < p.nyt; ++j)
-                    for (int i = 0; i < p.nxt; ++i) slab_[(size_t)g.px * j + g.off + i] = v;
-                CK(cudaMemcpyAsync(dst[a] + (size_t)g.plane * k, slab_.data(), (size_t)g.plane * sizeof(T),
-                                   cudaMemcpyHostToDevice, st));
-                CK(cudaStreamSynchronize(st));
-            }
+            for (int k = 0; k < p.nzt; ++k) lay[(size_t)a * p.nzt + k] = (T)src[a][k];
+        // staged in the profile table, which medium_uploaded writes after this
+        CK(cudaMemcpyAsync(dlay, lay.data(), lay.size() * sizeof(T), cudaMemcpyHostToDevice, st));
+        k_fill_layers<T><<<1184, 256, 0, st>>>(g, (T*)f.lam, (T*)f.mu, (T*)f.d, dlay);
+        CK(cudaGetLastError());
         return medium_uploaded();
     }
 

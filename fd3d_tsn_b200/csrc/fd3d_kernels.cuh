@@ -1423,6 +1423,26 @@ __device__ __forceinline__ void nucleation_body(Grid g, Fault<T> q, StepConst<T>
     q.T0X[g.at2(i, k)] = (T)(base + s.perturb * FXZ * GT);
 }
 
+// ---------------------------------------------------------------- set-up
+// A 1-D layered medium (lam, mu, d per plane in lay, nzt values each) into the padded 3-D
+// arrays, whose row padding stays 0; a CTA per row, bound by the stores.  The whole upload call of
+// a 0.9 M cell model takes 0.07 ms (5.5 ms with planes filled on the host and copied one by one).
+template <class T>
+__global__ void k_fill_layers(Grid g, T* lam, T* mu, T* d, const T* lay) {
+    const int nrows = g.nyt * g.nzl;  // rows of the stored planes, from kofs+1
+    for (int r = blockIdx.x; r < nrows; r += gridDim.x) {
+        const int k = g.kofs + 1 + r / g.nyt, j = 1 + r % g.nyt;
+        const long long row = g.at(1, j, k) - g.off;
+        const T l = lay[k - 1], m = lay[g.nzt + k - 1], dd = lay[2 * g.nzt + k - 1];
+        for (int x = threadIdx.x; x < g.px; x += blockDim.x) {
+            const bool in = x >= g.off && x < g.off + g.nxt;
+            lam[row + x] = in ? l : (T)0;
+            mu[row + x] = in ? m : (T)0;
+            d[row + x] = in ? dd : (T)0;
+        }
+    }
+}
+
 // ---------------------------------------------------------------- launch wrappers
 // A launch, with programmatic stream serialization when pdl is set: the kernel's CTAs may be
 // scheduled while the kernel before it drains, and wait in pdl_wait (which such a kernel starts
