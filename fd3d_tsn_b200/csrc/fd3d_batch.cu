@@ -241,16 +241,18 @@ __global__ void k_check_grid_barrier(BatchSync* sync, int* status) {
 // step limit is reached return at once).  Each kernel gets its own register and
 // shared-memory budget, so each region runs at its own occupancy.
 constexpr int NTYPES = 10;
+// dynamic shared memory of the kernels with interior tiles (1-D media only)
+constexpr int VEL_RING = TMA_NS * VelSlot::ELEMS * (int)sizeof(float) + TMA_SMEM_PAD, STR_RING = str_ring_bytes<float, true>();
 
-__device__ __forceinline__ bool item_live(const Work& it, const int* limit, const int* run_step, int& m) {
+__device__ __forceinline__ bool item_live(const Work& it, const int* limit, const int* run_step, int ofs, int& m) {
     m = it.tm >> 8;
-    return *run_step < limit[m];
+    return *run_step + ofs < limit[m];
 }
 
 template <bool STRESS>
 __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
                                               const Work* __restrict__ work, int b0, const int* __restrict__ limit,
-                                              const int* run_step, int kchunk, int* gstatus) {
+                                              const int* run_step, int ofs, int kchunk, int* gstatus) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float* ring = reinterpret_cast<float*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
     __shared__ __align__(8) uint64_t bars[TMA_NS];
@@ -258,7 +260,7 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
     pdl_launch_dependents();
     const Work it = work[b0 + blockIdx.x];
     int m;
-    if (!item_live(it, limit, run_step, m)) return;
+    if (!item_live(it, limit, run_step, ofs, m)) return;
     __shared__ ModelPar M;
     load_par(M, models[m]);
     tma_ring_init(bars);
@@ -274,7 +276,7 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
 template <bool STRESS>
 __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict__ models,
                                                       const Work* __restrict__ work, int b0,
-                                                      const int* __restrict__ limit, const int* run_step,
+                                                      const int* __restrict__ limit, const int* run_step, int ofs,
                                                       int* gstatus) {
     __shared__ __align__(128) float sm[PML_TILE * (STRESS ? AUX_NS : AUX_NV)];
     __shared__ __align__(8) uint64_t bar;
@@ -282,37 +284,77 @@ __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict
     pdl_launch_dependents();
     const Work it = work[b0 + blockIdx.x];
     int m;
-    if (!item_live(it, limit, run_step, m)) return;
+    if (!item_live(it, limit, run_step, ofs, m)) return;
     __shared__ ModelPar M;
     load_par(M, models[m]);
     if (STRESS) str_pml_tile<float, false, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
     else vel_pml_tile<float, false, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
 }
 
+// A half-step of a small batch in one launch: the interior, fault-band and PML items (contiguous
+// in the list by type), as k_vel_small / k_str_small do for one model.
+template <bool STRESS>
+__global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
+                                                  const Work* __restrict__ work, int b0, const int* __restrict__ limit,
+                                                  const int* run_step, int ofs, int kchunk, int* gstatus) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    float* ring = reinterpret_cast<float*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
+    __shared__ __align__(8) uint64_t bars[TMA_NS];
+    __shared__ ModelPar P;
+    const Work it = work[b0 + blockIdx.x];
+    pdl_wait();
+    pdl_launch_dependents();
+    int m;
+    if (!item_live(it, limit, run_step, ofs, m)) return;
+    const ModelDev& M = models[m];
+    load_par(P, M);
+    switch (it.tm & 255) {
+        case W_VEL_INT:
+        case W_STR_INT: {
+            tma_ring_init(bars);
+            unsigned pc = 0;
+            if (STRESS)
+                str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc, gstatus);
+            else
+                vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc, gstatus);
+            break;
+        }
+        case W_VEL_FAULT:
+        case W_STR_FAULT:
+            if (STRESS) str_fault_body<float>(P.g, P.f, M.q, P.c, it.bx, it.by, it.bz);
+            else vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
+            break;
+        default:
+            if (STRESS) str_pml_tile<float, false, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), 0u, gstatus);
+            else vel_pml_tile<float, false, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), 0u, gstatus);
+    }
+}
+
 // Plane items in three kernels by register need, so that light items are not held to a
-// heavy body's register count: KIND 1 the fused fault-BC tiles (and the fres items launched
+// heavy body's register count: KIND 3 the fused fault-BC tiles of slip-weakening models with a
+// thread per node and role (small batches: see launch_fault_bc), KIND 1 the fused fault-BC tiles (and the fres items launched
 // with them, 78 registers), KIND 2 the fault-band velocity (its rate-and-state Newton path
 // takes 114), KIND 0 the rest (free surface, stress fault band, nucleation ramp).
 template <int KIND>
-__global__ void __launch_bounds__(256, KIND == 1 ? 3 : 1) k_bplane(const ModelDev* __restrict__ models, const Work* __restrict__ work,
-                                                int b0, const int* __restrict__ limit, const int* run_step) {
-    __shared__ float sm[KIND == 1 ? FBC_SMEM : 1];
+__global__ void __launch_bounds__(KIND == 3 ? FBC_THREADS : 256, KIND == 3 ? 2 : KIND == 1 ? 3 : 1) k_bplane(const ModelDev* __restrict__ models, const Work* __restrict__ work,
+                                                int b0, const int* __restrict__ limit, const int* run_step, int ofs) {
+    __shared__ float sm[KIND & 1 ? FBC_SMEM : 1];
     pdl_wait();
     pdl_launch_dependents();
     const Work it = work[b0 + blockIdx.x];
     int m;
-    if (!item_live(it, limit, run_step, m)) return;
+    if (!item_live(it, limit, run_step, ofs, m)) return;
     const ModelDev& M = models[m];
     if (KIND == 2) {
         if ((it.tm & 255) == W_VEL_FAULT)
             vel_fault_body<float>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
         return;
     }
-    if (KIND == 1) {
+    if (KIND & 1) {
         if ((it.tm & 255) == W_FBC)
-            fault_bc_body<float, 256>(M.g, M.f, M.q, M.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by, sm,
-                                      threadIdx.y * 32 + threadIdx.x);
-        else if ((it.tm & 255) == W_STR_FS)
+            fault_bc_body<float, KIND == 3 ? FBC_THREADS : 256>(M.g, M.f, M.q, M.c, KIND == 3 ? 0 : M.law, M.fs, M.it_dev, M.h,
+                                                                M.status, it.bx, it.by, sm, threadIdx.y * 32 + threadIdx.x);
+        else if ((it.tm & 255) == W_STR_FS && threadIdx.y < 8)
             str_fs_body<float>(M.g, M.f, 1 + it.bx * 32 + threadIdx.x, 1 + it.by * 8 + threadIdx.y);
         return;
     }
@@ -325,10 +367,10 @@ __global__ void __launch_bounds__(256, KIND == 1 ? 3 : 1) k_bplane(const ModelDe
     }
 }
 
-__global__ void k_step_end(int* run_step) {
+__global__ void k_step_end(int* run_step, int n) {
     pdl_wait();
     pdl_launch_dependents();
-    *run_step += 1;
+    *run_step += n;
 }
 
 // OR of the live models' device status words into out (one read-back per sync)
@@ -641,11 +683,27 @@ int build_work(fd3d_batch* b) {
     return FD3D_OK;
 }
 
+// Whether a half-step of the batch is one launch (k_bhalf), its launches overlapped with the ones
+// before: up to 120 items per SM.  Beyond that the launches' tails no longer count, and the interior
+// tiles run best at the five and six CTAs per SM of their own kernel.  us a step, one launch /
+// separate: 0.7 K items (1 model) 48 / 68, 4 K 140 / 166 (32 planes a tile 146 / 199), 12 K 386 /
+// 400, 16 K 495 / 506; 33 K (32 models) 967 / 946.
+bool merged_step(const fd3d_batch* b) {
+    return !b->branches && b->tbeg[W_VEL_FS] - b->tbeg[W_VEL_INT] <= 120 * b->nsm;
+}
+bool all_slip_weakening(const fd3d_batch* b) {
+    for (const Model& M : b->models)
+        if (M.live && M.p.law != FD3D_LAW_SW) return false;
+    return true;
+}
+
 // one time step of the graph schedule on b->st (fork/join over the side streams)
-int enqueue_graph_step(fd3d_batch* b) {
+int enqueue_graph_step(fd3d_batch* b, int ofs) {
     const dim3 blk(32, 8);
     const int kc = b->tun.kchunk;
-    const bool pdl = b->pdl && !b->branches;  // on the one stream only
+    const bool small = merged_step(b);
+    const bool pdl = small || (b->pdl && !b->branches);  // on the one stream only
+    const bool wide_fbc = small && all_slip_weakening(b);
     cudaError_t err = cudaSuccess;             // the first failed launch
     auto chk = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
     auto n_of = [&](int t) { return b->tbeg[t + 1] - b->tbeg[t]; };
@@ -656,9 +714,11 @@ int enqueue_graph_step(fd3d_batch* b) {
         const int* rs = b->d_run_step;
         const ModelDev* md = b->d_models;
         const Work* wt = b->d_work_t;
-        if (t0 <= W_FBC && W_FBC < t1) chk(launch_kernel(pdl, k_bplane<1>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
-        else if (t0 == W_VEL_FAULT) chk(launch_kernel(pdl, k_bplane<2>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
-        else chk(launch_kernel(pdl, k_bplane<0>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs));
+        if (wide_fbc && t0 <= W_FBC && W_FBC < t1)
+            chk(launch_kernel(pdl, k_bplane<3>, dim3(n), dim3(32, FBC_THREADS / 32), 0, s, md, wt, b->tbeg[t0], lim, rs, ofs));
+        else if (t0 <= W_FBC && W_FBC < t1) chk(launch_kernel(pdl, k_bplane<1>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs, ofs));
+        else if (t0 == W_VEL_FAULT) chk(launch_kernel(pdl, k_bplane<2>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs, ofs));
+        else chk(launch_kernel(pdl, k_bplane<0>, dim3(n), blk, 0, s, md, wt, b->tbeg[t0], lim, rs, ofs));
     };
     // the fault-band and PML sweeps on side streams beside the interior sweep, or (branches
     // off) all on the main stream one after another
@@ -666,6 +726,13 @@ int enqueue_graph_step(fd3d_batch* b) {
     for (int half = 0; half < 2; ++half) {
         const int ti = half ? W_STR_INT : W_VEL_INT, tf = half ? W_STR_FAULT : W_VEL_FAULT;
         const int tp = half ? W_STR_PML : W_VEL_PML, tfs = half ? W_STR_FS : W_VEL_FS;
+        const size_t sm = half ? STR_RING : VEL_RING;
+        if (small) {
+            chk(launch_kernel(true, half ? k_bhalf<true> : k_bhalf<false>, dim3(b->tbeg[tfs] - b->tbeg[ti]), blk, sm, b->st, b->d_models,
+                              b->d_maps, b->d_work_t, b->tbeg[ti], b->d_limit, b->d_run_step, ofs, kc, b->d_status));
+            plane(b->st, tfs, half ? W_FBC + 1 : tfs + 1);
+            continue;
+        }
         if (b->branches) {
             BCK(cudaEventRecord(b->evf[0], b->st));
             BCK(cudaStreamWaitEvent(b->side[0], b->evf[0], 0));
@@ -677,14 +744,13 @@ int enqueue_graph_step(fd3d_batch* b) {
         const int* lim = b->d_limit;
         const int* rs = b->d_run_step;
         if (n_of(ti) > 0) {
-            const size_t sm = tma_ring_bytes<float>();
-            if (half) chk(launch_kernel(pdl, k_bint<true>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, kc, b->d_status));
-            else chk(launch_kernel(pdl, k_bint<false>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, kc, b->d_status));
+            if (half) chk(launch_kernel(pdl, k_bint<true>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, ofs, kc, b->d_status));
+            else chk(launch_kernel(pdl, k_bint<false>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, ofs, kc, b->d_status));
         }
         plane(s0, tf, tf + 1);
         if (n_of(tp) > 0) {
-            if (half) chk(launch_kernel(pdl, k_bpml<true>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, b->d_status));
-            else chk(launch_kernel(pdl, k_bpml<false>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, b->d_status));
+            if (half) chk(launch_kernel(pdl, k_bpml<true>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, ofs, b->d_status));
+            else chk(launch_kernel(pdl, k_bpml<false>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, ofs, b->d_status));
         }
         if (b->branches) {
             BCK(cudaEventRecord(b->evf[1], b->side[0]));
@@ -695,7 +761,6 @@ int enqueue_graph_step(fd3d_batch* b) {
         plane(b->st, tfs, half ? W_FBC + 1 : tfs + 1);  // after the stresses: fres and the fault BC tiles
     }
     plane(b->st, W_NUC, W_NUC + 1);
-    chk(launch_kernel(pdl, k_step_end, dim3(1), dim3(1), 0, b->st, b->d_run_step));
     BCK(err);
     BCK(cudaGetLastError());
     return FD3D_OK;
@@ -712,7 +777,8 @@ int get_batch_graph(fd3d_batch* b, int g, cudaGraphExec_t* out) {
         cudaGraph_t gr;
         BCK(cudaStreamBeginCapture(b->st, cudaStreamCaptureModeThreadLocal));
         int rc = FD3D_OK;
-        for (int s = 0; s < (32 >> g) && rc == FD3D_OK; ++s) rc = enqueue_graph_step(b);
+        for (int s = 0; s < (32 >> g) && rc == FD3D_OK; ++s) rc = enqueue_graph_step(b, s);
+        k_step_end<<<1, 1, 0, b->st>>>(b->d_run_step, 32 >> g);
         cudaError_t e = cudaStreamEndCapture(b->st, &gr);
         if (rc) {
             if (e == cudaSuccess) cudaGraphDestroy(gr);
@@ -878,10 +944,11 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
         if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return fail(FD3D_ERR_CUDA);
     for (cudaEvent_t& e : b->evf)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(FD3D_ERR_CUDA);
-    if (cudaFuncSetAttribute(k_bint<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_ring_bytes<float>()) !=
-            cudaSuccess ||
-        cudaFuncSetAttribute(k_bint<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_ring_bytes<float>()) !=
-            cudaSuccess) {
+    auto ring_ok = [](auto k, int bytes) {
+        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+    };
+    if (!ring_ok(k_bint<false>, VEL_RING) || !ring_ok(k_bint<true>, STR_RING) || !ring_ok(k_bhalf<false>, VEL_RING) ||
+        !ring_ok(k_bhalf<true>, STR_RING)) {
         cudaGetLastError();
         return fail(FD3D_ERR_CUDA);
     }
