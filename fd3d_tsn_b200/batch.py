@@ -144,8 +144,8 @@ class Batch:
         _ck(lib().fd3d_batch_set_tuning(self.h, kchunk, ctas_per_sm), "fd3d_batch_set_tuning")
 
     def set_schedule(self, mode: str):
-        """"persistent" (one cooperative kernel per run) or "graph" (CUDA graphs of
-        per-region kernels over all models)."""
+        """"graph" (CUDA graphs of kernels over all models) or "persistent", which runs the
+        same launches."""
         _ck(lib().fd3d_batch_set_schedule(self.h, SCHEDULES[mode]), "fd3d_batch_set_schedule")
 
     def tuning(self):

@@ -2,10 +2,8 @@
 //
 // Models of uneven size live in one device arena (first-fit, 256-byte aligned blocks,
 // each with its own padded pitch).  Their work is a host-built list of (model, tile)
-// items.  Two schedules run it: the persistent one is one cooperative kernel per run
-// whose CTAs walk the items phase by phase and meet at a bounded grid-wide barrier
-// between phases; the graph one replays CUDA graphs of per-region kernels over all
-// models (see k_bint).  A time step has five phases:
+// items, run by replaying CUDA graphs of kernels over all models: one per region (see
+// k_bint), or one per half-step for a small batch (k_bhalf).  A time step has five phases:
 //   0 velocity: interior tiles, fault band + fault plane, PML chunks
 //   1 free-surface velocity ghosts
 //   2 stress: interior tiles, fault band + fault plane, PML chunks
@@ -14,9 +12,13 @@
 //   4 nucleation ramp (rate-and-state models that have one; an empty phase is skipped)
 // Every item runs the same __device__ body as the single-model launch of that region
 // (fd3d_kernels.cuh / fd3d_opt.cuh), so a model's results do not depend on which other
-// models share the launch.  The schedule, the z-extent of the interior tiles and (for
-// the persistent kernel) the number of CTAs per SM are picked by an autotuner that
-// times the candidates on the live batch (and resets the models after).
+// models share the launch.  The z-extent of the interior tiles is picked by an autotuner
+// that times the candidates on the live batch (and resets the models after).
+//
+// FD3D_BATCH_PERSISTENT is accepted and runs the same launches.  One cooperative kernel whose CTAs
+// walked the items between grid barriers was slower at every size, us a step against these:
+// 1 model 70 / 48, 2 models 123 / 84, 4 models 198 / 146, 16 models 605 / 495, 64 models 2224 / 1820
+// (its one kernel ran every item at the registers of the largest body, 3 CTAs per SM).
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <chrono>
@@ -92,7 +94,7 @@ struct BatchSync {
 
 constexpr int BARRIER_SPIN_LIMIT = 1 << 22;
 
-// Sense-counting grid barrier with a bounded spin; false if this CTA gave up (or another did).
+// Sense-counting grid barrier with a bounded spin (of fd3d_check_waits); false if this CTA gave up (or another did).
 __device__ bool grid_barrier(BatchSync* b, unsigned nblocks, int* status) {
     __shared__ int ok;
     __syncthreads();
@@ -139,83 +141,6 @@ struct ModelMaps {  // TMA descriptors of one model's interior sweeps (global me
     StrMaps s;
 };
 
-#ifndef FD3D_BATCH_MINB
-#define FD3D_BATCH_MINB 3
-#endif
-constexpr int BATCH_MIN_CTAS = FD3D_BATCH_MINB;  // register cap so that this many CTAs of 256 threads fit an SM
-
-__global__ void __launch_bounds__(256, BATCH_MIN_CTAS)
-k_batch(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps, const Work* __restrict__ work,
-        const int* __restrict__ pbeg, const int* __restrict__ limit, int nsteps, int kchunk, BatchSync* sync,
-        int* gstatus) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    float* ring = reinterpret_cast<float*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
-    __shared__ __align__(8) uint64_t bars[TMA_NS];
-    __shared__ __align__(8) uint64_t pbar;  // PML tiles staged through the ring memory
-    if (threadIdx.x == 0 && threadIdx.y == 0) mbar_init(smem_addr(&pbar), 1);
-    tma_ring_init(bars);
-    __shared__ ModelPar P;
-    int pm = -1;      // the model that P holds
-    unsigned pt = 0;  // PML tiles this CTA has staged (mbarrier phase = pt & 1)
-    unsigned pc = 0;  // planes this CTA has put through its ring
-    const unsigned nb = gridDim.x;
-    for (int s = 0; s < nsteps; ++s) {
-        for (int ph = 0; ph < NPHASE; ++ph) {
-            const int b0 = pbeg[ph], b1 = pbeg[ph + 1];
-            if (b0 == b1) continue;  // an empty phase needs no barrier (uniform over the grid)
-            Work next = work[min(b0 + (int)blockIdx.x, b1 - 1)];
-            for (int w = b0 + blockIdx.x; w < b1; w += nb) {
-                const Work it = next;
-                next = work[min(w + (int)nb, b1 - 1)];  // (in flight during this item)
-                const int m = it.tm >> 8, type = it.tm & 255;
-                if (s >= limit[m]) continue;  // uniform over the CTA: the item belongs to one model
-                const ModelDev& M = models[m];
-                if (m != pm) load_par(P, M);  // (the last item ended with a barrier)
-                pm = m;
-                bool ok = true;
-                switch (type) {
-                    case W_VEL_INT:
-                        ok = vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz,
-                                                                ring, bars, pc, gstatus);
-                        break;
-                    case W_VEL_FAULT:
-                        vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
-                        break;
-                    case W_VEL_PML:
-                        ok = vel_pml_tile<float, false, true>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(&pbar),
-                                                             pt & 1u, gstatus);
-                        ++pt;
-                        break;
-                    case W_VEL_FS: vel_fs_body<float>(P.g, P.f, it.bx, it.by, 0); break;
-                    case W_STR_INT:
-                        ok = str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz,
-                                                                ring, bars, pc, gstatus);
-                        break;
-                    case W_STR_FAULT: str_fault_body<float>(P.g, P.f, M.q, P.c, it.bx, it.by, it.bz); break;
-                    case W_STR_PML:
-                        ok = str_pml_tile<float, false, true>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(&pbar),
-                                                             pt & 1u, gstatus);
-                        ++pt;
-                        break;
-                    case W_STR_FS: str_fs_body<float>(P.g, P.f, 1 + it.bx * 32 + threadIdx.x, 1 + it.by * 8 + threadIdx.y); break;
-                    case W_FBC:
-                        fault_bc_body<float, 256>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.h, M.status, it.bx, it.by,
-                                                  ring, threadIdx.y * 32 + threadIdx.x);
-                        break;
-                    case W_NUC: nucleation_body<float>(P.g, M.q, P.c, M.fs, M.it_dev, it.bx, it.by, 0); break;
-                    default: break;
-                }
-                if (!ok) {  // a ring wait timed out: make every CTA leave at its next barrier
-                    if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(&sync->abort, 1);
-                    return;
-                }
-                __syncthreads();  // the next item may reuse the ring
-            }
-            if (!grid_barrier(sync, nb, gstatus)) return;
-        }
-    }
-}
-
 // ---------------------------------------------------------------- self-test of the waits
 // An mbarrier phase that no copy or arrival completes, and a grid barrier that one CTA
 // never reaches: both waits must give up by their bound, record ST_TIMEOUT and return,
@@ -234,11 +159,10 @@ __global__ void k_check_grid_barrier(BatchSync* sync, int* status) {
 }
 
 // ---------------------------------------------------------------- graph schedule
-// The same items as k_batch, one kernel per region and step, every CTA one item.
-// A CUDA graph holds a chunk of steps: per step the interior, fault-band and PML
-// sweeps of a half-step run as three parallel branches, the plane regions follow in
-// order, and k_step_end advances the run's step counter (items of a model whose
-// step limit is reached return at once).  Each kernel gets its own register and
+// One kernel per region and step, every CTA one item.
+// A CUDA graph holds a chunk of steps, its launches in series; the ofs-th step of a graph is
+// step *run_step + ofs of the run, and k_step_end advances the counter at the graph's end
+// (items of a model whose step limit is reached return at once).  Each kernel gets its own register and
 // shared-memory budget, so each region runs at its own occupancy.
 constexpr int NTYPES = 10;
 // dynamic shared memory of the kernels with interior tiles (1-D media only)
@@ -264,13 +188,10 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
     __shared__ ModelPar M;
     load_par(M, models[m]);
     tma_ring_init(bars);
-    unsigned pc = 0;
-    if (STRESS)
-        str_interior_tma_body<float, true>(maps[m].s, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc,
-                                           gstatus);
+        if (STRESS)
+        str_interior_tma_body<float, true>(maps[m].s, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
     else
-        vel_interior_tma_body<float, true>(maps[m].v, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc,
-                                           gstatus);
+        vel_interior_tma_body<float, true>(maps[m].v, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
 }
 
 template <bool STRESS>
@@ -287,8 +208,8 @@ __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict
     if (!item_live(it, limit, run_step, ofs, m)) return;
     __shared__ ModelPar M;
     load_par(M, models[m]);
-    if (STRESS) str_pml_tile<float, false, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
-    else vel_pml_tile<float, false, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), 0u, gstatus);
+    if (STRESS) str_pml_tile<float, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
+    else vel_pml_tile<float, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
 }
 
 // A half-step of a small batch in one launch: the interior, fault-band and PML items (contiguous
@@ -312,11 +233,10 @@ __global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ m
         case W_VEL_INT:
         case W_STR_INT: {
             tma_ring_init(bars);
-            unsigned pc = 0;
-            if (STRESS)
-                str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc, gstatus);
+                        if (STRESS)
+                str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
             else
-                vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, pc, gstatus);
+                vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
             break;
         }
         case W_VEL_FAULT:
@@ -325,8 +245,8 @@ __global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ m
             else vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
             break;
         default:
-            if (STRESS) str_pml_tile<float, false, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), 0u, gstatus);
-            else vel_pml_tile<float, false, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), 0u, gstatus);
+            if (STRESS) str_pml_tile<float, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
+            else vel_pml_tile<float, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
     }
 }
 
@@ -487,7 +407,7 @@ enum { MODE_PERSISTENT = FD3D_BATCH_PERSISTENT, MODE_GRAPH = FD3D_BATCH_GRAPH };
 
 struct Tuning {
     int kchunk = 16;
-    int per_sm = 0;     // CTAs per SM (0 = occupancy limit), persistent schedule
+    int per_sm = 0;     // CTAs per SM the caller set (kept for fd3d_batch_get_tuning; no launch depends on it)
     int mode = MODE_GRAPH;
 };
 
@@ -503,14 +423,9 @@ struct fd3d_batch {
     ModelDev* d_models = nullptr;
     ModelMaps* d_maps = nullptr;
     int* d_limit = nullptr;
-    int* d_pbeg = nullptr;
-    Work* d_work = nullptr;
-    size_t work_cap = 0;
-    BatchSync* d_sync = nullptr;
     int* d_status = nullptr;
     bool dirty = true;           // work list must be rebuilt
     std::vector<Work> work;
-    int pbeg[NPHASE + 1] = {0};
     Tuning tun;
     int max_active = 0;          // CTAs per SM at the occupancy limit
     int nsm = 0;
@@ -539,7 +454,6 @@ struct fd3d_batch {
     int* d_status_or = nullptr;
     Work* h_stage = nullptr;     // page-locked staging of the work lists
     size_t stage_cap = 0;
-    bool work_t_ok = false;      // the type-sorted list matches the work list
 };
 
 namespace {
@@ -602,8 +516,7 @@ int stage_items(fd3d_batch* b, size_t n) {
     return FD3D_OK;
 }
 
-// The items of the live models grouped by type, for the graph schedule (built when a
-// graph run needs them after the work list changed)
+// The items of the live models grouped by type; the graphs of the old list go
 int build_work_t(fd3d_batch* b) {
     std::vector<std::vector<Work>> byt(NTYPES);
     for (const Work& w : b->work) byt[w.tm & 255].push_back(w);
@@ -626,7 +539,6 @@ int build_work_t(fd3d_batch* b) {
     for (cudaGraphExec_t& g : b->gx)
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     BCK(cudaStreamSynchronize(b->st));  // the staging buffer is reused by the next build
-    b->work_t_ok = true;
     return FD3D_OK;
 }
 
@@ -645,7 +557,6 @@ int build_work(fd3d_batch* b) {
     b->work.resize(n);
     size_t at = 0;
     for (int ph = 0; ph < NPHASE; ++ph) {
-        b->pbeg[ph] = (int)at;
         for (const Model& M : b->models)
             if (M.live && !M.items[ph].empty()) {
                 std::memcpy(b->work.data() + at, M.items[ph].data(), M.items[ph].size() * sizeof(Work));
@@ -660,24 +571,9 @@ int build_work(fd3d_batch* b) {
         if (!sp.empty())
             BCK(cudaMemcpyAsync(b->d_stptr, sp.data(), sp.size() * sizeof(int*), cudaMemcpyHostToDevice, b->st));
     }
-    b->work_t_ok = false;
-    b->pbeg[NPHASE] = (int)b->work.size();
-    if (b->work.size() > b->work_cap) {
-        if (b->d_work) cudaFree(b->d_work);
-        b->work_cap = b->work.size() + b->work.size() / 2 + 64;
-        BCK(cudaMalloc(&b->d_work, b->work_cap * sizeof(Work)));
-    }
-    if (!b->work.empty()) {
-        if (stage_items(b, b->work.size())) return FD3D_ERR_CUDA;
-        std::memcpy(b->h_stage, b->work.data(), b->work.size() * sizeof(Work));
-        BCK(cudaMemcpyAsync(b->d_work, b->h_stage, b->work.size() * sizeof(Work), cudaMemcpyHostToDevice, b->st));
-    }
-    BCK(cudaMemcpyAsync(b->d_pbeg, b->pbeg, sizeof(b->pbeg), cudaMemcpyHostToDevice, b->st));
     BCK(cudaStreamSynchronize(b->st));
-    if (b->tun.mode == MODE_GRAPH) {
-        int rc = build_work_t(b);
-        if (rc) return rc;
-    }
+    int rc = build_work_t(b);
+    if (rc) return rc;
     b->dirty = false;
     b->built_kchunk = b->tun.kchunk;
     return FD3D_OK;
@@ -794,10 +690,6 @@ int get_batch_graph(fd3d_batch* b, int g, cudaGraphExec_t* out) {
 }
 
 int launch_graphs(fd3d_batch* b, int nsteps) {
-    if (!b->work_t_ok) {
-        int rc = build_work_t(b);
-        if (rc) return rc;
-    }
     BCK(cudaMemsetAsync(b->d_run_step, 0, sizeof(int), b->st));
     int left = nsteps;
     for (int g = 0; g < fd3d_batch::NGRAPH && left > 0; ++g) {
@@ -811,17 +703,6 @@ int launch_graphs(fd3d_batch* b, int nsteps) {
             left -= n;
         }
     }
-    return FD3D_OK;
-}
-
-int launch_batch(fd3d_batch* b, int nsteps) {
-    if (b->tun.mode == MODE_GRAPH) return launch_graphs(b, nsteps);
-    const int per_sm = b->tun.per_sm > 0 ? std::min(b->tun.per_sm, b->max_active) : b->max_active;
-    const int grid = std::max(1, per_sm * b->nsm);
-    BCK(cudaMemsetAsync(b->d_sync, 0, sizeof(BatchSync), b->st));
-    void* args[] = {&b->d_models, &b->d_maps, &b->d_work, &b->d_pbeg, &b->d_limit, &nsteps, &b->tun.kchunk, &b->d_sync,
-                    &b->d_status};
-    BCK(cudaLaunchCooperativeKernel((void*)k_batch, dim3(grid), dim3(32, 8), args, tma_ring_bytes<float>(), b->st));
     return FD3D_OK;
 }
 
@@ -932,8 +813,7 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
     if (cudaMalloc(&b->d_models, sizeof(ModelDev) * max_models) != cudaSuccess ||
         cudaMalloc(&b->d_maps, sizeof(ModelMaps) * max_models) != cudaSuccess ||
         cudaMalloc(&b->d_limit, sizeof(int) * max_models) != cudaSuccess ||
-        cudaMalloc(&b->d_pbeg, sizeof(int) * (NPHASE + 1)) != cudaSuccess ||
-        cudaMalloc(&b->d_sync, sizeof(BatchSync)) != cudaSuccess || cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess ||
+        cudaMalloc(&b->d_status, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&b->d_run_step, sizeof(int)) != cudaSuccess ||
         cudaMalloc(&b->d_stptr, sizeof(int*) * max_models) != cudaSuccess ||
         cudaMalloc(&b->d_status_or, sizeof(int)) != cudaSuccess) {
@@ -955,8 +835,7 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
     cudaMemset(b->d_status, 0, sizeof(int));
     cudaEventCreate(&b->ev0);
     cudaEventCreate(&b->ev1);
-    if (cudaFuncSetAttribute(k_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_ring_bytes<float>()) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->max_active, k_batch, 256, tma_ring_bytes<float>()) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->max_active, k_bhalf<true>, 256, STR_RING) != cudaSuccess ||
         b->max_active < 1 || !tensor_map_encoder()) {
         cudaGetLastError();
         return fail(FD3D_ERR_CUDA);
@@ -982,10 +861,7 @@ int fd3d_batch_destroy(fd3d_batch* b) {
     cudaFree(b->d_models);
     cudaFree(b->d_maps);
     cudaFree(b->d_limit);
-    cudaFree(b->d_pbeg);
-    cudaFree(b->d_sync);
     cudaFree(b->d_status);
-    cudaFree(b->d_work);
     cudaFree(b->d_work_t);
     if (b->h_stage) cudaFreeHost(b->h_stage);
     cudaFree(b->d_run_step);
@@ -1167,7 +1043,7 @@ int fd3d_batch_run(fd3d_batch* b, int nsteps) {
     BCK(cudaEventRecord(b->ev0, b->st));
     if (smax > 0 && !b->work.empty()) {
         BCK(cudaMemcpyAsync(b->d_limit, limit.data(), limit.size() * sizeof(int), cudaMemcpyHostToDevice, b->st));
-        int rc = launch_batch(b, smax);
+        int rc = launch_graphs(b, smax);
         if (rc) return rc;
     }
     BCK(cudaEventRecord(b->ev1, b->st));
@@ -1358,27 +1234,14 @@ int fd3d_batch_autotune(fd3d_batch* b, int steps, const char* cache_path, const 
             }
         }
     }
-    // candidates: the graph schedule per interior tile depth, the persistent kernel per
-    // tile depth and CTAs per SM
     const int kcs[] = {4, 8, 16, 32};
     std::vector<Tuning> cand;
     for (int kc : kcs) {
         Tuning t;
-        t.mode = MODE_GRAPH;
+        t.mode = b->tun.mode;
         t.kchunk = kc;
         cand.push_back(t);
     }
-    std::vector<int> pss;
-    for (int ps = 1; ps <= b->max_active; ps *= 2) pss.push_back(ps);
-    if (pss.back() != b->max_active) pss.push_back(b->max_active);
-    for (int kc : kcs)
-        for (int ps : pss) {
-            Tuning t;
-            t.mode = MODE_PERSISTENT;
-            t.kchunk = kc;
-            t.per_sm = ps;
-            cand.push_back(t);
-        }
     float best = 1e30f;
     Tuning bt = b->tun;
     for (const Tuning& t : cand) {

@@ -318,16 +318,11 @@ __device__ __forceinline__ bool pml_cell(const PmlDesc& D, int s, long long t, i
 // at a time); all inputs through shared memory by bulk copies of row pieces (a copy is issued
 // by one lane, 30 a tile); u, v, w and the normal and shear stresses in CTAs of their own.
 //
-// Starts the copy of a tile's range of a group (bytes); every thread calls it.  REUSED: sm and
-// bar served an earlier tile of this CTA.
-template <bool REUSED>
+// Starts the copy of a tile's range of a group (bytes); every thread calls it.
 __device__ __forceinline__ void pml_tile_begin(uint32_t sm, const void* src, uint32_t bytes, uint32_t bar) {
-    if (REUSED) {
-        fence_proxy_async_smem();
-        __syncthreads();
-    }
     if (threadIdx.x == 0 && threadIdx.y == 0) {
-        if (!REUSED) { mbar_init(bar, 1); fence_mbar_init(); }
+        mbar_init(bar, 1);
+        fence_mbar_init();
         fence_proxy_async_global();
         mbar_expect_tx(bar, bytes);
         bulk_load(sm, src, bytes, bar);
@@ -335,11 +330,11 @@ __device__ __forceinline__ void pml_tile_begin(uint32_t sm, const void* src, uin
 }
 // Waits (bounded) for the tile's load; false on every thread if any thread gave up
 // (ST_TIMEOUT recorded after one more bounded wait for the copy in flight).
-__device__ __forceinline__ bool pml_tile_wait(uint32_t bar, uint32_t parity, int* status) {
-    const bool ok = mbar_wait(bar, parity);
+__device__ __forceinline__ bool pml_tile_wait(uint32_t bar, int* status) {
+    const bool ok = mbar_wait(bar, 0u);
     if (__syncthreads_or(!ok)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) atomicOr(status, ST_TIMEOUT);
-        mbar_wait(bar, parity);
+        mbar_wait(bar, 0u);
         return false;
     }
     return true;
@@ -455,12 +450,11 @@ __device__ __noinline__ void vel_pml_redo(const Grid* g, const Fields<T>* f, con
 }
 
 // pml_uvw in one tile of strip class C, one cell per thread.  false if the copy timed out.
-template <class T, int C, bool SLAB, bool REUSED>
+template <class T, int C, bool SLAB>
 __device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
-                                               const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar,
-                                               uint32_t parity, int* status) {
+                                               const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar, int* status) {
     constexpr uint32_t BYTES = PML_TILE * AUX_NV * sizeof(T);
-    pml_tile_begin<REUSED>(smem_addr(sm), X.vel + t0 * AUX_NV, BYTES, bar);
+    pml_tile_begin(smem_addr(sm), X.vel + t0 * AUX_NV, BYTES, bar);
     const Strip& S = D.s[s];
     const int l = threadIdx.y * blockDim.x + threadIdx.x;
     int i = 0, j = 0, k = 0;
@@ -468,11 +462,9 @@ __device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f
     const bool act = pml_cell<SLAB>(D, s, t0 + l, i, j, k);
     pml_damped<C>(g, S, act, i, j, wx, wy);
     VelPmlIn<T, C> q;
-    // (the persistent kernel has no registers to hold the inputs across the wait)
-    if (!REUSED && act) q.load(g, f, X, c, S, i, j, k, wx, wy);
-    if (!REUSED) __syncthreads();  // the barrier is initialised
-    if (!pml_tile_wait(bar, parity, status)) return false;
-    if (REUSED && act) q.load(g, f, X, c, S, i, j, k, wx, wy);
+    if (act) q.load(g, f, X, c, S, i, j, k, wx, wy);
+    __syncthreads();  // the barrier is initialised
+    if (!pml_tile_wait(bar, status)) return false;
     if (act) {
         const T* a = sm + aux_at(l, AUX_NV);
         T* ga = X.vel + aux_at(t0 + l, AUX_NV);
@@ -493,16 +485,15 @@ __device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f
 
 // pml_uvw: split-field PML velocity in the strips (fd3d_deriv.f90:1927-2293), one tile of
 // PML_TILE consecutive cells per CTA (a tile lies in one strip).
-template <class T, bool SLAB, bool REUSED>
+template <class T, bool SLAB>
 __device__ __forceinline__ bool vel_pml_tile(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
-                                             const StepConst<T>& c, int tile, T* sm, uint32_t bar, uint32_t parity,
-                                             int* status) {
+                                             const StepConst<T>& c, int tile, T* sm, uint32_t bar, int* status) {
     const long long t0 = (long long)tile * PML_TILE;
     const int s = pml_tile_strip(D, t0);
     switch (pml_class(s)) {
-        case 0: return vel_pml_tile_c<T, 0, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        case 1: return vel_pml_tile_c<T, 1, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        default: return vel_pml_tile_c<T, 2, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        case 0: return vel_pml_tile_c<T, 0, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
+        case 1: return vel_pml_tile_c<T, 1, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
+        default: return vel_pml_tile_c<T, 2, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
     }
 }
 
@@ -755,12 +746,11 @@ __device__ __noinline__ void str_pml_redo(const Grid* g, const Fields<T>* f, con
     str_pml_cell<T, C, DIV_FULL>(*g, *f, *c, *S, free_top, q, a, ga, i, j, k, wx, wy);
 }
 
-template <class T, int C, bool SLAB, bool REUSED>
+template <class T, int C, bool SLAB>
 __device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
-                                               const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar,
-                                               uint32_t parity, int* status) {
+                                               const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar, int* status) {
     constexpr uint32_t BYTES = PML_TILE * AUX_NS * sizeof(T);
-    pml_tile_begin<REUSED>(smem_addr(sm), X.str + t0 * AUX_NS, BYTES, bar);
+    pml_tile_begin(smem_addr(sm), X.str + t0 * AUX_NS, BYTES, bar);
     const Strip& S = D.s[s];
     const bool free_top = C <= 1 && !g.fspace;
     const int l = threadIdx.y * blockDim.x + threadIdx.x;
@@ -769,11 +759,9 @@ __device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f
     const bool act = pml_cell<SLAB>(D, s, t0 + l, i, j, k);
     pml_damped<C>(g, S, act, i, j, wx, wy);
     StrPmlIn<T, C> q;
-    // (the persistent kernel has no registers to hold the inputs across the wait)
-    if (!REUSED && act) q.load(g, f, X, S, i, j, k, wx, wy);
-    if (!REUSED) __syncthreads();  // the barrier is initialised
-    if (!pml_tile_wait(bar, parity, status)) return false;
-    if (REUSED && act) q.load(g, f, X, S, i, j, k, wx, wy);
+    if (act) q.load(g, f, X, S, i, j, k, wx, wy);
+    __syncthreads();  // the barrier is initialised
+    if (!pml_tile_wait(bar, status)) return false;
     if (act) {
         const T* a = sm + aux_at(l, AUX_NS);
         T* ga = X.str + aux_at(t0 + l, AUX_NS);
@@ -793,16 +781,15 @@ __device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f
 }
 
 // pml_xyz in the strips (fd3d_deriv.f90:2304-3143), one tile per CTA as vel_pml_tile
-template <class T, bool SLAB, bool REUSED>
+template <class T, bool SLAB>
 __device__ __forceinline__ bool str_pml_tile(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
-                                             const StepConst<T>& c, int tile, T* sm, uint32_t bar, uint32_t parity,
-                                             int* status) {
+                                             const StepConst<T>& c, int tile, T* sm, uint32_t bar, int* status) {
     const long long t0 = (long long)tile * PML_TILE;
     const int s = pml_tile_strip(D, t0);
     switch (pml_class(s)) {
-        case 0: return str_pml_tile_c<T, 0, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        case 1: return str_pml_tile_c<T, 1, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
-        default: return str_pml_tile_c<T, 2, SLAB, REUSED>(g, f, D, X, c, s, t0, sm, bar, parity, status);
+        case 0: return str_pml_tile_c<T, 0, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
+        case 1: return str_pml_tile_c<T, 1, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
+        default: return str_pml_tile_c<T, 2, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
     }
 }
 
@@ -1477,7 +1464,7 @@ k_vel_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, c
           const __grid_constant__ PmlAux<T> X, const __grid_constant__ StepConst<T> c, int* status, long long tile0) {
     __shared__ __align__(128) T sm[PML_TILE * AUX_NV];
     __shared__ __align__(8) uint64_t bar;
-    vel_pml_tile<T, SLAB, false>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), 0u, status);
+    vel_pml_tile<T, SLAB>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), status);
 }
 
 template <class T>
@@ -1500,7 +1487,7 @@ k_str_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, c
           const __grid_constant__ PmlAux<T> X, const __grid_constant__ StepConst<T> c, int* status, long long tile0) {
     __shared__ __align__(128) T sm[PML_TILE * AUX_NS];
     __shared__ __align__(8) uint64_t bar;
-    str_pml_tile<T, SLAB, false>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), 0u, status);
+    str_pml_tile<T, SLAB>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), status);
 }
 
 // The tiles of strip s that hold cells of planes klo..khi: [t0, t1) (k is the slowest

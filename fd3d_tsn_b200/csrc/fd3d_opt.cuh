@@ -459,12 +459,11 @@ k_vel_small(const __grid_constant__ VelMaps M, const __grid_constant__ Grid g, c
     const int n_int = (int)(ni.x * ni.y * ni.z), n_fault = (int)(nf.x * nf.y * nf.z);
     if (b < n_int) {
         tma_ring_init(bars);
-        unsigned pc = 0;
-        vel_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, b % ni.x, b / ni.x % ni.y, b / (ni.x * ni.y), ring, bars, pc, status);
+        vel_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, b % ni.x, b / ni.x % ni.y, b / (ni.x * ni.y), ring, bars, status);
     } else if ((b -= n_int) < n_fault) {
         vel_fault_body<T>(g, f, q, c, law, s, it_dev, status, b % nf.x, b / nf.x % nf.y, b / (nf.x * nf.y));
     } else {
-        vel_pml_tile<T, false, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), 0u, status);
+        vel_pml_tile<T, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), status);
     }
 }
 
@@ -482,12 +481,11 @@ k_str_small(const __grid_constant__ StrMaps M, const __grid_constant__ Grid g, c
     const int n_int = (int)(ni.x * ni.y * ni.z), n_fault = (int)(nf.x * nf.y * nf.z);
     if (b < n_int) {
         tma_ring_init(bars);
-        unsigned pc = 0;
-        str_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, b % ni.x, b / ni.x % ni.y, b / (ni.x * ni.y), ring, bars, pc, status);
+        str_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, b % ni.x, b / ni.x % ni.y, b / (ni.x * ni.y), ring, bars, status);
     } else if ((b -= n_int) < n_fault) {
         str_fault_body<T>(g, f, q, c, b % nf.x, b / nf.x % nf.y, b / (nf.x * nf.y));
     } else {
-        str_pml_tile<T, false, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), 0u, status);
+        str_pml_tile<T, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), status);
     }
 }
 

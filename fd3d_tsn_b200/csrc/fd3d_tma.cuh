@@ -64,9 +64,7 @@ __device__ __forceinline__ void vel_issue(const VelMaps& M, T* slot, uint32_t ba
     tma_load_3d(smem_addr(slot + VelSlot::W), &M.w, x0, y0, z, bar);
 }
 
-// Ring bookkeeping across the tiles one CTA processes: the n-th plane a CTA ever puts
-// through its ring uses slot n % TMA_NS and mbarrier phase (n / TMA_NS) & 1.  A tile
-// consumes every plane it issued, so `pc` (planes issued so far) is all that carries over.
+// Plane n of a CTA's tile uses slot n % TMA_NS and mbarrier phase (n / TMA_NS) & 1.
 __device__ __forceinline__ int ring_slot(unsigned n) { return (int)(n % TMA_NS); }
 __device__ __forceinline__ uint32_t ring_parity(unsigned n) { return (n / TMA_NS) & 1u; }
 
@@ -78,10 +76,10 @@ __device__ __forceinline__ void tma_ring_init(uint64_t* bars) {
     __syncthreads();
 }
 
-// wait (bounded) for every plane in [k0, ke] of the current tile that was issued, then return
-__device__ __forceinline__ void tma_drain_pc(const uint64_t* bars, unsigned pc, int k0, int ke, int kb) {
+// wait (bounded) for every plane in [k0, ke] of the tile that was issued, then return
+__device__ __forceinline__ void tma_drain(const uint64_t* bars, int k0, int ke, int kb) {
     for (int k = k0; k <= ke && k < k0 + TMA_NS; ++k) {
-        const unsigned n = pc + (unsigned)(k - kb);
+        const unsigned n = (unsigned)(k - kb);
         mbar_wait(smem_addr(&bars[ring_slot(n)]), ring_parity(n));
     }
 }
@@ -91,7 +89,7 @@ __device__ __forceinline__ void tma_drain_pc(const uint64_t* bars, unsigned pc, 
 template <class T, bool LAYERED = false>
 __device__ __forceinline__ bool vel_interior_tma_body(const VelMaps& M, const Grid& g, const Fields<T>& f,
                                                       const StepConst<T>& c, int kchunk, int bx_, int by_, int bz_,
-                                                      T* ring, uint64_t* bars, unsigned& pc, int* status) {
+                                                      T* ring, uint64_t* bars, int* status) {
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int i0 = g.nabc + 1 + bx_ * 32, j0 = g.nabc + 1 + by_ * 8;
     const int i = i0 + tx, j = j0 + ty;
@@ -100,10 +98,9 @@ __device__ __forceinline__ bool vel_interior_tma_body(const VelMaps& M, const Gr
     const int ke = min(kb + kchunk - 1, g.kin_hi());
     const int x0 = g.off + i0 - 1, y0 = j0 - 1;  // tensor coordinates of the tile origin
     const bool leader = (tx == 0 && ty == 0);
-    const unsigned p0 = pc;
     if (leader)
         for (int k = kb; k <= min(ke, kb + TMA_NS - 1); ++k) {
-            const unsigned n = p0 + (unsigned)(k - kb);
+            const unsigned n = (unsigned)(k - kb);
             vel_issue<T, LAYERED>(M, ring + (size_t)ring_slot(n) * VelSlot::ELEMS, smem_addr(&bars[ring_slot(n)]), x0, y0, k - g.kofs);
         }
     // z queues of the own column (plain loads, one plane ahead)
@@ -116,18 +113,17 @@ __device__ __forceinline__ bool vel_interior_tma_body(const VelMaps& M, const Gr
     T yq0, yq1 = yz[pcol - 2 * sz], yq2 = yz[pcol - sz], yq3 = yz[pcol], ny = yz[pcol + sz];
     const T c1 = c.c1, c2 = c.c2, dth = c.dth;
     for (int k = kb; k <= ke; ++k) {
-        const int n = k - kb;
-        const unsigned gn = p0 + (unsigned)n;
-        const int s = ring_slot(gn);
+        const unsigned n = (unsigned)(k - kb);
+        const int s = ring_slot(n);
         const long long pk = pcol + (long long)n * sz;
         zq0 = zq1; zq1 = zq2; zq2 = zq3; zq3 = nz;
         xq0 = xq1; xq1 = xq2; xq2 = xq3; xq3 = nx;
         yq0 = yq1; yq1 = yq2; yq2 = yq3; yq3 = ny;
         if (k < ke) { nz = zz[pk + 3 * sz]; nx = xz[pk + 2 * sz]; ny = yz[pk + 2 * sz]; }
         const T rk = LAYERED ? f.lay[3 * g.nzt + k - 1] : (T)0;  // dth / density of plane k (1-D medium)
-        if (!mbar_wait(smem_addr(&bars[s]), ring_parity(gn))) {
+        if (!mbar_wait(smem_addr(&bars[s]), ring_parity(n))) {
             atomicOr(status, ST_TIMEOUT);
-            tma_drain_pc(bars, p0, k, ke, kb);
+            tma_drain(bars, k, ke, kb);
             return false;
         }
         const T* sl = ring + (size_t)s * VelSlot::ELEMS;
@@ -155,7 +151,6 @@ __device__ __forceinline__ bool vel_interior_tma_body(const VelMaps& M, const Gr
             vel_issue<T, LAYERED>(M, ring + (size_t)s * VelSlot::ELEMS, smem_addr(&bars[s]), x0, y0, k + TMA_NS - g.kofs);
         }
     }
-    pc = p0 + (unsigned)(ke - kb + 1);
     return true;
 }
 
@@ -167,8 +162,7 @@ __global__ void __launch_bounds__(256) k_vel_interior_tma(const __grid_constant_
     T* ring = reinterpret_cast<T*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
     __shared__ __align__(8) uint64_t bars[TMA_NS];
     tma_ring_init(bars);
-    unsigned pc = 0;
-    vel_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, blockIdx.x, blockIdx.y, blockIdx.z, ring, bars, pc, status);
+    vel_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, blockIdx.x, blockIdx.y, blockIdx.z, ring, bars, status);
 }
 
 // Stress slot layout (elements)
@@ -219,7 +213,7 @@ __device__ __forceinline__ void str_issue(const StrMaps& M, T* slot, uint32_t ba
 template <class T, bool LAYERED = false>
 __device__ __forceinline__ bool str_interior_tma_body(const StrMaps& M, const Grid& g, const Fields<T>& f,
                                                       const StepConst<T>& c, int kchunk, int bx_, int by_, int bz_,
-                                                      T* ring, uint64_t* bars, unsigned& pc, int* status) {
+                                                      T* ring, uint64_t* bars, int* status) {
     using StrSlot = typename StrSlotOf<LAYERED>::type;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int i0 = g.nabc + 1 + bx_ * 32, j0 = g.nabc + 1 + by_ * 8;
@@ -229,10 +223,9 @@ __device__ __forceinline__ bool str_interior_tma_body(const StrMaps& M, const Gr
     const int ke = min(kb + kchunk - 1, g.kin_hi());
     const int x0 = g.off + i0 - 1, y0 = j0 - 1;
     const bool leader = (tx == 0 && ty == 0);
-    const unsigned p0 = pc;
     if (leader)
         for (int k = kb; k <= min(ke, kb + TMA_NS - 1); ++k) {
-            const unsigned n = p0 + (unsigned)(k - kb);
+            const unsigned n = (unsigned)(k - kb);
             str_issue<T, LAYERED>(M, ring + (size_t)ring_slot(n) * StrSlot::ELEMS, smem_addr(&bars[ring_slot(n)]), x0, y0, k - g.kofs);
         }
     const int ic = min(i, g.nxt - 1), jc = min(j, g.nyt - 1);  // keeps the (i+1,j+1) tap in range
@@ -246,9 +239,8 @@ __device__ __forceinline__ bool str_interior_tma_body(const StrMaps& M, const Gr
     T mq1 = LAYERED ? (T)0 : mu[pcol + sz], pmd = LAYERED ? (T)0 : mu[pcol + 1 + sy + sz];
     const T c1 = c.c1, c2 = c.c2, dth = c.dth;
     for (int k = kb; k <= ke; ++k) {
-        const int n = k - kb;
-        const unsigned gn = p0 + (unsigned)n;
-        const int s = ring_slot(gn);
+        const unsigned n = (unsigned)(k - kb);
+        const int s = ring_slot(n);
         const long long pk = pcol + (long long)n * sz;
         uq0 = uq1; uq1 = uq2; uq2 = uq3; uq3 = nu;
         vq0 = vq1; vq1 = vq2; vq2 = vq3; vq3 = nv;
@@ -262,9 +254,9 @@ __device__ __forceinline__ bool str_interior_tma_body(const StrMaps& M, const Gr
         // 1-D medium: lam, mu of plane k and mu of plane k+1 (every (i,j) of a plane is equal)
         const T lk = LAYERED ? f.lay[k - 1] : (T)0, mk = LAYERED ? f.lay[g.nzt + k - 1] : (T)0;
         const T mk1 = LAYERED ? f.lay[g.nzt + k] : (T)0;
-        if (!mbar_wait(smem_addr(&bars[s]), ring_parity(gn))) {
+        if (!mbar_wait(smem_addr(&bars[s]), ring_parity(n))) {
             atomicOr(status, ST_TIMEOUT);
-            tma_drain_pc(bars, p0, k, ke, kb);
+            tma_drain(bars, k, ke, kb);
             return false;
         }
         const T* sl = ring + (size_t)s * StrSlot::ELEMS;
@@ -297,7 +289,6 @@ __device__ __forceinline__ bool str_interior_tma_body(const StrMaps& M, const Gr
             str_issue<T, LAYERED>(M, ring + (size_t)s * StrSlot::ELEMS, smem_addr(&bars[s]), x0, y0, k + TMA_NS - g.kofs);
         }
     }
-    pc = p0 + (unsigned)(ke - kb + 1);
     return true;
 }
 
@@ -309,14 +300,7 @@ __global__ void __launch_bounds__(256) k_str_interior_tma(const __grid_constant_
     T* ring = reinterpret_cast<T*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
     __shared__ __align__(8) uint64_t bars[TMA_NS];
     tma_ring_init(bars);
-    unsigned pc = 0;
-    str_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, blockIdx.x, blockIdx.y, blockIdx.z, ring, bars, pc, status);
-}
-
-// dynamic shared memory of a CTA that runs both sweeps through one ring
-template <class T>
-constexpr int tma_ring_bytes() {
-    return TMA_NS * (VelSlot::ELEMS > StrSlot::ELEMS ? VelSlot::ELEMS : StrSlot::ELEMS) * (int)sizeof(T) + TMA_SMEM_PAD;
+    str_interior_tma_body<T, LAYERED>(M, g, f, c, kchunk, blockIdx.x, blockIdx.y, blockIdx.z, ring, bars, status);
 }
 
 }  // namespace fd3d

@@ -254,16 +254,15 @@ int fd3d_ctx_info(fd3d_ctx* ctx, int* interior_variant, int* layered_medium);
  * No counterpart in the reference, which runs one model per process
  * (src/dynamicsolver.f90:66).  Independent forward models of uneven size share one
  * device arena of arena_bytes; fd3d_batch_run advances every live model by up to
- * nsteps steps (each stops at its own ntfd).  Two schedules run the same work items:
- * FD3D_BATCH_PERSISTENT, one cooperative kernel per run whose CTAs walk the items
- * phase by phase between grid barriers, and FD3D_BATCH_GRAPH, CUDA graphs of 32, 16,
- * 8, 4, 2 or 1 steps with one kernel per region and step over all models, in series
- * on one stream (FD3D_BATCH_BRANCHES=1 runs the interior, fault-band and PML sweeps of
- * a half-step as parallel branches instead).
- * fd3d_batch_autotune picks the schedule and its tile shape.  Models use the FP32
+ * nsteps steps (each stops at its own ntfd), by replaying CUDA graphs of 32, 16, 8, 4, 2
+ * or 1 steps with one kernel per region and step over all models, or one per half-step for
+ * a small batch, in series on one stream (FD3D_BATCH_BRANCHES=1 runs the interior, fault-band
+ * and PML sweeps of a half-step as parallel branches instead).  FD3D_BATCH_PERSISTENT is
+ * accepted beside FD3D_BATCH_GRAPH and runs the same launches.
+ * fd3d_batch_autotune picks the tile shape.  Models use the FP32
  * build, a 1-D layered medium (one value per k, as readcrustalmodel builds) and keep
  * the last history_capacity records (default 16) of their history planes.  A model's
- * results are the same bits whether it runs alone or among others, in either schedule. */
+ * results are the same bits whether it runs alone or among others. */
 #define FD3D_BATCH_PERSISTENT 0
 #define FD3D_BATCH_GRAPH 1
 typedef struct fd3d_batch fd3d_batch;
@@ -284,7 +283,7 @@ int fd3d_batch_fetch_plane(fd3d_batch* b, int slot, int plane, double* host);
 int fd3d_batch_fetch_final(fd3d_batch* b, int slot, double* slipX, double* slipZ, double* ruptime,
                            double* rise, double* sliptime);
 int fd3d_batch_fetch_history(fd3d_batch* b, int slot, int field, int rec0, int nrec, double* host);
-/* tile shape: z-planes per interior tile and, for the persistent schedule, CTAs per SM (0 = max) */
+/* tile shape: z-planes per interior tile; ctas_per_sm (0 = max) is kept and reported, no launch depends on it */
 int fd3d_batch_set_tuning(fd3d_batch* b, int kchunk, int ctas_per_sm);
 int fd3d_batch_get_tuning(fd3d_batch* b, int* kchunk, int* ctas_per_sm, int* max_ctas_per_sm);
 /* schedule: FD3D_BATCH_PERSISTENT or FD3D_BATCH_GRAPH (the default) */
