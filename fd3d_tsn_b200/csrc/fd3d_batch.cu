@@ -580,10 +580,10 @@ int build_work(fd3d_batch* b) {
 }
 
 // Whether a half-step of the batch is one launch (k_bhalf), its launches overlapped with the ones
-// before: up to 120 items per SM.  Beyond that the launches' tails no longer count, and the interior
-// tiles run best at the five and six CTAs per SM of their own kernel.  us a step, one launch /
-// separate: 0.7 K items (1 model) 48 / 68, 4 K 140 / 166 (32 planes a tile 146 / 199), 12 K 386 /
-// 400, 16 K 495 / 506; 33 K (32 models) 967 / 946.
+// before: up to 120 items per SM.  Beyond that the launches' tails no longer count, and each region
+// runs at the occupancy of its own kernel.  us a step, one launch / a launch per region, tiles of 8
+// planes: 1 model (0.7 K items or more) 48 / 67, 4 models 148 / 170, 12 models 393 / 400, 16 models 505 /
+// 506, 32 models 967 / 946; tiles of 32 planes: 74 / 103, 140 / 193, 386 / 407, 495 / 519, 957 / 957.
 bool merged_step(const fd3d_batch* b) {
     return !b->branches && b->tbeg[W_VEL_FS] - b->tbeg[W_VEL_INT] <= 120 * b->nsm;
 }

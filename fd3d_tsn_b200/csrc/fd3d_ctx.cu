@@ -964,8 +964,8 @@ static int create_ctx(const fd3d_params* p, int slab_lo, int slab_hi, fd3d_ctx**
     if (const char* e = std::getenv("FD3D_PML_MINB")) {
         int v = 1, s = 0;
         const int n = std::sscanf(e, "%d,%d", &v, &s);
-        c->pml_minb_vel = std::min(6, std::max(1, v));
-        c->pml_minb_str = n == 2 ? std::min(6, std::max(1, s)) : c->pml_minb_vel;
+        c->pml_minb_vel = std::min(5, std::max(1, v));
+        c->pml_minb_str = n == 2 ? std::min(5, std::max(1, s)) : c->pml_minb_vel;
     }
     if (slab && c->icfg.variant != IV_TMA) { delete c; return FD3D_ERR_ARG; }  // z-slabs: the TMA sweeps only
     rc = c->alloc();
