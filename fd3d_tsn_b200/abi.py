@@ -152,6 +152,7 @@ def load_library(path: str | None = None) -> C.CDLL:
         "fd3d_read_deck_ex": (i, [C.c_char_p, i, C.POINTER(Params), C.POINTER(dp), C.POINTER(dp), C.POINTER(dp)]),
         "fd3d_free": (None, [vp]),
         "fd3d_check_division": (i, [fp, i, C.POINTER(C.c_ulonglong), C.POINTER(C.c_uint)]),
+        "fd3d_division_form": (i, [C.c_float, i, C.POINTER(i)]),
         "fd3d_check_waits": (i, [C.POINTER(i), C.POINTER(i)]),
         "fd3d_checkpoint": (i, [vp, C.c_char_p]),
         "fd3d_restore": (i, [C.c_char_p, C.POINTER(vp)]),

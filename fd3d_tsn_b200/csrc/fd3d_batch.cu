@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
         vel_interior_tma_body<float, true>(maps[m].v, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
 }
 
-template <bool STRESS>
+template <bool STRESS, bool ANY>
 __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict__ models,
                                                       const Work* __restrict__ work, int b0,
                                                       const int* __restrict__ limit, const int* run_step, int ofs,
@@ -208,13 +208,13 @@ __global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict
     if (!item_live(it, limit, run_step, ofs, m)) return;
     __shared__ ModelPar M;
     load_par(M, models[m]);
-    if (STRESS) str_pml_tile<float, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
-    else vel_pml_tile<float, false>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
+    if (STRESS) str_pml_tile<float, false, ANY>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
+    else vel_pml_tile<float, false, ANY>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
 }
 
 // A half-step of a small batch in one launch: the interior, fault-band and PML items (contiguous
 // in the list by type), as k_vel_small / k_str_small do for one model.
-template <bool STRESS>
+template <bool STRESS, bool ANY>
 __global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
                                                   const Work* __restrict__ work, int b0, const int* __restrict__ limit,
                                                   const int* run_step, int ofs, int kchunk, int* gstatus) {
@@ -245,8 +245,8 @@ __global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ m
             else vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
             break;
         default:
-            if (STRESS) str_pml_tile<float, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
-            else vel_pml_tile<float, false>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
+            if (STRESS) str_pml_tile<float, false, ANY>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
+            else vel_pml_tile<float, false, ANY>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
     }
 }
 
@@ -437,6 +437,7 @@ struct fd3d_batch {
     // and graphs of 32, 16, 8, 4, 2 and 1 steps captured for the current work list
     std::vector<Work> work_t;
     int tbeg[NTYPES + 1] = {0};
+    int pml_pair = 0;            // the first items of W_VEL_PML (and W_STR_PML): of models with PML_PAIR quotients
     Work* d_work_t = nullptr;
     size_t work_t_cap = 0;
     int* d_run_step = nullptr;
@@ -520,6 +521,11 @@ int stage_items(fd3d_batch* b, size_t n) {
 int build_work_t(fd3d_batch* b) {
     std::vector<std::vector<Work>> byt(NTYPES);
     for (const Work& w : b->work) byt[w.tm & 255].push_back(w);
+    auto pair = [&](const Work& w) { return b->models[w.tm >> 8].dev.c.pml_form == PML_PAIR; };
+    // the items of PML_PAIR models first: a launch of their own where there is one per region (40 models,
+    // one of another form: 1222 us a step, 1231 with one kernel for all of them)
+    for (int t : {W_VEL_PML, W_STR_PML})
+        b->pml_pair = (int)(std::stable_partition(byt[t].begin(), byt[t].end(), pair) - byt[t].begin());
     b->work_t.clear();
     for (int t = 0; t < NTYPES; ++t) {
         b->tbeg[t] = (int)b->work_t.size();
@@ -603,6 +609,7 @@ int enqueue_graph_step(fd3d_batch* b, int ofs) {
     cudaError_t err = cudaSuccess;             // the first failed launch
     auto chk = [&](cudaError_t e) { if (err == cudaSuccess) err = e; };
     auto n_of = [&](int t) { return b->tbeg[t + 1] - b->tbeg[t]; };
+    const bool any = b->pml_pair < n_of(W_VEL_PML);  // models whose PML quotients take another form
     auto plane = [&](cudaStream_t s, int t0, int t1) {  // item types [t0, t1) in one launch
         const int n = b->tbeg[t1] - b->tbeg[t0];
         if (n == 0) return;
@@ -624,7 +631,8 @@ int enqueue_graph_step(fd3d_batch* b, int ofs) {
         const int tp = half ? W_STR_PML : W_VEL_PML, tfs = half ? W_STR_FS : W_VEL_FS;
         const size_t sm = half ? STR_RING : VEL_RING;
         if (small) {
-            chk(launch_kernel(true, half ? k_bhalf<true> : k_bhalf<false>, dim3(b->tbeg[tfs] - b->tbeg[ti]), blk, sm, b->st, b->d_models,
+            auto k = half ? (any ? k_bhalf<true, true> : k_bhalf<true, false>) : (any ? k_bhalf<false, true> : k_bhalf<false, false>);
+            chk(launch_kernel(true, k, dim3(b->tbeg[tfs] - b->tbeg[ti]), blk, sm, b->st, b->d_models,
                               b->d_maps, b->d_work_t, b->tbeg[ti], b->d_limit, b->d_run_step, ofs, kc, b->d_status));
             plane(b->st, tfs, half ? W_FBC + 1 : tfs + 1);
             continue;
@@ -644,10 +652,12 @@ int enqueue_graph_step(fd3d_batch* b, int ofs) {
             else chk(launch_kernel(pdl, k_bint<false>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, ofs, kc, b->d_status));
         }
         plane(s0, tf, tf + 1);
-        if (n_of(tp) > 0) {
-            if (half) chk(launch_kernel(pdl, k_bpml<true>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, ofs, b->d_status));
-            else chk(launch_kernel(pdl, k_bpml<false>, dim3(n_of(tp)), blk, 0, s1, md, wt, b->tbeg[tp], lim, rs, ofs, b->d_status));
-        }
+        auto pml = [&](void (*k)(const ModelDev*, const Work*, int, const int*, const int*, int, int*), int b0, int b1) {
+            if (b1 > b0) chk(launch_kernel(pdl, k, dim3(b1 - b0), blk, 0, s1, md, wt, b0, lim, rs, ofs, b->d_status));
+        };
+        const int p0 = b->tbeg[tp], p1 = p0 + b->pml_pair;
+        pml(half ? k_bpml<true, false> : k_bpml<false, false>, p0, p1);
+        pml(half ? k_bpml<true, true> : k_bpml<false, true>, p1, b->tbeg[tp + 1]);
         if (b->branches) {
             BCK(cudaEventRecord(b->evf[1], b->side[0]));
             BCK(cudaEventRecord(b->evf[2], b->side[1]));
@@ -827,15 +837,15 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
     auto ring_ok = [](auto k, int bytes) {
         return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
     };
-    if (!ring_ok(k_bint<false>, VEL_RING) || !ring_ok(k_bint<true>, STR_RING) || !ring_ok(k_bhalf<false>, VEL_RING) ||
-        !ring_ok(k_bhalf<true>, STR_RING)) {
+    if (!ring_ok(k_bint<false>, VEL_RING) || !ring_ok(k_bint<true>, STR_RING) || !ring_ok(k_bhalf<false, false>, VEL_RING) ||
+        !ring_ok(k_bhalf<true, false>, STR_RING) || !ring_ok(k_bhalf<false, true>, VEL_RING) || !ring_ok(k_bhalf<true, true>, STR_RING)) {
         cudaGetLastError();
         return fail(FD3D_ERR_CUDA);
     }
     cudaMemset(b->d_status, 0, sizeof(int));
     cudaEventCreate(&b->ev0);
     cudaEventCreate(&b->ev1);
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->max_active, k_bhalf<true>, 256, STR_RING) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b->max_active, k_bhalf<true, false>, 256, STR_RING) != cudaSuccess ||
         b->max_active < 1 || !tensor_map_encoder()) {
         cudaGetLastError();
         return fail(FD3D_ERR_CUDA);

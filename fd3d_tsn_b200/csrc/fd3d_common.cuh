@@ -118,8 +118,9 @@ template <class T>
 struct StepConst {
     T dt, dh, dth, dth2, dht, damp_s, c1, c2;
     T rdh, rdl;              // the pair of dh for div_by
+    T ydh;                   // RN(1/dh) for div_steps
     T ds, dsi;               // the scale S of the dividends and 1/S (div_scale)
-    int pml_exact;           // 1: some divisor of the PML sweeps has no such pair, every cell uses div_exact
+    int pml_form;            // how the PML sweeps form their quotients (PmlForm)
     double dtA, dhA, dthA;   // FP64 copies for the FP64 parts
 };
 
@@ -149,6 +150,19 @@ struct StepConst {
 // result that is not finite (x*l and x*h can cancel to NaN where x/b is infinite) with
 // div_exact.  An exhaustive GPU test over all 2^32 dividends (fd3d_check_division) holds all
 // three to the IEEE quotient.
+//
+// Not every divisor has a pair.  Of 20000 random significands 1218 have none with l >= 0 (nor have
+// 11.3, 45.2 or 40000/650) and 38 have none at all (56.3, 112.6, 225.2).  PmlForm is what a model's
+// sweeps do about it, one form for the whole model:
+//   PML_PAIR    dh has a pair with l >= 0, every 1 + omega a pair: div_by and div_by_signed
+//   PML_SIGNED  the pair of dh has l < 0: div_by_signed for both, one operation more a quotient
+//   PML_STEPS   some divisor has no pair: div_steps for both
+//   PML_EXACT   some divisor is outside [2^-20, 2^20]: div_exact for both
+// The last three are kernels of their own (ANY), so that the first keeps its registers.  us a step at
+// spacings of the four forms (45.0, 45.2, 56.3, 1.5e6 m): 1.6 M cells 65.3, 66.3, 67.1, 74.0, 68 M cells
+// 1547, 1546, 1550, 1853.  (With div_exact for all but the first, formed after div_by's result was
+// thrown away: 65.3, 92.6, 92.6, 92.6 and 1547, 2006, 2006, 2006.)
+enum PmlForm { PML_PAIR = 0, PML_SIGNED = 1, PML_STEPS = 2, PML_EXACT = 3 };
 constexpr unsigned DIV_KEY = 2u * 0x1c800000u - 1u;  // the key of 2^-70
 __device__ __forceinline__ float div_by(float x, float h, float l, unsigned& key) {
     key = min(key, 2u * __float_as_uint(x) - 1u);
@@ -157,14 +171,29 @@ __device__ __forceinline__ float div_by(float x, float h, float l, unsigned& key
 __device__ __forceinline__ float div_by_signed(float x, float h, float l, unsigned& key) {
     return __uint_as_float(__float_as_uint(div_by(x, h, l, key)) | (__float_as_uint(x) & 0x80000000u));
 }
-// x / b for every finite x: scaled by 2^80 the quotient is div_by's.  Scaling it back rounds a
+// The same in five operations from y = RN(1/b) alone, for a divisor without a pair.  Markstein's
+// theorem (P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", IBM J. Res. Dev. 34(1), 1990): if y is within half an ulp of 1/b and q within one
+// ulp of x/b, the remainder r = x - b*q is exact and RN(q + r*y) = RN(x/b).  RN(x*y) can be 1.5
+// ulp off, so one correction brings it within one first; the second is the theorem's.  The remainder
+// is exact while it does not underflow, and |x| >= 2^-70 leaves it 2^-117 or more.
+__device__ __forceinline__ float div_steps(float x, float b, float y, unsigned& key) {
+    key = min(key, 2u * __float_as_uint(x) - 1u);
+    float q = __fmul_rn(x, y);
+    q = __fmaf_rn(__fmaf_rn(-q, b, x), y, q);
+    q = __fmaf_rn(__fmaf_rn(-q, b, x), y, q);
+    return __uint_as_float(__float_as_uint(q) | (__float_as_uint(x) & 0x80000000u));
+}
+// x / b for every finite x: scaled by 2^80 the quotient is div_by's (STEPS: div_steps's, from y = h;
+// right for every divisor in range where x / b is finite).  Scaling it back rounds a
 // second time if the result is subnormal; where that went to the wrong side of a tie, the
 // residual x - q*b (exact here: q is a multiple of 2^-149, and less than a unit off) is more
 // than half a unit times b.
+template <bool STEPS>
 __device__ __forceinline__ float div_small(float x, float b, float h, float l) {
     unsigned key = 0;
     const bool small = fabsf(x) < 0x1p-10f;
-    const float xs = x * (small ? 0x1p80f : 1.0f), qs = div_by_signed(xs, h, l, key);
+    const float xs = x * (small ? 0x1p80f : 1.0f), qs = STEPS ? div_steps(xs, b, h, key) : div_by_signed(xs, h, l, key);
     float q = qs * (small ? 0x1p-80f : 1.0f);
     if (small && fabsf(qs) < 0x1p-46f) {
         const float rest = __fmaf_rn(-(q * 0x1p80f), b, xs), half = b * 0x1p-70f;

@@ -179,7 +179,7 @@ struct PmlDesc {
     int ns;                       // strips present: 4, or 5 under FSPACE
     int klo, khi;                 // planes updated (Grid::klo, khi)
     int tile0[PML_MAXS + 1];      // cum in tiles
-    int exact;                    // a divisor 1 + omega has no pair for div_by (StepConst::pml_exact)
+    int form;                     // the PmlForm that the divisors 1 + omega ask for
     double bmax;                  // the largest of them
 };
 
@@ -199,7 +199,8 @@ inline size_t pml_aux_elems(const PmlDesc& D) { return (size_t)pml_aux_cells(D) 
 
 // One entry of a damping profile (init_pml's omega at one index): the factors
 // 1 - omega and 1 + omega of the split-field update, formed on the host with the same IEEE
-// operations the reference performs, and the pair of 1 + omega for div_by_signed.
+// operations the reference performs, and the pair of 1 + omega for div_by_signed (h = RN(1/(1 +
+// omega)) always, for div_steps).
 template <class T>
 struct alignas(4 * sizeof(T)) Damp {
     T m, p, h, l;  // 1 - omega, 1 + omega, pair
@@ -227,8 +228,9 @@ __host__ __device__ constexpr int split_mode(int C, int DIR) {
 //             all of them are right.  The quotient by dh stays scaled: its only use is an
 //             addition, where a multiply-add takes the factor out without a rounding.
 //   DIV_TINY: right for finite operands of any size, DIV_FULL: for all
+// FORM (PML_PAIR, PML_SIGNED, PML_STEPS): the quotients of the first two.
 enum { DIV_FAST = 0, DIV_TINY = 1, DIV_FULL = 2 };
-template <class T, int HOW>
+template <class T, int HOW, int FORM>
 struct PmlDiv {
     const StepConst<T>& c;
     unsigned key = 0xffffffffu;
@@ -238,8 +240,11 @@ struct PmlDiv {
     }
     // x / dh (of a scaled x: scaled)
     __device__ __forceinline__ T by_dh(T x) {
-        if constexpr (HOW == DIV_FAST) return div_by(x, c.rdh, c.rdl, key);
-        else if constexpr (HOW == DIV_TINY) return div_small(x, c.dh, c.rdh, c.rdl);
+        if constexpr (HOW == DIV_FAST && FORM == PML_STEPS) return div_steps(x, c.dh, c.ydh, key);
+        else if constexpr (HOW == DIV_FAST && FORM == PML_SIGNED) return div_by_signed(x, c.rdh, c.rdl, key);
+        else if constexpr (HOW == DIV_FAST) return div_by(x, c.rdh, c.rdl, key);
+        else if constexpr (HOW == DIV_TINY && FORM == PML_STEPS) return div_small<true>(x, c.dh, c.ydh, (T)0);
+        else if constexpr (HOW == DIV_TINY) return div_small<false>(x, c.dh, c.rdh, c.rdl);
         else return div_exact(x, c.dh);
     }
     __device__ __forceinline__ T plus(T a, T q) const {  // a + x / dh
@@ -251,8 +256,9 @@ struct PmlDiv {
     __device__ __forceinline__ T split(T p, T q, const Damp<T>& o, bool warp_damped) {
         if (MODE == SPLIT_NEVER || (MODE == SPLIT_MAYBE && !warp_damped)) return plus(p, q);
         const T x = plus(p * o.m, q);
-        if constexpr (HOW == DIV_FAST) return div_by_signed(x * c.ds, o.h, o.l, key) * c.dsi;
-        else if constexpr (HOW == DIV_TINY) return div_small(x, o.p, o.h, o.l);
+        if constexpr (HOW == DIV_FAST && FORM == PML_STEPS) return div_steps(x * c.ds, o.p, o.h, key) * c.dsi;
+        else if constexpr (HOW == DIV_FAST) return div_by_signed(x * c.ds, o.h, o.l, key) * c.dsi;
+        else if constexpr (HOW == DIV_TINY) return div_small<FORM == PML_STEPS>(x, o.p, o.h, o.l);
         else return div_exact(x, o.p);
     }
 };
@@ -392,14 +398,14 @@ struct VelPmlIn {
 
 // pml_uvw at one cell of strip S (fd3d_deriv.f90:1927-2293); a: its first split component in
 // shared memory.  Returns HOW, or the form that the cell needs, with nothing stored.
-template <class T, int C, int HOW>
+template <class T, int C, int HOW, int FORM>
 __device__ __forceinline__ int vel_pml_cell(const Grid& g, const Fields<T>& f, const StepConst<T>& c, const Strip& S,
                                             const VelPmlIn<T, C>& q, const T* a, T* ga, int i, int j,
                                             int k, bool wx, bool wy) {
     constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
     const bool dov = j <= S.nye;
     // p = (p*(1 - omega) + (dt/d)*diff/dh) / (1 + omega), every division rounded as IEEE
-    PmlDiv<T, HOW> dv{c};
+    PmlDiv<T, HOW, FORM> dv{c};
     const T r = dv.scaled(q.r);
     auto inc = [&](T diff) { return dv.by_dh(r * diff); };
     auto at = [&](int n) { return a[32 * n]; };
@@ -416,7 +422,7 @@ __device__ __forceinline__ int vel_pml_cell(const Grid& g, const Fields<T>& f, c
     const T v2 = dv.template split<MZ>(at(AX_V2), inc((dov ? q.yz0 : (T)0) - q.yz2), q.oz, true);
     const T u = u0 + u1 + u2, w = w0 + w1 + w2, v = v0 + v1 + v2;
     if constexpr (HOW == DIV_FAST) {
-        if (c.pml_exact || !pml_finite(fabsf(u) + fabsf(v) + fabsf(w))) return DIV_FULL;
+        if (!pml_finite(fabsf(u) + fabsf(v) + fabsf(w))) return DIV_FULL;
         if (dv.key < DIV_KEY) return DIV_TINY;
     }
     put(AX_U0) = u0; put(AX_U1) = u1; put(AX_U2) = u2; put(AX_W0) = w0; put(AX_W1) = w1; put(AX_W2) = w2;
@@ -440,17 +446,18 @@ __device__ __forceinline__ int vel_pml_cell(const Grid& g, const Fields<T>& f, c
     return HOW;
 }
 
-// The cells that need the full form, out of line.
-template <class T, int C>
+// The cells that need another form than DIV_FAST, out of line.
+template <class T, int C, int HOW>
 __device__ __noinline__ void vel_pml_redo(const Grid* g, const Fields<T>* f, const PmlAux<T>* X, const StepConst<T>* c,
                                           const Strip* S, const T* a, T* ga, int i, int j, int k, bool wx, bool wy) {
     VelPmlIn<T, C> q;
     q.load(*g, *f, *X, *c, *S, i, j, k, wx, wy);
-    vel_pml_cell<T, C, DIV_FULL>(*g, *f, *c, *S, q, a, ga, i, j, k, wx, wy);
+    vel_pml_cell<T, C, HOW, PML_STEPS>(*g, *f, *c, *S, q, a, ga, i, j, k, wx, wy);
 }
 
-// pml_uvw in one tile of strip class C, one cell per thread.  false if the copy timed out.
-template <class T, int C, bool SLAB>
+// pml_uvw in one tile of strip class C, one cell per thread.  false if the copy timed out.  ANY: the
+// model's quotients may take any form (PmlForm; those of a pair with l >= 0 are also div_by_signed's).
+template <class T, int C, bool SLAB, bool ANY>
 __device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
                                                const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar, int* status) {
     constexpr uint32_t BYTES = PML_TILE * AUX_NV * sizeof(T);
@@ -468,15 +475,24 @@ __device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f
     if (act) {
         const T* a = sm + aux_at(l, AUX_NV);
         T* ga = X.vel + aux_at(t0 + l, AUX_NV);
-        constexpr int HOW = sizeof(T) == 8 ? DIV_FULL : DIV_FAST;
-        const int how = vel_pml_cell<T, C, HOW>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
-        if constexpr (HOW == DIV_FAST) {
+        if constexpr (sizeof(T) == 8) {
+            vel_pml_cell<T, C, DIV_FULL, PML_PAIR>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+        } else {
+            int how = DIV_FAST;
+            if (!ANY) how = vel_pml_cell<T, C, DIV_FAST, PML_PAIR>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+            else if (c.pml_form <= PML_SIGNED) how = vel_pml_cell<T, C, DIV_FAST, PML_SIGNED>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+            else if (c.pml_form == PML_STEPS) how = vel_pml_cell<T, C, DIV_FAST, PML_STEPS>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+            else vel_pml_cell<T, C, DIV_FULL, PML_EXACT>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
             if (how == DIV_TINY) {  // the same again: nothing is stored yet
-                asm volatile("" ::: "memory");  // (the inputs are loaded anew, not kept in registers)
-                q.load(g, f, X, c, S, i, j, k, wx, wy);
-                vel_pml_cell<T, C, DIV_TINY>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+                if (ANY) {
+                    vel_pml_redo<T, C, DIV_TINY>(&g, &f, &X, &c, &S, a, ga, i, j, k, wx, wy);
+                } else {
+                    asm volatile("" ::: "memory");  // (the inputs are loaded anew, not kept in registers)
+                    q.load(g, f, X, c, S, i, j, k, wx, wy);
+                    vel_pml_cell<T, C, DIV_TINY, PML_PAIR>(g, f, c, S, q, a, ga, i, j, k, wx, wy);
+                }
             } else if (how == DIV_FULL) {
-                vel_pml_redo<T, C>(&g, &f, &X, &c, &S, a, ga, i, j, k, wx, wy);
+                vel_pml_redo<T, C, DIV_FULL>(&g, &f, &X, &c, &S, a, ga, i, j, k, wx, wy);
             }
         }
     }
@@ -485,15 +501,15 @@ __device__ __forceinline__ bool vel_pml_tile_c(const Grid& g, const Fields<T>& f
 
 // pml_uvw: split-field PML velocity in the strips (fd3d_deriv.f90:1927-2293), one tile of
 // PML_TILE consecutive cells per CTA (a tile lies in one strip).
-template <class T, bool SLAB>
+template <class T, bool SLAB, bool ANY>
 __device__ __forceinline__ bool vel_pml_tile(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
                                              const StepConst<T>& c, int tile, T* sm, uint32_t bar, int* status) {
     const long long t0 = (long long)tile * PML_TILE;
     const int s = pml_tile_strip(D, t0);
     switch (pml_class(s)) {
-        case 0: return vel_pml_tile_c<T, 0, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
-        case 1: return vel_pml_tile_c<T, 1, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
-        default: return vel_pml_tile_c<T, 2, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
+        case 0: return vel_pml_tile_c<T, 0, SLAB, ANY>(g, f, D, X, c, s, t0, sm, bar, status);
+        case 1: return vel_pml_tile_c<T, 1, SLAB, ANY>(g, f, D, X, c, s, t0, sm, bar, status);
+        default: return vel_pml_tile_c<T, 2, SLAB, ANY>(g, f, D, X, c, s, t0, sm, bar, status);
     }
 }
 
@@ -658,14 +674,14 @@ struct StrPmlIn {
 
 // pml_xyz at one cell of a strip (fd3d_deriv.f90:2304-3143), as vel_pml_cell; free_top: the
 // strip's xz and yz components are zeroed at its top row (strips 1-3, not FSPACE)
-template <class T, int C, int HOW>
+template <class T, int C, int HOW, int FORM>
 __device__ __forceinline__ int str_pml_cell(const Grid& g, const Fields<T>& f, const StepConst<T>& c, const Strip& S,
                                             bool free_top, const StrPmlIn<T, C>& q, const T* a, T* ga, int i, int j,
                                             int k, bool wx, bool wy) {
     constexpr int MX = split_mode(C, 0), MY = split_mode(C, 1), MZ = split_mode(C, 2);
     const bool dxy = j <= S.nye;
     // p = (p*(1 - omega) + dt*modulus*diff/dh) / (1 + omega), every division rounded as IEEE
-    PmlDiv<T, HOW> dv{c};
+    PmlDiv<T, HOW, FORM> dv{c};
     auto at = [&](int comp) { return a[32 * (comp - AUX_NV)]; };
     auto put = [&](int comp) -> T& { return ga[32 * (comp - AUX_NV)]; };
     const T dt = c.dt;
@@ -699,8 +715,7 @@ __device__ __forceinline__ int str_pml_cell(const Grid& g, const Fields<T>& f, c
     }
     const T xy = e0 + e1, yz = h0 + h1;
     if constexpr (HOW == DIV_FAST) {
-        if (c.pml_exact || !pml_finite(fabsf(xx) + fabsf(yy) + fabsf(zz) + fabsf(xy) + fabsf(xz) + fabsf(yz)))
-            return DIV_FULL;
+        if (!pml_finite(fabsf(xx) + fabsf(yy) + fabsf(zz) + fabsf(xy) + fabsf(xz) + fabsf(yz))) return DIV_FULL;
         if (dv.key < DIV_KEY) return DIV_TINY;
     }
     if (free_top && k == S.nze) q0 = q1 = h0 = h1 = (T)0;
@@ -737,16 +752,16 @@ __device__ __forceinline__ int str_pml_cell(const Grid& g, const Fields<T>& f, c
     return HOW;
 }
 
-template <class T, int C>
+template <class T, int C, int HOW>
 __device__ __noinline__ void str_pml_redo(const Grid* g, const Fields<T>* f, const PmlAux<T>* X, const StepConst<T>* c,
                                           const Strip* S, bool free_top, const T* a, T* ga, int i, int j, int k,
                                           bool wx, bool wy) {
     StrPmlIn<T, C> q;
     q.load(*g, *f, *X, *S, i, j, k, wx, wy);
-    str_pml_cell<T, C, DIV_FULL>(*g, *f, *c, *S, free_top, q, a, ga, i, j, k, wx, wy);
+    str_pml_cell<T, C, HOW, PML_STEPS>(*g, *f, *c, *S, free_top, q, a, ga, i, j, k, wx, wy);
 }
 
-template <class T, int C, bool SLAB>
+template <class T, int C, bool SLAB, bool ANY>
 __device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
                                                const StepConst<T>& c, int s, long long t0, T* sm, uint32_t bar, int* status) {
     constexpr uint32_t BYTES = PML_TILE * AUX_NS * sizeof(T);
@@ -765,15 +780,24 @@ __device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f
     if (act) {
         const T* a = sm + aux_at(l, AUX_NS);
         T* ga = X.str + aux_at(t0 + l, AUX_NS);
-        constexpr int HOW = sizeof(T) == 8 ? DIV_FULL : DIV_FAST;
-        const int how = str_pml_cell<T, C, HOW>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
-        if constexpr (HOW == DIV_FAST) {
+        if constexpr (sizeof(T) == 8) {
+            str_pml_cell<T, C, DIV_FULL, PML_PAIR>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+        } else {
+            int how = DIV_FAST;
+            if (!ANY) how = str_pml_cell<T, C, DIV_FAST, PML_PAIR>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+            else if (c.pml_form <= PML_SIGNED) how = str_pml_cell<T, C, DIV_FAST, PML_SIGNED>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+            else if (c.pml_form == PML_STEPS) how = str_pml_cell<T, C, DIV_FAST, PML_STEPS>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+            else str_pml_cell<T, C, DIV_FULL, PML_EXACT>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
             if (how == DIV_TINY) {  // the same again: nothing is stored yet
-                asm volatile("" ::: "memory");  // (the inputs are loaded anew, not kept in registers)
-                q.load(g, f, X, S, i, j, k, wx, wy);
-                str_pml_cell<T, C, DIV_TINY>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+                if (ANY) {
+                    str_pml_redo<T, C, DIV_TINY>(&g, &f, &X, &c, &S, free_top, a, ga, i, j, k, wx, wy);
+                } else {
+                    asm volatile("" ::: "memory");  // (the inputs are loaded anew, not kept in registers)
+                    q.load(g, f, X, S, i, j, k, wx, wy);
+                    str_pml_cell<T, C, DIV_TINY, PML_PAIR>(g, f, c, S, free_top, q, a, ga, i, j, k, wx, wy);
+                }
             } else if (how == DIV_FULL) {
-                str_pml_redo<T, C>(&g, &f, &X, &c, &S, free_top, a, ga, i, j, k, wx, wy);
+                str_pml_redo<T, C, DIV_FULL>(&g, &f, &X, &c, &S, free_top, a, ga, i, j, k, wx, wy);
             }
         }
     }
@@ -781,15 +805,15 @@ __device__ __forceinline__ bool str_pml_tile_c(const Grid& g, const Fields<T>& f
 }
 
 // pml_xyz in the strips (fd3d_deriv.f90:2304-3143), one tile per CTA as vel_pml_tile
-template <class T, bool SLAB>
+template <class T, bool SLAB, bool ANY>
 __device__ __forceinline__ bool str_pml_tile(const Grid& g, const Fields<T>& f, const PmlDesc& D, const PmlAux<T>& X,
                                              const StepConst<T>& c, int tile, T* sm, uint32_t bar, int* status) {
     const long long t0 = (long long)tile * PML_TILE;
     const int s = pml_tile_strip(D, t0);
     switch (pml_class(s)) {
-        case 0: return str_pml_tile_c<T, 0, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
-        case 1: return str_pml_tile_c<T, 1, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
-        default: return str_pml_tile_c<T, 2, SLAB>(g, f, D, X, c, s, t0, sm, bar, status);
+        case 0: return str_pml_tile_c<T, 0, SLAB, ANY>(g, f, D, X, c, s, t0, sm, bar, status);
+        case 1: return str_pml_tile_c<T, 1, SLAB, ANY>(g, f, D, X, c, s, t0, sm, bar, status);
+        default: return str_pml_tile_c<T, 2, SLAB, ANY>(g, f, D, X, c, s, t0, sm, bar, status);
     }
 }
 
@@ -1458,13 +1482,13 @@ k_vel_fault(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f,
 
 // One PML tile per CTA of PML_TILE threads.  MINB: CTAs that must fit one SM
 // (register cap); 1 leaves it free.
-template <class T, int MINB = 1, bool SLAB = false>
+template <class T, int MINB, bool SLAB, bool ANY>
 __global__ void __launch_bounds__(PML_TILE, MINB)
 k_vel_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ PmlDesc D,
           const __grid_constant__ PmlAux<T> X, const __grid_constant__ StepConst<T> c, int* status, long long tile0) {
     __shared__ __align__(128) T sm[PML_TILE * AUX_NV];
     __shared__ __align__(8) uint64_t bar;
-    vel_pml_tile<T, SLAB>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), status);
+    vel_pml_tile<T, SLAB, ANY>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), status);
 }
 
 template <class T>
@@ -1481,13 +1505,13 @@ k_str_fault(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f,
     str_fault_body<T>(g, f, q, c, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-template <class T, int MINB = 1, bool SLAB = false>
+template <class T, int MINB, bool SLAB, bool ANY>
 __global__ void __launch_bounds__(PML_TILE, MINB)
 k_str_pml(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ PmlDesc D,
           const __grid_constant__ PmlAux<T> X, const __grid_constant__ StepConst<T> c, int* status, long long tile0) {
     __shared__ __align__(128) T sm[PML_TILE * AUX_NS];
     __shared__ __align__(8) uint64_t bar;
-    str_pml_tile<T, SLAB>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), status);
+    str_pml_tile<T, SLAB, ANY>(g, f, D, X, c, tile0 + blockIdx.x, sm, smem_addr(&bar), status);
 }
 
 // The tiles of strip s that hold cells of planes klo..khi: [t0, t1) (k is the slowest
@@ -1502,38 +1526,43 @@ inline void pml_strip_tiles(const PmlDesc& D, int s, long long& t0, long long& t
     t1 = (D.cum[s] + (long long)(ke - S.nzb + 1) * per_k + PML_TILE - 1) / PML_TILE;
 }
 
+template <class T, int MINB, bool SLAB, bool ANY>
+inline void launch_pml_n(bool stress, cudaStream_t st, const Grid& g, const Fields<T>& f, const PmlDesc& D,
+                         const PmlAux<T>& X, const StepConst<T>& c, int* status, long long t0, long long t1) {
+    if (t1 <= t0) return;
+    const unsigned n = (unsigned)(t1 - t0);
+    if (stress) k_str_pml<T, MINB, SLAB, ANY><<<n, PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
+    else k_vel_pml<T, MINB, SLAB, ANY><<<n, PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
+}
 // launch of a PML sweep: one launch over every tile for a whole model (with a register
-// cap picked at run time), one per strip over the tiles of its planes for a z-slab
+// cap picked at run time; four CTAs per SM where the quotients take a form of their own), one
+// per strip over the tiles of its planes for a z-slab
 template <class T>
 inline void launch_pml(bool stress, int minb, cudaStream_t st, const Grid& g, const Fields<T>& f, const PmlDesc& D,
                        const PmlAux<T>& X, const StepConst<T>& c, int* status) {
+    constexpr bool F32 = sizeof(T) == 4;  // (FP64 divides directly: one form)
+    const bool any = F32 && c.pml_form != PML_PAIR;
     if (D.klo > 1 || D.khi < g.nzt) {  // a z-slab: the tiles of its planes, strip by strip
         for (int s = 0; s < D.ns; ++s) {
             long long t0, t1;
             pml_strip_tiles(D, s, t0, t1);
-            if (t1 <= t0) continue;
-            if (stress) k_str_pml<T, 1, true><<<(unsigned)(t1 - t0), PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
-            else k_vel_pml<T, 1, true><<<(unsigned)(t1 - t0), PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
+            if (any) launch_pml_n<T, 1, true, F32>(stress, st, g, f, D, X, c, status, t0, t1);
+            else launch_pml_n<T, 1, true, false>(stress, st, g, f, D, X, c, status, t0, t1);
         }
         return;
     }
-    const unsigned nblk = (unsigned)((D.cum[PML_MAXS] + PML_TILE - 1) / PML_TILE);
-    if (nblk == 0) return;
-#define FD3D_PML_CASE(MB)                                                                  \
-    case MB:                                                                               \
-        if (stress) k_str_pml<T, MB><<<nblk, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);  \
-        else k_vel_pml<T, MB><<<nblk, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);         \
-        break;
-    switch (minb) {
-        FD3D_PML_CASE(2)
-        FD3D_PML_CASE(3)
-        FD3D_PML_CASE(4)
-        FD3D_PML_CASE(5)
-        default:
-            if (stress) k_str_pml<T, 1><<<nblk, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);
-            else k_vel_pml<T, 1><<<nblk, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);
+    const long long n = D.cum[PML_MAXS] / PML_TILE;
+    if (any) {
+        launch_pml_n<T, 4, false, F32>(stress, st, g, f, D, X, c, status, 0, n);
+        return;
     }
-#undef FD3D_PML_CASE
+    switch (minb) {
+        case 2: launch_pml_n<T, 2, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
+        case 3: launch_pml_n<T, 3, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
+        case 4: launch_pml_n<T, 4, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
+        case 5: launch_pml_n<T, 5, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
+        default: launch_pml_n<T, 1, false, false>(stress, st, g, f, D, X, c, status, 0, n);
+    }
 }
 
 template <class T>

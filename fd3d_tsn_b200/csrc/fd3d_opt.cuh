@@ -444,7 +444,7 @@ bool make_interior_maps(const Grid& g, const Fields<T>& f, VelMaps& V, StrMaps& 
 // disjoint cells), in that order, the longest-running CTAs first.  A step is then four launches
 // one after the other, each started while the one before drains, instead of eight over two
 // streams with two forks and joins: see small_step for where that is faster.
-template <class T, bool LAYERED>
+template <class T, bool LAYERED, bool ANY>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 k_vel_small(const __grid_constant__ VelMaps M, const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f,
             const __grid_constant__ Fault<T> q, const __grid_constant__ PmlDesc D, const __grid_constant__ PmlAux<T> X,
@@ -463,11 +463,11 @@ k_vel_small(const __grid_constant__ VelMaps M, const __grid_constant__ Grid g, c
     } else if ((b -= n_int) < n_fault) {
         vel_fault_body<T>(g, f, q, c, law, s, it_dev, status, b % nf.x, b / nf.x % nf.y, b / (nf.x * nf.y));
     } else {
-        vel_pml_tile<T, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), status);
+        vel_pml_tile<T, false, ANY>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), status);
     }
 }
 
-template <class T, bool LAYERED>
+template <class T, bool LAYERED, bool ANY>
 __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2)
 k_str_small(const __grid_constant__ StrMaps M, const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f,
             const __grid_constant__ Fault<T> q, const __grid_constant__ PmlDesc D, const __grid_constant__ PmlAux<T> X,
@@ -485,7 +485,7 @@ k_str_small(const __grid_constant__ StrMaps M, const __grid_constant__ Grid g, c
     } else if ((b -= n_int) < n_fault) {
         str_fault_body<T>(g, f, q, c, b % nf.x, b / nf.x % nf.y, b / (nf.x * nf.y));
     } else {
-        str_pml_tile<T, false>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), status);
+        str_pml_tile<T, false, ANY>(g, f, D, X, c, b - n_fault, ring, smem_addr(bars), status);
     }
 }
 
@@ -497,10 +497,12 @@ bool prepare_tma_kernels() {
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_vel_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssl) == cudaSuccess;
-    ok &= cudaFuncSetAttribute(k_vel_small<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
-    ok &= cudaFuncSetAttribute(k_vel_small<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
-    ok &= cudaFuncSetAttribute(k_str_small<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) == cudaSuccess;
-    ok &= cudaFuncSetAttribute(k_str_small<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssl) == cudaSuccess;
+    constexpr bool F32 = sizeof(T) == 4;
+    auto ring = [&](auto k, int bytes) { ok &= cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; };
+    ring(k_vel_small<T, false, false>, vs); ring(k_vel_small<T, false, F32>, vs);
+    ring(k_vel_small<T, true, false>, vs); ring(k_vel_small<T, true, F32>, vs);
+    ring(k_str_small<T, false, false>, ss); ring(k_str_small<T, false, F32>, ss);
+    ring(k_str_small<T, true, false>, ssl); ring(k_str_small<T, true, F32>, ssl);
     if (!ok) cudaGetLastError();
     return ok;
 }
@@ -533,14 +535,18 @@ void launch_half_small(bool stress, const VelMaps& V, const StrMaps& S, const In
     int kch;
     dim3 ni, nf;
     const dim3 grid(half_small_grid(stress, cfg, g, D, kch, ni, nf)), blk(32, 8);
+    constexpr bool F32 = sizeof(T) == 4;
+    const bool any = F32 && c.pml_form != PML_PAIR;
     if (!stress) {
         const size_t sm = TMA_NS * VelSlot::ELEMS * sizeof(T) + TMA_SMEM_PAD;
-        if (f.lay) launch_kernel(true, k_vel_small<T, true>, grid, blk, sm, st, V, g, f, q, D, X, c, law, s, it_dev, status, kch, ni, nf);
-        else launch_kernel(true, k_vel_small<T, false>, grid, blk, sm, st, V, g, f, q, D, X, c, law, s, it_dev, status, kch, ni, nf);
-    } else if (f.lay) {
-        launch_kernel(true, k_str_small<T, true>, grid, blk, str_ring_bytes<T, true>(), st, S, g, f, q, D, X, c, status, kch, ni, nf);
+        auto k = f.lay ? (any ? k_vel_small<T, true, F32> : k_vel_small<T, true, false>)
+                       : (any ? k_vel_small<T, false, F32> : k_vel_small<T, false, false>);
+        launch_kernel(true, k, grid, blk, sm, st, V, g, f, q, D, X, c, law, s, it_dev, status, kch, ni, nf);
     } else {
-        launch_kernel(true, k_str_small<T, false>, grid, blk, str_ring_bytes<T, false>(), st, S, g, f, q, D, X, c, status, kch, ni, nf);
+        auto k = f.lay ? (any ? k_str_small<T, true, F32> : k_str_small<T, true, false>)
+                       : (any ? k_str_small<T, false, F32> : k_str_small<T, false, false>);
+        launch_kernel(true, k, grid, blk, f.lay ? str_ring_bytes<T, true>() : str_ring_bytes<T, false>(), st, S, g, f, q, D, X, c,
+                      status, kch, ni, nf);
     }
 }
 

@@ -1,8 +1,8 @@
 // fd3d_selftest.cu -- exhaustive device check of the PML quotients against the IEEE division.
 //
 // The PML updates divide by dh and by 1 + omega, divisors known before the launch; div_by and
-// div_by_signed (fd3d_common.cuh) form those quotients from a pair made on the host, and
-// div_small and div_exact those they do not cover.  fd3d_check_division runs them, chosen as the
+// div_by_signed (fd3d_common.cuh) form those quotients from a pair made on the host, div_steps
+// those of a divisor without one, and div_small and div_exact those they do not cover.  fd3d_check_division runs them, chosen as the
 // sweeps choose them, and __fdiv_rn on every one of the 2^32 float bit patterns for each divisor
 // given and counts the dividends whose results differ in any bit (two NaNs count as equal).
 #include <cuda_runtime.h>
@@ -17,16 +17,25 @@ namespace {
 
 struct Pair { float h, l, s; int ok; };
 
+// as quotient() below, for PML_STEPS: y = RN(1/b)
+__device__ float quotient_steps(float x, float b, float y, float s) {
+    unsigned key = 0xffffffffu;
+    const float q = div_steps(x * s, b, y, key) * (1.0f / s);
+    if (!pml_finite(q)) return div_exact(x, b);
+    return key < DIV_KEY ? div_small<true>(x, b, y, 0.0f) : q;
+}
+
 // the sweeps' quotient: div_by on the scaled dividend, or what its key or result asks for
 __device__ float quotient(float x, float b, const Pair& y, bool sign) {
     unsigned key = 0xffffffffu;
     const float xs = x * y.s, q = (sign ? div_by_signed(xs, y.h, y.l, key) : div_by(xs, y.h, y.l, key)) * (1.0f / y.s);
     if (!y.ok || !pml_finite(q)) return div_exact(x, b);
-    return key < DIV_KEY ? div_small(x, b, y.h, y.l) : q;
+    return key < DIV_KEY ? div_small<false>(x, b, y.h, y.l) : q;
 }
 
-// y: the pair with l >= 0 (the divisor dh), ys: the pair of any sign (1 + omega)
-__global__ void k_check_division(float b, Pair y, Pair ys, unsigned long long* bad, unsigned* first) {
+// y: the pair with l >= 0 (the divisor dh), ys: the pair of any sign (1 + omega), recip: RN(1/b), 0
+// for a divisor out of range
+__global__ void k_check_division(float b, Pair y, Pair ys, float recip, unsigned long long* bad, unsigned* first) {
     const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
     unsigned long long local = 0;
     unsigned ex = 0;
@@ -36,7 +45,8 @@ __global__ void k_check_division(float b, Pair y, Pair ys, unsigned long long* b
         const float r = __fdiv_rn(x, b);
         auto is = [&](float q) { return (__float_as_uint(q) == __float_as_uint(r)) || (q != q && r != r); };
         bool same = is(quotient(x, b, y, false)) && is(quotient(x, b, ys, true)) && is(div_exact(x, b));
-        if (ys.ok && pml_finite(x)) same = same && is(div_small(x, b, ys.h, ys.l));
+        if (ys.ok && pml_finite(x)) same = same && is(div_small<false>(x, b, ys.h, ys.l));
+        if (recip != 0.0f) same = same && is(quotient_steps(x, b, recip, y.s)) && (!pml_finite(r) || is(div_small<true>(x, b, recip, 0.0f)));
         if (!same) {
             if (local == 0) ex = bits;
             ++local;
@@ -49,6 +59,13 @@ __global__ void k_check_division(float b, Pair y, Pair ys, unsigned long long* b
 }
 
 }  // namespace
+
+extern "C" int fd3d_division_form(float divisor, int damping, int* form) {
+    if (!form) return FD3D_ERR_ARG;
+    float h, l, y;
+    *form = div_form(divisor, damping != 0, h, l, y);
+    return FD3D_OK;
+}
 
 extern "C" int fd3d_check_division(const float* divisors, int n, unsigned long long* mismatches,
                                    unsigned* first_bad) {
@@ -69,13 +86,14 @@ extern "C" int fd3d_check_division(const float* divisors, int n, unsigned long l
         y.s = ys.s = b > 0 ? (float)div_scale(b) : 1.0f;
         y.ok = div_pair(b, true, y.h, y.l);
         ys.ok = div_pair(b, false, ys.h, ys.l);
+        const float recip = div_in_range(b) ? ys.h : 0.0f;
         const unsigned none = 0xffffffffu;
         if (cudaMemset(dbad, 0, sizeof(unsigned long long)) != cudaSuccess ||
             cudaMemcpy(dfirst, &none, sizeof(unsigned), cudaMemcpyHostToDevice) != cudaSuccess) {
             rc = FD3D_ERR_CUDA;
             break;
         }
-        k_check_division<<<nsm * 8, 256>>>(b, y, ys, dbad, dfirst);
+        k_check_division<<<nsm * 8, 256>>>(b, y, ys, recip, dbad, dfirst);
         unsigned long long hb = 0;
         unsigned hf = none;
         if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||

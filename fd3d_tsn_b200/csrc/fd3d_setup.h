@@ -117,11 +117,12 @@ inline bool div_pair_holds(float b, float h, float l, int64_t RM) {
     }
     return true;
 }
-// nonneg: only pairs with l >= 0 (the sign of a zero dividend is kept without more work).
-// false: no pair found (or b out of range); the sweeps use div_exact then.
+// nonneg: only pairs with l >= 0 (the sign of a zero dividend is kept without more work); otherwise h
+// is RN(1/b), with or without a pair.  false: no pair found (see PmlForm), or b out of range.
+inline bool div_in_range(float b) { return b >= 0x1p-20f && b <= 0x1p20f; }
 inline bool div_pair(float b, bool nonneg, float& h, float& l) {
     h = l = 0.f;
-    if (!(b >= 0x1p-20f && b <= 0x1p20f)) return false;
+    if (!div_in_range(b)) return false;
     const double z = 1.0 / (double)b;
     h = (float)z;
     if (nonneg && (double)h > z) h = std::nextafterf(h, 0.f);
@@ -133,9 +134,18 @@ inline bool div_pair(float b, bool nonneg, float& h, float& l) {
             if (div_pair_holds(b, h, l, nonneg ? 80 : 16)) return true;
         }
     }
+    h = (float)z;
     return false;
 }
-inline bool div_pair(double, bool, double& h, double& l) { h = l = 0; return true; }  // divides directly
+// The PmlForm that one divisor asks for; h, l its pair if it has one, y = RN(1/b) (0 out of range).
+// signed_ok: a pair of either sign serves as well as one with l >= 0 (1 + omega)
+inline int div_form(float b, bool signed_ok, float& h, float& l, float& y) {
+    y = div_in_range(b) ? (float)(1.0 / (double)b) : 0.f;
+    if (div_pair(b, !signed_ok, h, l)) return PML_PAIR;
+    if (!signed_ok && div_pair(b, false, h, l)) return PML_SIGNED;
+    return div_in_range(b) ? PML_STEPS : PML_EXACT;
+}
+inline int div_form(double, bool, double& h, double& l, double& y) { h = l = y = 0; return PML_PAIR; }  // divides directly
 // The scale of div_by's dividends for divisors up to b: a scaled dividend of 2^-70 or more has a
 // quotient by b that is a normal number when it is scaled back, 2^-70 / S / b >= 2^-126.
 inline double div_scale(double b) { return std::ldexp(1.0, std::min(56, 56 - (int)std::ceil(std::log2(b)))); }
@@ -210,7 +220,7 @@ void make_pml(const fd3d_params& p, PmlDesc& D, std::vector<Damp<T>>& prof) {
     }
     for (int s = 0; s <= PML_MAXS; ++s) D.tile0[s] = (int)(D.cum[s] / PML_TILE);
     std::vector<Damp<T>> pairs;  // the strips share their divisors: one search for each
-    D.exact = 0;
+    D.form = PML_PAIR;
     D.bmax = 1.0;
     for (int s = 0; s < D.ns; ++s) {
         Strip& S = D.s[s];
@@ -225,7 +235,9 @@ void make_pml(const fd3d_params& p, PmlDesc& D, std::vector<Damp<T>>& prof) {
                 if (last < 0 || pairs[last].p != e.p) {
                     for (last = 0; last < (int)pairs.size() && pairs[last].p != e.p;) ++last;
                     if (last == (int)pairs.size()) {
-                        if (!div_pair(e.p, false, e.h, e.l)) D.exact = 1;
+                        T y;
+                        D.form = std::max(D.form, div_form(e.p, true, e.h, e.l, y));
+                        e.h = y;  // (the pair's, if there is one)
                         pairs.push_back(e);
                     }
                 }
@@ -281,7 +293,7 @@ StepConst<T> make_const(const fd3d_params& p, const PmlDesc& D) {
     const double scale = div_scale(std::max(D.bmax, (double)c.dh));
     c.ds = (T)scale;
     c.dsi = (T)(1.0 / scale);
-    c.pml_exact = !div_pair(c.dh, true, c.rdh, c.rdl) || D.exact;
+    c.pml_form = std::max(D.form, div_form(c.dh, false, c.rdh, c.rdl, c.ydh));
     c.dtA = p.dt;
     c.dhA = (double)c.dh;
     c.dthA = c.dtA / c.dhA;

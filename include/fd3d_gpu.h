@@ -340,6 +340,15 @@ int fd3d_slab_run(fd3d_ctx* ctx, int nsteps);       /* then fd3d_sync(ctx) */
  * of dividends whose quotients differ (0 expected) and the first such bit pattern
  * (0xffffffff if none). */
 int fd3d_check_division(const float* divisors, int n, unsigned long long* mismatches, unsigned* first_bad);
+/* Which quotient the single-precision PML kernels use for a divisor (host arithmetic only): a
+ * spacing dh (damping 0) or a 1 + omega (damping 1).  A model takes the largest form of its
+ * divisors for all of them: two operations; two and a sign, for a spacing; five; or FP64 division,
+ * outside [2^-20, 2^20] only. */
+#define FD3D_DIVISION_PAIR   0
+#define FD3D_DIVISION_SIGNED 1
+#define FD3D_DIVISION_STEPS  2
+#define FD3D_DIVISION_EXACT  3
+int fd3d_division_form(float divisor, int damping, int* form);
 /* Self-test of the bounded device waits (no counterpart in the reference, whose GPU
  * regions never wait on each other): a kernel waits on an mbarrier phase that nothing
  * completes and a grid barrier that one CTA never reaches.  Both waits must give up after
