@@ -233,6 +233,8 @@ struct CtxBase {
     virtual int save_state(std::FILE* fp) = 0;
     virtual int load_state(std::FILE* fp) = 0;
     virtual bool layered() const = 0;
+    // fd3d_ctx_step_info
+    virtual int step_info(int* one_launch, int* pml_form, int* pml_ctas_vel, int* pml_ctas_str) = 0;
 };
 
 template <class T>
@@ -370,10 +372,8 @@ struct Ctx : CtxBase {
         X.prof = dprof;
         tma_ok = make_interior_maps<T>(g, f, vmaps, smaps) && prepare_tma_kernels<T>();
         if (slab && !tma_ok) return FD3D_ERR_CUDA;
-        // measured fastest (0.214 G cells, us): velocity 293 at 4 (330 at 3, 72 registers), stress 389
-        // at 4 (424 at 3; 5 spills, 399); FP64 (0.6 M cells) 20 at 3, 30 at 2 (no spills)
-        if (!pml_minb_vel) pml_minb_vel = sizeof(T) == 8 ? 3 : 4;
-        if (!pml_minb_str) pml_minb_str = sizeof(T) == 8 ? 2 : 4;
+        if (!pml_minb_vel) pml_minb_vel = pml_minb<T>(false);
+        if (!pml_minb_str) pml_minb_str = pml_minb<T>(true);
         small_grid = small_step(icfg, g, D);
         if (!tma_ok && icfg.variant == IV_TMA) {
             std::fprintf(stderr, "fd3d: tensor maps of the interior sweeps could not be encoded for this grid; "
@@ -688,6 +688,27 @@ struct Ctx : CtxBase {
         return FD3D_OK;
     }
 
+    // the half-steps as one launch each (small_step), unless something asks for the separate launches
+    bool one_launch() const { return small_grid && overlap > 0 && !profiling && !split_bc && icfg.variant == IV_TMA; }
+
+    int step_info(int* one, int* form, int* ctas_vel, int* ctas_str) override {
+        const bool any = c.pml_form != PML_PAIR;
+        if (one) *one = one_launch();
+        if (form) *form = c.pml_form;
+        int* out[2] = {ctas_vel, ctas_str};
+        for (int s = 0; s < 2; ++s) {
+            if (!out[s]) continue;
+            if (one_launch()) {
+                CK(s ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(out[s], str_small_kernel<T>(f.lay, any), 256, str_small_smem<T>(f.lay))
+                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(out[s], vel_small_kernel<T>(f.lay, any), 256, vel_ring_bytes<T>()));
+            } else {
+                CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                    out[s], pml_kernel<T>(s, s ? pml_minb_str : pml_minb_vel, pml_slab(g, D), any), PML_TILE, 0));
+            }
+        }
+        return FD3D_OK;
+    }
+
     // Phase 0 the velocity half-step, 1 the stress sweeps, 2-4 the fault boundary
     // condition (fused into phase 2 for a whole model; fres + traction, friction, output
     // as separate launches for a z-slab or when split_bc is set) and the nucleation ramp.
@@ -696,7 +717,7 @@ struct Ctx : CtxBase {
         const int nzT = std::max(1, g.kin_hi() - g.kin_lo() + 1);  // fault rows updated (a launch has one at least)
         const dim3 b2(32, 8);
         const bool ov = overlap > 0 && !profiling;
-        const bool small = small_grid && ov && !split_bc && icfg.variant == IV_TMA;
+        const bool small = one_launch();
         const bool top = g.owns(g.ks());  // the free-surface rows are this context's
         cudaStream_t sp = ov ? st2 : st;  // fault band and PML
         auto fork = [&](int e) { cudaEventRecord(evf[e], st); cudaStreamWaitEvent(st2, evf[e], 0); };
@@ -1156,6 +1177,11 @@ int fd3d_ctx_info(fd3d_ctx* ctx, int* interior_variant, int* layered_medium) {
     if (interior_variant) *interior_variant = c->icfg.variant;
     if (layered_medium) *layered_medium = c->layered() ? 1 : 0;
     return FD3D_OK;
+}
+
+int fd3d_ctx_step_info(fd3d_ctx* ctx, int* one_launch, int* pml_form, int* pml_ctas_vel, int* pml_ctas_str) {
+    if (!ctx) return FD3D_ERR_ARG;
+    return ctx->impl->step_info(one_launch, pml_form, pml_ctas_vel, pml_ctas_str);
 }
 
 int fd3d_history_records(fd3d_ctx* ctx, int* nrec) {

@@ -1526,42 +1526,54 @@ inline void pml_strip_tiles(const PmlDesc& D, int s, long long& t0, long long& t
     t1 = (D.cum[s] + (long long)(ke - S.nzb + 1) * per_k + PML_TILE - 1) / PML_TILE;
 }
 
-template <class T, int MINB, bool SLAB, bool ANY>
-inline void launch_pml_n(bool stress, cudaStream_t st, const Grid& g, const Fields<T>& f, const PmlDesc& D,
-                         const PmlAux<T>& X, const StepConst<T>& c, int* status, long long t0, long long t1) {
-    if (t1 <= t0) return;
-    const unsigned n = (unsigned)(t1 - t0);
-    if (stress) k_str_pml<T, MINB, SLAB, ANY><<<n, PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
-    else k_vel_pml<T, MINB, SLAB, ANY><<<n, PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
+// CTAs per SM that the PML sweeps are compiled for, measured fastest.  0.214 G cells, us: velocity 293
+// at 4 (330 at 3, 72 registers), stress 389 at 4 (424 at 3; 5 spills, 399); FP64 (0.6 M cells) 20 at 3, 30
+// at 2 (no spills).  A z-slab (us a step of two slabs of 14 M and 68 M cells: 519 and 1641 against 539 and
+// 1684 without a cap) and quotients of a form of their own always take these.
+template <class T>
+constexpr int pml_minb(bool stress) { return sizeof(T) == 4 ? 4 : stress ? 2 : 3; }
+template <class T>
+using PmlKernel = void (*)(Grid, Fields<T>, PmlDesc, PmlAux<T>, StepConst<T>, int*, long long);
+template <class T, bool STRESS, bool SLAB, bool ANY, int MINB = pml_minb<T>(STRESS)>
+constexpr PmlKernel<T> pml_kernel_of() {
+    if constexpr (STRESS) return k_str_pml<T, MINB, SLAB, ANY>;
+    else return k_vel_pml<T, MINB, SLAB, ANY>;
 }
+template <class T, bool STRESS>
+inline PmlKernel<T> pml_kernel(int minb, bool slab, bool any) {
+    constexpr bool F32 = sizeof(T) == 4;  // (FP64 divides directly: one form)
+    if (slab) return any ? pml_kernel_of<T, STRESS, true, F32>() : pml_kernel_of<T, STRESS, true, false>();
+    if (any) return pml_kernel_of<T, STRESS, false, F32>();
+    switch (minb) {
+        case 2: return pml_kernel_of<T, STRESS, false, false, 2>();
+        case 3: return pml_kernel_of<T, STRESS, false, false, 3>();
+        case 4: return pml_kernel_of<T, STRESS, false, false, 4>();
+        case 5: return pml_kernel_of<T, STRESS, false, false, 5>();
+        default: return pml_kernel_of<T, STRESS, false, false, 1>();
+    }
+}
+template <class T>
+inline PmlKernel<T> pml_kernel(bool stress, int minb, bool slab, bool any) {
+    return stress ? pml_kernel<T, true>(minb, slab, any) : pml_kernel<T, false>(minb, slab, any);
+}
+inline bool pml_slab(const Grid& g, const PmlDesc& D) { return D.klo > 1 || D.khi < g.nzt; }
+
 // launch of a PML sweep: one launch over every tile for a whole model (with a register
-// cap picked at run time; four CTAs per SM where the quotients take a form of their own), one
-// per strip over the tiles of its planes for a z-slab
+// cap picked at run time), one per strip over the tiles of its planes for a z-slab
 template <class T>
 inline void launch_pml(bool stress, int minb, cudaStream_t st, const Grid& g, const Fields<T>& f, const PmlDesc& D,
                        const PmlAux<T>& X, const StepConst<T>& c, int* status) {
-    constexpr bool F32 = sizeof(T) == 4;  // (FP64 divides directly: one form)
-    const bool any = F32 && c.pml_form != PML_PAIR;
-    if (D.klo > 1 || D.khi < g.nzt) {  // a z-slab: the tiles of its planes, strip by strip
-        for (int s = 0; s < D.ns; ++s) {
-            long long t0, t1;
-            pml_strip_tiles(D, s, t0, t1);
-            if (any) launch_pml_n<T, 1, true, F32>(stress, st, g, f, D, X, c, status, t0, t1);
-            else launch_pml_n<T, 1, true, false>(stress, st, g, f, D, X, c, status, t0, t1);
-        }
+    const bool slab = pml_slab(g, D);
+    const PmlKernel<T> k = pml_kernel<T>(stress, minb, slab, c.pml_form != PML_PAIR);
+    if (!slab) {
+        const unsigned n = (unsigned)(D.cum[PML_MAXS] / PML_TILE);
+        if (n) k<<<n, PML_TILE, 0, st>>>(g, f, D, X, c, status, 0);
         return;
     }
-    const long long n = D.cum[PML_MAXS] / PML_TILE;
-    if (any) {
-        launch_pml_n<T, 4, false, F32>(stress, st, g, f, D, X, c, status, 0, n);
-        return;
-    }
-    switch (minb) {
-        case 2: launch_pml_n<T, 2, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
-        case 3: launch_pml_n<T, 3, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
-        case 4: launch_pml_n<T, 4, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
-        case 5: launch_pml_n<T, 5, false, false>(stress, st, g, f, D, X, c, status, 0, n); break;
-        default: launch_pml_n<T, 1, false, false>(stress, st, g, f, D, X, c, status, 0, n);
+    for (int s = 0; s < D.ns; ++s) {
+        long long t0, t1;
+        pml_strip_tiles(D, s, t0, t1);
+        if (t1 > t0) k<<<(unsigned)(t1 - t0), PML_TILE, 0, st>>>(g, f, D, X, c, status, t0);
     }
 }
 

@@ -489,20 +489,38 @@ k_str_small(const __grid_constant__ StrMaps M, const __grid_constant__ Grid g, c
     }
 }
 
+// the kernels of a medium (layered or not) and quotient form (FP64 has one)
+template <class T>
+inline auto vel_small_kernel(bool layered, bool any) {
+    constexpr bool F32 = sizeof(T) == 4;
+    return layered ? (any ? k_vel_small<T, true, F32> : k_vel_small<T, true, false>)
+                   : (any ? k_vel_small<T, false, F32> : k_vel_small<T, false, false>);
+}
+template <class T>
+inline auto str_small_kernel(bool layered, bool any) {
+    constexpr bool F32 = sizeof(T) == 4;
+    return layered ? (any ? k_str_small<T, true, F32> : k_str_small<T, true, false>)
+                   : (any ? k_str_small<T, false, F32> : k_str_small<T, false, false>);
+}
+template <class T>
+constexpr int vel_ring_bytes() { return TMA_NS * VelSlot::ELEMS * (int)sizeof(T) + TMA_SMEM_PAD; }
+template <class T>
+constexpr int str_small_smem(bool layered) { return layered ? str_ring_bytes<T, true>() : str_ring_bytes<T, false>(); }
+
 template <class T>
 bool prepare_tma_kernels() {
-    const int vs = TMA_NS * VelSlot::ELEMS * (int)sizeof(T) + TMA_SMEM_PAD, ss = str_ring_bytes<T, false>(),
+    const int vs = vel_ring_bytes<T>(), ss = str_ring_bytes<T, false>(),
               ssl = str_ring_bytes<T, true>();
     bool ok = cudaFuncSetAttribute(k_vel_interior_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_vel_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssl) == cudaSuccess;
-    constexpr bool F32 = sizeof(T) == 4;
-    auto ring = [&](auto k, int bytes) { ok &= cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess; };
-    ring(k_vel_small<T, false, false>, vs); ring(k_vel_small<T, false, F32>, vs);
-    ring(k_vel_small<T, true, false>, vs); ring(k_vel_small<T, true, F32>, vs);
-    ring(k_str_small<T, false, false>, ss); ring(k_str_small<T, false, F32>, ss);
-    ring(k_str_small<T, true, false>, ssl); ring(k_str_small<T, true, F32>, ssl);
+    for (bool layered : {false, true})
+        for (bool any : {false, true}) {
+            ok &= cudaFuncSetAttribute(vel_small_kernel<T>(layered, any), cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
+            ok &= cudaFuncSetAttribute(str_small_kernel<T>(layered, any), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       layered ? ssl : ss) == cudaSuccess;
+        }
     if (!ok) cudaGetLastError();
     return ok;
 }
@@ -535,19 +553,13 @@ void launch_half_small(bool stress, const VelMaps& V, const StrMaps& S, const In
     int kch;
     dim3 ni, nf;
     const dim3 grid(half_small_grid(stress, cfg, g, D, kch, ni, nf)), blk(32, 8);
-    constexpr bool F32 = sizeof(T) == 4;
-    const bool any = F32 && c.pml_form != PML_PAIR;
-    if (!stress) {
-        const size_t sm = TMA_NS * VelSlot::ELEMS * sizeof(T) + TMA_SMEM_PAD;
-        auto k = f.lay ? (any ? k_vel_small<T, true, F32> : k_vel_small<T, true, false>)
-                       : (any ? k_vel_small<T, false, F32> : k_vel_small<T, false, false>);
-        launch_kernel(true, k, grid, blk, sm, st, V, g, f, q, D, X, c, law, s, it_dev, status, kch, ni, nf);
-    } else {
-        auto k = f.lay ? (any ? k_str_small<T, true, F32> : k_str_small<T, true, false>)
-                       : (any ? k_str_small<T, false, F32> : k_str_small<T, false, false>);
-        launch_kernel(true, k, grid, blk, f.lay ? str_ring_bytes<T, true>() : str_ring_bytes<T, false>(), st, S, g, f, q, D, X, c,
+    const bool any = c.pml_form != PML_PAIR;
+    if (!stress)
+        launch_kernel(true, vel_small_kernel<T>(f.lay, any), grid, blk, vel_ring_bytes<T>(), st, V, g, f, q, D, X, c, law, s, it_dev,
                       status, kch, ni, nf);
-    }
+    else
+        launch_kernel(true, str_small_kernel<T>(f.lay, any), grid, blk, str_small_smem<T>(f.lay), st, S, g, f, q, D, X, c, status,
+                      kch, ni, nf);
 }
 
 template <class T>

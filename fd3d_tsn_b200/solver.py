@@ -147,6 +147,14 @@ class Solver:
         _ck(lib().fd3d_ctx_info(self.h, C.byref(v), C.byref(lay)), "fd3d_ctx_info")
         return dict(interior_variant=self.INTERIOR_VARIANTS.get(v.value, str(v.value)), layered_medium=bool(lay.value))
 
+    def step_info(self) -> dict:
+        """Which launches the next step takes: one per half-step or several, the form of the PML
+        quotients (0 pair, 1 signed pair, 2 five operations, 3 FP64) and the CTAs per SM of the
+        kernels that hold the PML tiles."""
+        v = [C.c_int() for _ in range(4)]
+        _ck(lib().fd3d_ctx_step_info(self.h, *(C.byref(x) for x in v)), "fd3d_ctx_step_info")
+        return dict(one_launch=bool(v[0].value), pml_form=v[1].value, pml_ctas_vel=v[2].value, pml_ctas_str=v[3].value)
+
     # ------------------------------------------------------------ outputs
     def history_records(self) -> int:
         n = C.c_int()

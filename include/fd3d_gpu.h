@@ -246,6 +246,11 @@ int fd3d_kernel_times(fd3d_ctx* ctx, float* ms /* FD3D_NKERNELS */, int* launche
 #define FD3D_INTERIOR_PIPE  2
 #define FD3D_INTERIOR_TMA   3
 int fd3d_ctx_info(fd3d_ctx* ctx, int* interior_variant, int* layered_medium);
+/* Which launches the next step takes.  one_launch: 1 when each half-step is one launch (small
+ * grids, no profiling, no z-slab).  pml_form: the FD3D_DIVISION_* form of the model's PML
+ * quotients.  pml_ctas_vel, pml_ctas_str: CTAs per SM at which the kernels that hold the velocity
+ * and stress PML tiles run.  Any pointer may be NULL. */
+int fd3d_ctx_step_info(fd3d_ctx* ctx, int* one_launch, int* pml_form, int* pml_ctas_vel, int* pml_ctas_str);
 #define FD3D_NKERNELS 8
 /* kernel ids in fd3d_kernel_times: 0 vel_interior, 1 vel_fault, 2 vel_pml, 3 vel_fs,
    4 str_interior, 5 str_fault, 6 str_pml, 7 fault_bc (traction+friction+output) */
