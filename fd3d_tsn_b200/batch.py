@@ -37,6 +37,7 @@ def _bind():
         "fd3d_batch_set_tuning": (i, [vp, i, i]),
         "fd3d_batch_get_tuning": (i, [vp, C.POINTER(i), C.POINTER(i), C.POINTER(i)]),
         "fd3d_batch_autotune": (i, [vp, i, C.c_char_p, C.c_char_p]),
+        "fd3d_batch_step_info": (i, [vp, C.POINTER(i), C.POINTER(i)]),
         "fd3d_batch_set_schedule": (i, [vp, i]),
         "fd3d_batch_get_schedule": (i, [vp, C.POINTER(i)]),
     }
@@ -147,6 +148,13 @@ class Batch:
         """"graph" (CUDA graphs of kernels over all models) or "persistent", which runs the
         same launches."""
         _ck(lib().fd3d_batch_set_schedule(self.h, SCHEDULES[mode]), "fd3d_batch_set_schedule")
+
+    def step_info(self) -> dict:
+        """Which launches the next run takes: one per half-step (merged) or one per region, and the
+        work items of a velocity half-step."""
+        a, n = C.c_int(), C.c_int()
+        _ck(lib().fd3d_batch_step_info(self.h, C.byref(a), C.byref(n)), "fd3d_batch_step_info")
+        return dict(merged=bool(a.value), items=n.value)
 
     def tuning(self):
         a, b, c = C.c_int(), C.c_int(), C.c_int()

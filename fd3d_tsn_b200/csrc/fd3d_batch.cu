@@ -450,6 +450,7 @@ struct fd3d_batch {
                                  // (measured 2.3-2.5% slower: the early CTAs hold SM slots in the tail)
     int branches = 0;            // graph schedule: fault-band and PML sweeps on side streams (1) or in
                                  // series on the main stream (0, measured 9-11% faster: the branches interfered)
+    int merged = -1;             // 1 / 0: one launch per half-step always / never (-1: merged_step's rule)
     int** d_stptr = nullptr;     // status words of the live models (k_or_status)
     int n_stptr = 0;
     int* d_status_or = nullptr;
@@ -591,7 +592,8 @@ int build_work(fd3d_batch* b) {
 // planes: 1 model (0.7 K items or more) 48 / 67, 4 models 148 / 170, 12 models 393 / 400, 16 models 505 /
 // 506, 32 models 967 / 946; tiles of 32 planes: 74 / 103, 140 / 193, 386 / 407, 495 / 519, 957 / 957.
 bool merged_step(const fd3d_batch* b) {
-    return !b->branches && b->tbeg[W_VEL_FS] - b->tbeg[W_VEL_INT] <= 120 * b->nsm;
+    if (b->branches || b->merged == 0) return false;
+    return b->merged == 1 || b->tbeg[W_VEL_FS] - b->tbeg[W_VEL_INT] <= 120 * b->nsm;
 }
 bool all_slip_weakening(const fd3d_batch* b) {
     for (const Model& M : b->models)
@@ -856,6 +858,8 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
     if (const char* e = std::getenv("FD3D_BATCH_BRANCHES")) b->branches = std::atoi(e) != 0;
     // FD3D_BATCH_PDL=1: the graph schedule's kernels with programmatic dependent launch
     if (const char* e = std::getenv("FD3D_BATCH_PDL")) b->pdl = std::atoi(e) != 0;
+    // FD3D_BATCH_MERGED=1|0: one launch per half-step, or one per region, whatever the batch's size
+    if (const char* e = std::getenv("FD3D_BATCH_MERGED")) b->merged = std::atoi(e) != 0;
     // FD3D_BATCH_MODE=persistent|graph
     if (const char* e = std::getenv("FD3D_BATCH_MODE"))
         b->tun.mode = std::strcmp(e, "persistent") == 0 ? MODE_PERSISTENT : MODE_GRAPH;
@@ -1059,6 +1063,18 @@ int fd3d_batch_run(fd3d_batch* b, int nsteps) {
     BCK(cudaEventRecord(b->ev1, b->st));
     for (size_t m = 0; m < b->models.size(); ++m)
         if (b->models[m].live) b->models[m].steps += limit[m];
+    return FD3D_OK;
+}
+
+int fd3d_batch_step_info(fd3d_batch* b, int* merged, int* items) {
+    if (!b) return FD3D_ERR_ARG;
+    std::lock_guard<std::mutex> lk(b->mu);
+    if (b->dirty || b->built_kchunk != b->tun.kchunk) {
+        int rc = build_work(b);
+        if (rc) return rc;
+    }
+    if (merged) *merged = merged_step(b);
+    if (items) *items = b->tbeg[W_VEL_FS] - b->tbeg[W_VEL_INT];
     return FD3D_OK;
 }
 

@@ -291,6 +291,10 @@ int fd3d_batch_fetch_history(fd3d_batch* b, int slot, int field, int rec0, int n
 /* tile shape: z-planes per interior tile; ctas_per_sm (0 = max) is kept and reported, no launch depends on it */
 int fd3d_batch_set_tuning(fd3d_batch* b, int kchunk, int ctas_per_sm);
 int fd3d_batch_get_tuning(fd3d_batch* b, int* kchunk, int* ctas_per_sm, int* max_ctas_per_sm);
+/* Which launches the next run takes: merged, 1 when each half-step is one launch (small batches;
+ * FD3D_BATCH_MERGED=1 or 0 in the environment at creation fixes it); items, the work items of a
+ * velocity half-step, which the rule goes by.  Either pointer may be NULL. */
+int fd3d_batch_step_info(fd3d_batch* b, int* merged, int* items);
 /* schedule: FD3D_BATCH_PERSISTENT or FD3D_BATCH_GRAPH (the default) */
 int fd3d_batch_set_schedule(fd3d_batch* b, int mode);
 int fd3d_batch_get_schedule(fd3d_batch* b, int* mode);
