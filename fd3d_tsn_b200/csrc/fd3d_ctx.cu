@@ -374,7 +374,7 @@ struct Ctx : CtxBase {
         if (slab && !tma_ok) return FD3D_ERR_CUDA;
         if (!pml_minb_vel) pml_minb_vel = pml_minb<T>(false);
         if (!pml_minb_str) pml_minb_str = pml_minb<T>(true);
-        small_grid = small_step(icfg, g, D);
+        small_grid = small_step<T>(icfg, law, g, D);
         if (!tma_ok && icfg.variant == IV_TMA) {
             std::fprintf(stderr, "fd3d: tensor maps of the interior sweeps could not be encoded for this grid; "
                                  "the interior sweeps fall back to plain loads (fd3d_ctx_info reports it)\n");

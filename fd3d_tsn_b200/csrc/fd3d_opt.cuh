@@ -534,15 +534,26 @@ inline unsigned half_small_grid(bool stress, const InteriorCfg& cfg, const Grid&
     nf = dim3(stress ? (nxT + 31) / 32 : (g.nxt + 31) / 32, (nzT + 7) / 8, stress ? STR_FAULT_PARTS : VEL_FAULT_PARTS);
     return ni.x * ni.y * ni.z + nf.x * nf.y * nf.z + (unsigned)(D.cum[PML_MAXS] / PML_TILE);
 }
-// Whether a model takes one launch per half-step: up to twelve CTAs per SM, three waves at the
-// four that fit (FP32).  Beyond that the interior CTAs miss the fifth and sixth place per SM that
-// they have in a launch of their own.  A solve, one launch / separate launches: 0.2 K CTAs 1.76 /
-// 1.95 ms, 1.4 K 36.7 / 38.7, 1.5 K 13.4 / 15.1 (rate-and-state), FP64 1.4 K 13.9 / 14.1; 2.7 K 88.4 /
-// 87.7 and 18.7 / 17.7, 9 K 22.3 / 21.7.
-inline bool small_step(const InteriorCfg& cfg, const Grid& g, const PmlDesc& D) {
+// Whether a model takes one launch per half-step: up to twelve CTAs per SM, nine and a half for
+// slip weakening in FP64, where only two fit (four in FP32).  Beyond that the interior CTAs miss the
+// places per SM that they have in a launch of their own; below it the launches' starts and tails
+// count for more, most of all the rate-and-state fault kernels'.  Speed of one launch over that
+// of separate launches, mean over the shapes in each range of CTAs of the velocity half-step:
+//   thousand CTAs              0.4-1.0  1.0-1.2  1.2-1.4  1.4-1.8  2.0-2.8
+//   FP32 slip weakening           1.09     1.07     1.04     1.02     0.93
+//     3-D medium                  1.08     1.05     1.02     0.99     0.93
+//     full space                  1.10     1.08     1.04     1.03     0.95
+//   FP32 rate-and-state           1.21              1.20     1.17     1.01
+//   FP64 slip weakening           1.08     1.01     0.96     0.93     0.92
+//   FP64 rate-and-state           1.22     1.09     1.06     1.02     0.95
+// (FP64 slip weakening from 1.2 to 1.4 K runs from 0.89 to 1.01 by shape, above that from 0.87 to 0.97 but for
+// one at 1.05.)
+template <class T>
+inline bool small_step(const InteriorCfg& cfg, int law, const Grid& g, const PmlDesc& D) {
     int kch;
     dim3 ni, nf;
-    return half_small_grid(false, cfg, g, D, kch, ni, nf) <= 12u * (unsigned)cfg.nsm;
+    const unsigned halves = sizeof(T) == 8 && law == 0 ? 19 : 24;
+    return 2 * half_small_grid(false, cfg, g, D, kch, ni, nf) <= halves * (unsigned)cfg.nsm;
 }
 
 // the two half-steps of a small grid (k_vel_small, k_str_small)

@@ -8,7 +8,8 @@ from fd3d_tsn_b200.solver import Solver
 pytestmark = pytest.mark.gpu
 
 
-# CTAs of a velocity half-step (12 x 148 = 1776 is the border): 62 to 338, 1625, 2219 and 2000
+# CTAs of a velocity half-step (12 x 148 = 1776 is the border): 62 to 338, 1625, 2219 and 2000; for slip
+# weakening in double precision 9.5 x 148 = 1406: 1171 and 1359, 1438 and 1556
 @pytest.mark.parametrize("law,precision,fspace,size,one_launch", [
     ("sw", "f32", False, (14, 9, 13), True),
     ("sw", "f32", False, (33, 12, 41), True),
@@ -20,6 +21,12 @@ pytestmark = pytest.mark.gpu
     ("sw", "f32", False, (121, 47, 83), True),
     ("sw", "f32", False, (161, 61, 93), False),
     ("sw", "f32", True, (129, 55, 87), False),
+    ("sw", "f64", False, (90, 50, 70), True),
+    ("sw", "f64", False, (101, 47, 73), True),
+    ("sw", "f64", False, (96, 56, 80), False),
+    ("sw", "f64", False, (160, 40, 70), False),
+    ("fvw", "f64", False, (160, 40, 70), True),
+    ("sw", "f32", False, (160, 40, 70), True),
 ])
 def test_one_launch_per_half_step_by_size(law, precision, fspace, size, one_launch, monkeypatch):
     nx, ny, nz = size
