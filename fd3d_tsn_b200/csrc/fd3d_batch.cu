@@ -405,6 +405,10 @@ struct Model {
 
 enum { MODE_PERSISTENT = FD3D_BATCH_PERSISTENT, MODE_GRAPH = FD3D_BATCH_GRAPH };
 
+// Part of the key of a saved tuning: raised whenever the launches that it was timed on change, so
+// that an older line is timed again (a line without it may be of the cooperative kernel that is gone).
+constexpr int TUNING_LAUNCHES = 2;
+
 struct Tuning {
     int kchunk = 16;
     int per_sm = 0;     // CTAs per SM the caller set (kept for fd3d_batch_get_tuning; no launch depends on it)
@@ -1226,7 +1230,7 @@ int fd3d_batch_get_tuning(fd3d_batch* b, int* kchunk, int* ctas_per_sm, int* max
     return FD3D_OK;
 }
 
-// Times each (kchunk, CTAs/SM) candidate for `steps` steps on the live models (all
+// Times each tile depth for `steps` steps on the live models (all
 // of which must be at step 0), keeps the fastest, resets every model to step 0, and
 // records the choice under `key` in the JSON-lines cache file (if given).  A cache
 // hit skips the timing.
@@ -1236,21 +1240,21 @@ int fd3d_batch_autotune(fd3d_batch* b, int steps, const char* cache_path, const 
     for (const Model& M : b->models)
         if (M.live && M.steps != 0) return FD3D_ERR_STATE;
     std::string k = key ? key : "";
-    if (!k.empty()) {  // a tuning holds for one kind of device only
+    if (!k.empty()) {  // a tuning holds for one kind of device, and for the launches it was timed on
         int dev = 0;
         cudaDeviceProp prop{};
         BCK(cudaGetDevice(&dev));
         BCK(cudaGetDeviceProperties(&prop, dev));
         for (char& ch : prop.name) if (ch == '"') ch = '\'';
-        k += std::string("|") + prop.name + "|sm" + std::to_string(prop.multiProcessorCount);
+        k += std::string("|") + prop.name + "|sm" + std::to_string(prop.multiProcessorCount) + "|launches" + std::to_string(TUNING_LAUNCHES);
     }
     if (cache_path && !k.empty()) {
         std::ifstream in(cache_path);
         std::string line;
         while (std::getline(in, line)) {
             int kc = 0, ps = 0, mode = -1;
-            char buf[256] = {0};
-            if (std::sscanf(line.c_str(), "{\"key\": \"%255[^\"]\", \"schedule\": %d, \"kchunk\": %d, \"ctas_per_sm\": %d",
+            char buf[512] = {0};
+            if (std::sscanf(line.c_str(), "{\"key\": \"%511[^\"]\", \"schedule\": %d, \"kchunk\": %d, \"ctas_per_sm\": %d",
                             buf, &mode, &kc, &ps) == 4 &&
                 k == buf && kc > 0 && (mode == MODE_GRAPH || mode == MODE_PERSISTENT)) {
                 b->tun.mode = mode;
