@@ -815,10 +815,7 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
     if (cudaGetDeviceCount(&n) != cudaSuccess || n == 0) { cudaGetLastError(); return FD3D_ERR_NODEV; }
     fd3d_batch* b = new fd3d_batch();
     cudaGetDevice(&b->dev);
-    int coop = 0;
-    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, b->dev);
     cudaDeviceGetAttribute(&b->nsm, cudaDevAttrMultiProcessorCount, b->dev);
-    if (!coop) { delete b; return FD3D_ERR_NODEV; }
     auto fail = [&](int rc) { fd3d_batch_destroy(b); return rc; };
     if (cudaStreamCreateWithFlags(&b->st, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&b->sst, cudaStreamNonBlocking) != cudaSuccess)
