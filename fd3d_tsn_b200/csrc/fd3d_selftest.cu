@@ -1,10 +1,12 @@
-// fd3d_selftest.cu -- exhaustive device check of the PML quotients against the IEEE division.
+// fd3d_selftest.cu -- checks that run on the device: the PML quotients against the IEEE division,
+// over every dividend, and the bounded waits.
 //
 // The PML updates divide by dh and by 1 + omega, divisors known before the launch; div_by and
 // div_by_signed (fd3d_common.cuh) form those quotients from a pair made on the host, div_steps
-// those of a divisor without one, and div_small and div_exact those they do not cover.  fd3d_check_division runs them, chosen as the
-// sweeps choose them, and __fdiv_rn on every one of the 2^32 float bit patterns for each divisor
-// given and counts the dividends whose results differ in any bit (two NaNs count as equal).
+// those of a divisor without one, and div_small and div_exact those they do not cover.
+// fd3d_check_division runs them, chosen as the sweeps choose them, and __fdiv_rn on every one of the
+// 2^32 float bit patterns for each divisor given and counts the dividends whose results differ in
+// any bit (two NaNs count as equal).
 #include <cuda_runtime.h>
 #include <cstdint>
 #include "../../include/fd3d_gpu.h"
@@ -58,6 +60,67 @@ __global__ void k_check_division(float b, Pair y, Pair ys, float recip, unsigned
     }
 }
 
+// ---------------------------------------------------------------- self-test of the waits
+// An mbarrier phase that no copy or arrival completes, and a grid barrier that one CTA
+// never reaches: both waits must give up by their bound, record ST_TIMEOUT and return,
+// leaving the context usable (failure detection without a hung or faulted GPU).
+__global__ void k_check_mbar_wait(int* status) {
+    __shared__ __align__(8) uint64_t bar;
+    if (threadIdx.x == 0) { mbar_init(smem_addr(&bar), 1); fence_mbar_init(); }
+    __syncthreads();
+    const bool done = mbar_wait(smem_addr(&bar), 0u);  // nothing ever arrives on this phase
+    if (__syncthreads_or(!done) && threadIdx.x == 0) atomicOr(status, ST_TIMEOUT);
+}
+
+struct BarrierSync {
+    unsigned count;
+    unsigned gen;
+    int abort;
+    int pad;
+};
+
+constexpr int BARRIER_SPIN_LIMIT = 1 << 22;
+
+// Sense-counting grid barrier with a bounded spin; false if this CTA gave up (or another did).  No
+// kernel of a step waits for another CTA: this is the pattern of such a wait, kept under test.
+__device__ bool grid_barrier(BarrierSync* b, unsigned nblocks, int* status) {
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        ok = 1;
+        volatile unsigned* vgen = &b->gen;
+        volatile int* vab = &b->abort;
+        const unsigned g0 = *vgen;
+        __threadfence();
+        const unsigned arrived = atomicAdd(&b->count, 1u);
+        if (arrived == nblocks - 1) {
+            atomicExch(&b->count, 0u);
+            __threadfence();
+            atomicAdd(&b->gen, 1u);
+        } else {
+            int n = 0;
+            while (*vgen == g0) {
+                if (*vab) { ok = 0; break; }
+                if (++n > BARRIER_SPIN_LIMIT) {
+                    atomicOr(status, ST_TIMEOUT);
+                    atomicExch(&b->abort, 1);
+                    ok = 0;
+                    break;
+                }
+                __nanosleep(64);
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__global__ void k_check_grid_barrier(BarrierSync* sync, int* status) {
+    if (blockIdx.x == gridDim.x - 1) return;  // this CTA never arrives
+    grid_barrier(sync, gridDim.x, status);
+}
+
 }  // namespace
 
 extern "C" int fd3d_division_form(float divisor, int damping, int* form) {
@@ -107,5 +170,30 @@ extern "C" int fd3d_check_division(const float* divisors, int n, unsigned long l
     }
     cudaFree(dbad);
     cudaFree(dfirst);
+    return rc;
+}
+
+extern "C" int fd3d_check_waits(int* mbar_status, int* barrier_status) {
+    if (!mbar_status || !barrier_status) return FD3D_ERR_ARG;
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { cudaGetLastError(); return FD3D_ERR_NODEV; }
+    int* st = nullptr;
+    BarrierSync* sync = nullptr;
+    if (cudaMalloc(&st, 2 * sizeof(int)) != cudaSuccess) return FD3D_ERR_NOMEM;
+    if (cudaMalloc(&sync, sizeof(BarrierSync)) != cudaSuccess) { cudaFree(st); return FD3D_ERR_NOMEM; }
+    int rc = FD3D_OK, h[2] = {0, 0};
+    if (cudaMemset(st, 0, 2 * sizeof(int)) != cudaSuccess || cudaMemset(sync, 0, sizeof(BarrierSync)) != cudaSuccess)
+        rc = FD3D_ERR_CUDA;
+    if (rc == FD3D_OK) {
+        k_check_mbar_wait<<<1, 64>>>(st);
+        k_check_grid_barrier<<<2, 64>>>(sync, st + 1);
+        if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
+            cudaMemcpy(h, st, sizeof(h), cudaMemcpyDeviceToHost) != cudaSuccess)
+            rc = FD3D_ERR_CUDA;
+    }
+    cudaFree(st);
+    cudaFree(sync);
+    *mbar_status = h[0];
+    *barrier_status = h[1];
     return rc;
 }

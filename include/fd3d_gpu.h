@@ -360,7 +360,8 @@ int fd3d_check_division(const float* divisors, int n, unsigned long long* mismat
 int fd3d_division_form(float divisor, int damping, int* form);
 /* Self-test of the bounded device waits (no counterpart in the reference, whose GPU
  * regions never wait on each other): a kernel waits on an mbarrier phase that nothing
- * completes and a grid barrier that one CTA never reaches.  Both waits must give up after
+ * completes, another at a grid barrier (a pattern that no kernel of a step uses) that one CTA never
+ * reaches.  Both waits must give up after
  * their bound and record the timeout bit (4) in the status word returned here; the device
  * stays usable.  Takes about a second. */
 int fd3d_check_waits(int* mbar_status, int* barrier_status);
