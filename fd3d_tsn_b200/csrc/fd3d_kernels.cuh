@@ -1295,7 +1295,6 @@ __device__ __forceinline__ void fault_bc_body(const Grid& g, const Fields<T>& f,
         has_x = tid >= NZ && x_node(tid - NZ, xi, xk);
         if (has_x) x.load(g, f, q, law, distX_rd, xi, xk);
     }
-    __syncthreads();                      // the shared memory may hold the previous item's values
 
     // 1. trial tractions of the tile and its ring; the owner stores a node's state
     for (int n = tid; n < FBC_HX * FBC_HZ; n += NT) {
