@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
     __shared__ ModelPar M;
     load_par(M, models[m]);
     tma_ring_init(bars);
-        if (STRESS)
+    if (STRESS)
         str_interior_tma_body<float, true>(maps[m].s, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
     else
         vel_interior_tma_body<float, true>(maps[m].v, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ m
         case W_VEL_INT:
         case W_STR_INT: {
             tma_ring_init(bars);
-                        if (STRESS)
+            if (STRESS)
                 str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
             else
                 vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
@@ -227,11 +227,8 @@ __global__ void __launch_bounds__(KIND == 3 ? FBC_THREADS : 256, KIND == 3 ? 2 :
     }
 }
 
-__global__ void k_step_end(int* run_step, int n) {
-    pdl_wait();
-    pdl_launch_dependents();
-    *run_step += n;
-}
+// (launched plainly: after the last step's kernels, before the next graph)
+__global__ void k_step_end(int* run_step, int n) { *run_step += n; }
 
 // OR of the live models' device status words into out (one read-back per sync)
 __global__ void k_or_status(int* const* __restrict__ st, int n, int* out) {
