@@ -1636,7 +1636,8 @@ inline void launch_fault_bc(bool pdl, int law, int nsm, cudaStream_t st, const G
     int nfres, tiles_x, tiles;
     fault_bc_grid(g, 8, nfres, tiles_x, tiles);
     if (law == 0) {
-        if (sizeof(T) == 4 || tiles <= nsm) launch_fault_bc_n<T, 0, FBC_THREADS>(pdl, st, g, f, q, c, s, it_dev, h, status);
+        if constexpr (sizeof(T) == 4) launch_fault_bc_n<T, 0, FBC_THREADS>(pdl, st, g, f, q, c, s, it_dev, h, status);
+        else if (tiles <= nsm) launch_fault_bc_n<T, 0, FBC_THREADS>(pdl, st, g, f, q, c, s, it_dev, h, status);
         else launch_fault_bc_n<T, 0, 256>(pdl, st, g, f, q, c, s, it_dev, h, status);
     } else {
         if (tiles <= nsm) launch_fault_bc_n<T, 1, FBC_THREADS>(pdl, st, g, f, q, c, s, it_dev, h, status);
