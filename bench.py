@@ -449,7 +449,7 @@ def batch_section(args, world, rank, local, pg):
                           key=f"batch{len(models)}-seed{2024 + rank}")
     else:  # a fixed schedule at its usual tile depth, no tuning launches
         b.set_schedule(args.batch_schedule)
-        b.set_tuning(32 if args.batch_schedule == "graph" else 8, 3 if args.batch_schedule == "persistent" else 0)
+        b.set_tuning(32 if args.batch_schedule == "graph" else 8)
         tune = b.tuning()
     t_setup = time.perf_counter() - t_setup
     barrier(pg, local)

@@ -36,7 +36,7 @@ class Result:
 
 
 def pretune(models, cache_path: str | None = None, key: str | None = None, steps: int = 8):
-    """Tile shape and schedule for a request mix, picked before serving starts: a scratch
+    """Tile depth for a request mix, picked before serving starts: a scratch
     batch of the given sample models is autotuned (and cached under key), then dropped.
     Returns the tuning dict."""
     arena = int(sum(bytes_needed(m) for m in models) * 1.05) + (64 << 20)
@@ -56,12 +56,12 @@ def serve(stream, hbm_budget_bytes: int, chunk: int = 32, max_models: int = 1024
     (asynchronous), admits the requests that arrived meanwhile while that run is on the
     GPU (their set-up goes on the batch's own set-up stream), then waits for the run
     and retires the models that reached their last step.  tuning (from pretune) fixes
-    the schedule and tile shape.  keep_final(request) -> bool selects the requests whose
+    the tile depth.  keep_final(request) -> bool selects the requests whose
     final planes are kept in the results (all if None).  Returns (results, stats)."""
     b = Batch(hbm_budget_bytes, max_models)
     if tuning:
         b.set_schedule(tuning["schedule"])
-        b.set_tuning(tuning["kchunk"], tuning["ctas_per_sm"] if tuning["schedule"] == "persistent" else 0)
+        b.set_tuning(tuning["kchunk"])
     need = {id(m): bytes_needed(m) for _, m in stream}
     waiting = []           # (arrival, model) arrived but not admitted
     resident = {}          # slot -> (arrival, admitted, model)
