@@ -190,6 +190,12 @@ __global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ m
     }
 }
 
+// room for the ring in a kernel's dynamic shared memory
+template <class K>
+bool ring_ok(K k, int bytes) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
+}
+
 // Plane items in three kernels by register need, so that light items are not held to a
 // heavy body's register count: KIND 3 the fused fault-BC tiles of slip-weakening models with a
 // thread per node and role (small batches: see launch_fault_bc), KIND 1 the fused fault-BC tiles (and the fres items launched
@@ -474,6 +480,10 @@ int build_work_t(fd3d_batch* b) {
         b->work_t.insert(b->work_t.end(), byt[t].begin(), byt[t].end());
     }
     b->tbeg[NTYPES] = (int)b->work_t.size();
+    if (b->pml_pair < (int)byt[W_VEL_PML].size() && !(ring_ok(k_bhalf<false, true>, VEL_RING) && ring_ok(k_bhalf<true, true>, STR_RING))) {
+        cudaGetLastError();
+        return FD3D_ERR_CUDA;
+    }
     if (b->work_t.size() > b->work_t_cap) {
         if (b->d_work_t) cudaFree(b->d_work_t);
         b->work_t_cap = b->work_t.size() + b->work_t.size() / 2 + 64;
@@ -749,11 +759,8 @@ int fd3d_batch_create(size_t arena_bytes, int max_models, fd3d_batch** out) {
         if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return fail(FD3D_ERR_CUDA);
     for (cudaEvent_t& e : b->evf)
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return fail(FD3D_ERR_CUDA);
-    auto ring_ok = [](auto k, int bytes) {
-        return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
-    };
     if (!ring_ok(k_bint<false>, VEL_RING) || !ring_ok(k_bint<true>, STR_RING) || !ring_ok(k_bhalf<false, false>, VEL_RING) ||
-        !ring_ok(k_bhalf<true, false>, STR_RING) || !ring_ok(k_bhalf<false, true>, VEL_RING) || !ring_ok(k_bhalf<true, true>, STR_RING)) {
+        !ring_ok(k_bhalf<true, false>, STR_RING)) {
         cudaGetLastError();
         return fail(FD3D_ERR_CUDA);
     }

@@ -370,7 +370,7 @@ struct Ctx : CtxBase {
         if (dalloc(&dprof, prof.size())) return FD3D_ERR_NOMEM;
         CK(cudaMemcpyAsync(dprof, prof.data(), prof.size() * sizeof(Damp<T>), cudaMemcpyHostToDevice, st));
         X.prof = dprof;
-        tma_ok = make_interior_maps<T>(g, f, vmaps, smaps) && prepare_tma_kernels<T>();
+        tma_ok = make_interior_maps<T>(g, f, vmaps, smaps) && prepare_tma_kernels<T>(c.pml_form != PML_PAIR);
         if (slab && !tma_ok) return FD3D_ERR_CUDA;
         if (!pml_minb_vel) pml_minb_vel = pml_minb<T>(false);
         if (!pml_minb_str) pml_minb_str = pml_minb<T>(true);

@@ -507,20 +507,20 @@ constexpr int vel_ring_bytes() { return TMA_NS * VelSlot::ELEMS * (int)sizeof(T)
 template <class T>
 constexpr int str_small_smem(bool layered) { return layered ? str_ring_bytes<T, true>() : str_ring_bytes<T, false>(); }
 
+// any: the model's quotients take a form of their own (the other kernels are not loaded for it)
 template <class T>
-bool prepare_tma_kernels() {
+bool prepare_tma_kernels(bool any) {
     const int vs = vel_ring_bytes<T>(), ss = str_ring_bytes<T, false>(),
               ssl = str_ring_bytes<T, true>();
     bool ok = cudaFuncSetAttribute(k_vel_interior_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, ss) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_vel_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
     ok &= cudaFuncSetAttribute(k_str_interior_tma<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, ssl) == cudaSuccess;
-    for (bool layered : {false, true})
-        for (bool any : {false, true}) {
-            ok &= cudaFuncSetAttribute(vel_small_kernel<T>(layered, any), cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
-            ok &= cudaFuncSetAttribute(str_small_kernel<T>(layered, any), cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       layered ? ssl : ss) == cudaSuccess;
-        }
+    for (bool layered : {false, true}) {
+        ok &= cudaFuncSetAttribute(vel_small_kernel<T>(layered, any), cudaFuncAttributeMaxDynamicSharedMemorySize, vs) == cudaSuccess;
+        ok &= cudaFuncSetAttribute(str_small_kernel<T>(layered, any), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   layered ? ssl : ss) == cudaSuccess;
+    }
     if (!ok) cudaGetLastError();
     return ok;
 }
