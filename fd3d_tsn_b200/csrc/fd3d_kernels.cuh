@@ -1538,11 +1538,14 @@ constexpr PmlKernel<T> pml_kernel_of() {
     if constexpr (STRESS) return k_str_pml<T, MINB, SLAB, ANY>;
     else return k_vel_pml<T, MINB, SLAB, ANY>;
 }
+// the kernels of quotients with a form of their own, in a module of their own (fd3d_forms.cu): a
+// program whose models do not take them does not load them
+PmlKernel<float> pml_kernel_forms(bool stress, bool slab);
 template <class T, bool STRESS>
 inline PmlKernel<T> pml_kernel(int minb, bool slab, bool any) {
-    constexpr bool F32 = sizeof(T) == 4;  // (FP64 divides directly: one form)
-    if (slab) return any ? pml_kernel_of<T, STRESS, true, F32>() : pml_kernel_of<T, STRESS, true, false>();
-    if (any) return pml_kernel_of<T, STRESS, false, F32>();
+    if constexpr (sizeof(T) == 4)  // (FP64 divides directly: one form)
+        if (any) return pml_kernel_forms(STRESS, slab);
+    if (slab) return pml_kernel_of<T, STRESS, true, false>();
     switch (minb) {
         case 2: return pml_kernel_of<T, STRESS, false, false, 2>();
         case 3: return pml_kernel_of<T, STRESS, false, false, 3>();

@@ -491,16 +491,23 @@ k_str_small(const __grid_constant__ StrMaps M, const __grid_constant__ Grid g, c
 
 // the kernels of a medium (layered or not) and quotient form (FP64 has one)
 template <class T>
-inline auto vel_small_kernel(bool layered, bool any) {
-    constexpr bool F32 = sizeof(T) == 4;
-    return layered ? (any ? k_vel_small<T, true, F32> : k_vel_small<T, true, false>)
-                   : (any ? k_vel_small<T, false, F32> : k_vel_small<T, false, false>);
+using VelSmallKernel = void (*)(VelMaps, Grid, Fields<T>, Fault<T>, PmlDesc, PmlAux<T>, StepConst<T>, int, FvwScalars, int*, int*,
+                                int, dim3, dim3);
+template <class T>
+using StrSmallKernel = void (*)(StrMaps, Grid, Fields<T>, Fault<T>, PmlDesc, PmlAux<T>, StepConst<T>, int*, int, dim3, dim3);
+VelSmallKernel<float> vel_small_forms(bool layered);  // (fd3d_forms.cu, as pml_kernel_forms)
+StrSmallKernel<float> str_small_forms(bool layered);
+template <class T>
+inline VelSmallKernel<T> vel_small_kernel(bool layered, bool any) {
+    if constexpr (sizeof(T) == 4)
+        if (any) return vel_small_forms(layered);
+    return layered ? k_vel_small<T, true, false> : k_vel_small<T, false, false>;
 }
 template <class T>
-inline auto str_small_kernel(bool layered, bool any) {
-    constexpr bool F32 = sizeof(T) == 4;
-    return layered ? (any ? k_str_small<T, true, F32> : k_str_small<T, true, false>)
-                   : (any ? k_str_small<T, false, F32> : k_str_small<T, false, false>);
+inline StrSmallKernel<T> str_small_kernel(bool layered, bool any) {
+    if constexpr (sizeof(T) == 4)
+        if (any) return str_small_forms(layered);
+    return layered ? k_str_small<T, true, false> : k_str_small<T, false, false>;
 }
 template <class T>
 constexpr int vel_ring_bytes() { return TMA_NS * VelSlot::ELEMS * (int)sizeof(T) + TMA_SMEM_PAD; }
