@@ -33,6 +33,7 @@
 #include <string>
 #include <vector>
 #include "../../include/fd3d_gpu.h"
+#include "fd3d_batch.cuh"
 #include "fd3d_common.cuh"
 #include "fd3d_kernels.cuh"
 #include "fd3d_opt.cuh"
@@ -53,50 +54,7 @@ using namespace fd3d;
 
 namespace {
 
-enum WorkType : int {
-    W_VEL_INT = 0, W_VEL_FAULT, W_VEL_PML, W_VEL_FS, W_STR_INT, W_STR_FAULT, W_STR_PML, W_STR_FS, W_FBC, W_NUC
-};
 constexpr int NPHASE = 5;
-
-struct Work {
-    int tm;          // type | model << 8
-    int bx, by, bz;
-};
-
-// what the sweeps read of a model: a CTA copies it to shared memory first (load_par), where a
-// store to the wave field cannot alias it (from global memory each pointer and size was
-// loaded again after each store: 705 instructions a cell in the stress PML tiles)
-struct ModelPar {
-    Grid g;
-    Fields<float> f;
-    StepConst<float> c;
-    PmlDesc D;
-    PmlAux<float> X;
-};
-
-struct ModelDev : ModelPar {
-    Fault<float> q;
-    FvwScalars fs;
-    HistDesc h;
-    int law;
-    int* it_dev;
-    int* status;
-    double* psiX0;
-    double* psiZ0;
-};
-
-// every thread of the CTA calls it
-__device__ __forceinline__ void load_par(ModelPar& dst, const ModelPar& src) {
-    static_assert(sizeof(ModelPar) % 4 == 0, "copied by words");
-    for (int w = threadIdx.y * blockDim.x + threadIdx.x; w < (int)(sizeof(ModelPar) / 4); w += blockDim.x * blockDim.y)
-        reinterpret_cast<int*>(&dst)[w] = reinterpret_cast<const int*>(&src)[w];
-    __syncthreads();
-}
-
-struct ModelMaps {  // TMA descriptors of one model's interior sweeps (global memory, 64-byte aligned)
-    VelMaps v;
-    StrMaps s;
-};
 
 // ---------------------------------------------------------------- graph schedule
 // One kernel per region and step, every CTA one item.
@@ -105,13 +63,6 @@ struct ModelMaps {  // TMA descriptors of one model's interior sweeps (global me
 // (items of a model whose step limit is reached return at once).  Each kernel gets its own register and
 // shared-memory budget, so each region runs at its own occupancy.
 constexpr int NTYPES = 10;
-// dynamic shared memory of the kernels with interior tiles (1-D media only)
-constexpr int VEL_RING = TMA_NS * VelSlot::ELEMS * (int)sizeof(float) + TMA_SMEM_PAD, STR_RING = str_ring_bytes<float, true>();
-
-__device__ __forceinline__ bool item_live(const Work& it, const int* limit, const int* run_step, int ofs, int& m) {
-    m = it.tm >> 8;
-    return *run_step + ofs < limit[m];
-}
 
 template <bool STRESS>
 __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
@@ -132,62 +83,6 @@ __global__ void __launch_bounds__(256) k_bint(const ModelDev* __restrict__ model
         str_interior_tma_body<float, true>(maps[m].s, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
     else
         vel_interior_tma_body<float, true>(maps[m].v, M.g, M.f, M.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
-}
-
-template <bool STRESS, bool ANY>
-__global__ void __launch_bounds__(PML_TILE, 4) k_bpml(const ModelDev* __restrict__ models,
-                                                      const Work* __restrict__ work, int b0,
-                                                      const int* __restrict__ limit, const int* run_step, int ofs,
-                                                      int* gstatus) {
-    __shared__ __align__(128) float sm[PML_TILE * (STRESS ? AUX_NS : AUX_NV)];
-    __shared__ __align__(8) uint64_t bar;
-    pdl_wait();
-    pdl_launch_dependents();
-    const Work it = work[b0 + blockIdx.x];
-    int m;
-    if (!item_live(it, limit, run_step, ofs, m)) return;
-    __shared__ ModelPar M;
-    load_par(M, models[m]);
-    if (STRESS) str_pml_tile<float, false, ANY>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
-    else vel_pml_tile<float, false, ANY>(M.g, M.f, M.D, M.X, M.c, it.bx, sm, smem_addr(&bar), gstatus);
-}
-
-// A half-step of a small batch in one launch: the interior, fault-band and PML items (contiguous
-// in the list by type), as k_vel_small / k_str_small do for one model.
-template <bool STRESS, bool ANY>
-__global__ void __launch_bounds__(256, 4) k_bhalf(const ModelDev* __restrict__ models, const ModelMaps* __restrict__ maps,
-                                                  const Work* __restrict__ work, int b0, const int* __restrict__ limit,
-                                                  const int* run_step, int ofs, int kchunk, int* gstatus) {
-    extern __shared__ __align__(128) unsigned char smem_raw[];
-    float* ring = reinterpret_cast<float*>(smem_raw + ((128u - (smem_addr(smem_raw) & 127u)) & 127u));
-    __shared__ __align__(8) uint64_t bars[TMA_NS];
-    __shared__ ModelPar P;
-    const Work it = work[b0 + blockIdx.x];
-    pdl_wait();
-    pdl_launch_dependents();
-    int m;
-    if (!item_live(it, limit, run_step, ofs, m)) return;
-    const ModelDev& M = models[m];
-    load_par(P, M);
-    switch (it.tm & 255) {
-        case W_VEL_INT:
-        case W_STR_INT: {
-            tma_ring_init(bars);
-            if (STRESS)
-                str_interior_tma_body<float, true>(maps[m].s, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
-            else
-                vel_interior_tma_body<float, true>(maps[m].v, P.g, P.f, P.c, kchunk, it.bx, it.by, it.bz, ring, bars, gstatus);
-            break;
-        }
-        case W_VEL_FAULT:
-        case W_STR_FAULT:
-            if (STRESS) str_fault_body<float>(P.g, P.f, M.q, P.c, it.bx, it.by, it.bz);
-            else vel_fault_body<float>(P.g, P.f, M.q, P.c, M.law, M.fs, M.it_dev, M.status, it.bx, it.by, it.bz);
-            break;
-        default:
-            if (STRESS) str_pml_tile<float, false, ANY>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
-            else vel_pml_tile<float, false, ANY>(P.g, P.f, P.D, P.X, P.c, it.bx, ring, smem_addr(bars), gstatus);
-    }
 }
 
 // room for the ring in a kernel's dynamic shared memory
@@ -480,7 +375,7 @@ int build_work_t(fd3d_batch* b) {
         b->work_t.insert(b->work_t.end(), byt[t].begin(), byt[t].end());
     }
     b->tbeg[NTYPES] = (int)b->work_t.size();
-    if (b->pml_pair < (int)byt[W_VEL_PML].size() && !(ring_ok(k_bhalf<false, true>, VEL_RING) && ring_ok(k_bhalf<true, true>, STR_RING))) {
+    if (b->pml_pair < (int)byt[W_VEL_PML].size() && !(ring_ok(batch_half_forms(false), VEL_RING) && ring_ok(batch_half_forms(true), STR_RING))) {
         cudaGetLastError();
         return FD3D_ERR_CUDA;
     }
@@ -584,7 +479,7 @@ int enqueue_graph_step(fd3d_batch* b, int ofs) {
         const int tp = half ? W_STR_PML : W_VEL_PML, tfs = half ? W_STR_FS : W_VEL_FS;
         const size_t sm = half ? STR_RING : VEL_RING;
         if (small) {
-            auto k = half ? (any ? k_bhalf<true, true> : k_bhalf<true, false>) : (any ? k_bhalf<false, true> : k_bhalf<false, false>);
+            const BatchHalfKernel k = any ? batch_half_forms(half) : half ? k_bhalf<true, false> : k_bhalf<false, false>;
             chk(launch_kernel(true, k, dim3(b->tbeg[tfs] - b->tbeg[ti]), blk, sm, b->st, b->d_models,
                               b->d_maps, b->d_work_t, b->tbeg[ti], b->d_limit, b->d_run_step, ofs, kc, b->d_status));
             plane(b->st, tfs, half ? W_FBC + 1 : tfs + 1);
@@ -605,12 +500,12 @@ int enqueue_graph_step(fd3d_batch* b, int ofs) {
             else chk(launch_kernel(pdl, k_bint<false>, dim3(n_of(ti)), blk, sm, b->st, md, mp, wt, b->tbeg[ti], lim, rs, ofs, kc, b->d_status));
         }
         plane(s0, tf, tf + 1);
-        auto pml = [&](void (*k)(const ModelDev*, const Work*, int, const int*, const int*, int, int*), int b0, int b1) {
+        auto pml = [&](BatchPmlKernel k, int b0, int b1) {
             if (b1 > b0) chk(launch_kernel(pdl, k, dim3(b1 - b0), blk, 0, s1, md, wt, b0, lim, rs, ofs, b->d_status));
         };
         const int p0 = b->tbeg[tp], p1 = p0 + b->pml_pair;
         pml(half ? k_bpml<true, false> : k_bpml<false, false>, p0, p1);
-        pml(half ? k_bpml<true, true> : k_bpml<false, true>, p1, b->tbeg[tp + 1]);
+        pml(batch_pml_forms(half), p1, b->tbeg[tp + 1]);
         if (b->branches) {
             BCK(cudaEventRecord(b->evf[1], b->side[0]));
             BCK(cudaEventRecord(b->evf[2], b->side[1]));
