@@ -17,7 +17,7 @@
 //
 // FD3D_BATCH_PERSISTENT is accepted and runs the same launches.  One cooperative kernel whose CTAs
 // walked the items between grid barriers was slower at every size, us a step against these:
-// 1 model 70 / 48, 2 models 123 / 84, 4 models 198 / 146, 16 models 605 / 495, 64 models 2224 / 1820
+// 1 model 68 / 47, 2 models 128 / 85, 4 models 193 / 147, 16 models 626 / 504, 64 models 2292 / 1845
 // (its one kernel ran every item at the registers of the largest body, 3 CTAs per SM).
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -91,11 +91,10 @@ bool ring_ok(K k, int bytes) {
     return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess;
 }
 
-// Plane items in three kernels by register need, so that light items are not held to a
-// heavy body's register count: KIND 3 the fused fault-BC tiles of slip-weakening models with a
-// thread per node and role (small batches: see launch_fault_bc), KIND 1 the fused fault-BC tiles (and the fres items launched
-// with them, 78 registers), KIND 2 the fault-band velocity (its rate-and-state Newton path
-// takes 114), KIND 0 the rest (free surface, stress fault band, nucleation ramp).
+// Plane items: KIND 1 the fused fault-BC tiles and the fres items launched with them (80 registers, 16 B
+// spilled), KIND 3 the same for a small batch of slip-weakening models with a thread per node and
+// role (launch_fault_bc; 56 registers, 160 B spilled), KIND 2 the fault-band velocity (62
+// registers), KIND 0 the rest (56): free surface, stress fault band, nucleation ramp.
 template <int KIND>
 __global__ void __launch_bounds__(KIND == 3 ? FBC_THREADS : 256, KIND == 3 ? 2 : KIND == 1 ? 3 : 1) k_bplane(const ModelDev* __restrict__ models, const Work* __restrict__ work,
                                                 int b0, const int* __restrict__ limit, const int* run_step, int ofs) {
@@ -434,9 +433,14 @@ int build_work(fd3d_batch* b) {
 
 // Whether a half-step of the batch is one launch (k_bhalf), its launches overlapped with the ones
 // before: up to 120 items per SM.  Beyond that the launches' tails no longer count, and each region
-// runs at the occupancy of its own kernel.  us a step, one launch / a launch per region, tiles of 8
-// planes: 1 model (0.7 K items or more) 48 / 67, 4 models 148 / 170, 12 models 393 / 400, 16 models 505 /
-// 506, 32 models 967 / 946; tiles of 32 planes: 74 / 103, 140 / 193, 386 / 407, 495 / 519, 957 / 957.
+// runs at the occupancy of its own kernel.  us a step, one launch / a launch per region:
+//   models               1         4          12         16         24         32         64
+//   slip weakening
+//   tiles of 8 planes    47 / 66   147 / 168  392 / 398  505 / 504  730 / 719  966 / 947  1904 / 1845
+//   tiles of 32          73 / 101  140 / 192  385 / 407  494 / 535  722 / 733  955 / 964  1886 / 1858
+//   rate-and-state (1.4 K items, 16 models 18-21 K, 32 models 36-41 K)
+//   tiles of 8           51 / 70   145 / 170  403 / 421  530 / 543  767 / 773  985 / 985
+//   tiles of 32          81 / 106  141 / 194  394 / 436  521 / 570  755 / 785  973 / 1002
 bool merged_step(const fd3d_batch* b) {
     if (b->branches || b->merged == 0) return false;
     return b->merged == 1 || b->tbeg[W_VEL_FS] - b->tbeg[W_VEL_INT] <= 120 * b->nsm;

@@ -1,7 +1,8 @@
 // fd3d_kernels.cuh -- sm_100a kernels of one FD3D_TSN time step (templated on the
 // field type T: float for the production build, double for the FP64 build).
 //
-// The step is eight launches, each a set of reference regions whose write sets are
+// The step is eight launches, or four on a small grid (small_step, fd3d_opt.cuh: 1-3 share a launch and
+// 5-7 another), each a set of reference regions whose write sets are
 // disjoint and which read nothing another thread of the same launch writes (the fused
 // fault boundary condition forms what its fres CTAs write from what they read):
 //   1 vel_interior  uxx1/vyy1/wzz1 (fd3d_deriv.f90:50-193)
@@ -316,7 +317,10 @@ __device__ __forceinline__ bool pml_cell(const PmlDesc& D, int s, long long t, i
 // thread loads its cell's neighbours, profile entries and medium (all before the wait); the new
 // components go straight back from registers, one full line per warp and component (a bulk
 // copy back had to drain before the CTA could leave: 25% slower at 0.5 M cells, 3% at 12 M).
-// Bound by memory latency and instruction issue together at 4 CTAs per SM (64 registers).
+// Bound by memory latency at 4 CTAs per SM (64 registers): on 2.3 M PML cells the velocity / stress sweep
+// moves 5.0 / 4.5 TB/s of DRAM (61 / 55% of peak) and issues in 51 / 42% of cycles, 430 / 528 instructions
+// a cell (546 / 702 with the five-operation quotients), its warps waiting for memory in 5.4 / 7.6 of the
+// cycles between two instructions.
 // Measured, velocity / stress, in us, against five-operation quotients with a branch each and
 // partly written sectors in the x strips (pml_sector_rest): 11.9 M PML cells 279 / 381 (340 /
 // 543), 13 M cells of 64 models 375 / 526 (446 / 638), 0.5 M cells 14.3 / 18.9 (15.5 / 22.7).
@@ -1603,7 +1607,7 @@ __global__ void k_output(Grid g, Fields<T> f, Fault<T> q, int law, const int* it
 
 // The fused fault boundary condition of one step: nfres CTAs of fres, then the fault tiles
 // (tiles_x per row of tiles); CTA of NT threads.  LAW is a template argument for its registers:
-// slip weakening in FP32 fits two CTAs of FBC_THREADS per SM, the others one.
+// slip weakening in FP32 fits two CTAs of FBC_THREADS per SM (56 registers, 100 B spilled), the others one.
 template <class T, int LAW, int NT>
 __global__ void __launch_bounds__(NT, NT == 256 ? (sizeof(T) == 4 ? 3 : 2) : LAW == 0 && sizeof(T) == 4 ? 2 : 1)
 k_fault_bc(const __grid_constant__ Grid g, const __grid_constant__ Fields<T> f, const __grid_constant__ Fault<T> q,
