@@ -123,6 +123,8 @@ __global__ void k_check_grid_barrier(BarrierSync* sync, int* status) {
 
 }  // namespace
 
+static_assert(FD3D_DIVISION_PAIR == PML_PAIR && FD3D_DIVISION_SIGNED == PML_SIGNED && FD3D_DIVISION_STEPS == PML_STEPS &&
+              FD3D_DIVISION_EXACT == PML_EXACT, "the header's forms are PmlForm's");
 extern "C" int fd3d_division_form(float divisor, int damping, int* form) {
     if (!form) return FD3D_ERR_ARG;
     float h, l, y;
